@@ -22,6 +22,7 @@
 // and all sums in FP64).
 #include "kevd_internal.cuh"
 #include "kevd_rng.cuh"
+#include "kevd_round.cuh"
 
 #include <algorithm>
 #include <cstring>
@@ -33,6 +34,18 @@ bool update_tc_supported(const float* F, int64_t ldF, int d);
 int launch_update_tc(kevd_ctx* ctx, float* F, int64_t ldF, int64_t N, int64_t k_max, const float* X, int d,
                      double scale, const int64_t* sacc, const float* minv_f, int b, const void* round_state,
                      double* dvec, double* dblk, int* err, cudaStream_t s);
+
+bool rpchol_small_supported(int b);
+int64_t rpchol_small_blocks(int64_t N);
+int launch_rpchol_small_init(kevd_ctx* ctx, double* dvec, double* dsub, int64_t N, RoundState* st, cudaStream_t s);
+int launch_rpchol_small_propose(kevd_ctx* ctx, const double* F, int64_t ldF, const float* X, int64_t N, int d,
+                                double scale, const double* dvec, const double* dsub, int round, int b, uint64_t seed,
+                                const double* uniforms, double tol, int64_t k_max, int max_rounds, double err_target,
+                                RoundState* st, double* minv, int64_t* sacc, int64_t* piv, double* err, int32_t* hm,
+                                cudaStream_t s);
+int launch_rpchol_small_update(kevd_ctx* ctx, double* F, int64_t ldF, const float* X, int64_t N, int d, double scale,
+                               const int64_t* sacc, const double* minv, int b, const RoundState* st, double* dvec,
+                               double* dsub, cudaStream_t s);
 
 constexpr int kRowBlock = 128;   // rows per update CTA (= rows per d partial sum)
 constexpr int kMaxBlock = 512;   // proposals per round (the reference's default BLK, ks_arpclm.cu:38)
@@ -54,16 +67,6 @@ constexpr int kSampleThreads = 1024;
 // error, the mean residual diagonal, has fallen below the same level.  The
 // FP64 form keeps the reference's tolerance alone (ks_arpclm.cu:329-331).
 constexpr double kMixedFloor = 16.0 / 16777216.0;
-
-struct RoundState {
-    int64_t rank;    // columns of F written
-    int64_t r_old;   // rank before this round's update
-    int32_t nacc;    // accepted this round
-    int32_t done;    // set once the factorisation has stopped
-    int32_t rounds;  // rounds executed
-    int32_t pad;
-    double total;    // sum of d after the last update
-};
 
 // Host side of a capture-safe factorisation: no host read inside the round
 // loop (all max_rounds rounds are enqueued; the kernels return at once after
@@ -767,8 +770,12 @@ static int rpchol_impl(kevd_ctx* ctx, const float* X, int64_t N, int d, double s
     const int n_split = (int)((p->k_max + kColChunk - 1) / kColChunk);
     const int n_kss = 32;   // CTAs sharing the FP64 K(S', S') block (one element per thread, same order)
     int st = KEVD_OK;
+    // few proposals in FP64: two kernels a round that touch the accepted columns
+    // only (kevd_rpchol_small.cu).  The FP32 form keeps the general kernels: a
+    // pivot sequence follows every rounding of its residual diagonal.
+    const bool small = sizeof(T) == 8 && rpchol_small_supported(b);
     double* dvec = arena_get<double>(ctx, "rp.d", N, &st);
-    double* dblk = arena_get<double>(ctx, "rp.dblk", nblk, &st);
+    double* dblk = arena_get<double>(ctx, "rp.dblk", small ? rpchol_small_blocks(N) : nblk, &st);
     RoundState* rs = arena_get<RoundState>(ctx, "rp.state", 1, &st);
     int64_t* props = arena_get<int64_t>(ctx, "rp.props", kMaxBlock, &st);
     int64_t* sacc = arena_get<int64_t>(ctx, "rp.sacc", kMaxBlock, &st);
@@ -787,8 +794,12 @@ static int rpchol_impl(kevd_ctx* ctx, const float* X, int64_t N, int d, double s
                                        cudaMemcpyHostToDevice, s));
     KEVD_CUDA(ctx, cudaMemsetAsync(err, 0, p->max_rounds * sizeof(double), s));
     KEVD_CUDA(ctx, cudaMemsetAsync(hm, 0, p->max_rounds * sizeof(int32_t), s));
-    rp_init_kernel<<<ctx->num_sms * 4, 256, 0, s>>>(dvec, dblk, N, nblk, rs);
-    KEVD_LAUNCH(ctx);
+    if (small) {
+        KEVD_TRY(launch_rpchol_small_init(ctx, dvec, dblk, N, rs, s));
+    } else {
+        rp_init_kernel<<<ctx->num_sms * 4, 256, 0, s>>>(dvec, dblk, N, nblk, rs);
+        KEVD_LAUNCH(ctx);
+    }
 
     const bool big = b > kSmallBlock;
     const size_t fsm = big ? 0 : (size_t)3 * b * b * sizeof(double);
@@ -813,55 +824,72 @@ static int rpchol_impl(kevd_ctx* ctx, const float* X, int64_t N, int d, double s
     if (st != KEVD_OK) return st;
     KEVD_CUDA(ctx, cudaMemsetAsync(tc_err, 0, sizeof(int), s));
     int round = 0;
+    auto propose_small = [&](int rnd, int nb, int limit) {
+        return launch_rpchol_small_propose(ctx, (const double*)F, ldF, X, N, d, scale, dvec, dblk, rnd, nb, p->seed,
+                                           unif, p->tol, p->k_max, limit, p->err_target, rs, minv, sacc, piv, err, hm,
+                                           s);
+    };
+    // rounds between two reads of the done flag (each read waits for the stream):
+    // a small round is short, and the rounds after the stop return at once
+    const int poll = small ? 16 : 4;
     for (; round < p->max_rounds; ++round) {
-        {
-            ProfScope ps(ctx, "rp_sample", s);
-            rp_sample_kernel<<<1, kSampleThreads, 0, s>>>(dvec, dblk, N, nblk, round, b, p->seed,
-                                                          unif, props, rs, p->k_max, p->max_rounds,
-                                                          p->err_target, floor_rel, err);
-            KEVD_LAUNCH(ctx);
-        }
-        {
-            ProfScope ps(ctx, "rp_hgram", s);
-            rp_hgram_kernel<T><<<n_split + n_kss, 256, hsm, s>>>(F, ldF, X, d, scale, props, b,
-                                                               n_split, rs, hpart, kss);
-            KEVD_LAUNCH(ctx);
-        }
-        {
-            ProfScope ps(ctx, "rp_factor", s);
-            if (big)
-                rp_factor_big_kernel<<<1, kBigFactorThreads, 0, s>>>(kss, hpart, b, round, p->seed, unif, p->tol,
-                                                                      floor_rel, p->k_max, props, rs, minv, minv_f,
-                                                                      sacc, piv, hm, hbig, hbig + (size_t)b * b,
-                                                                      hbig + (size_t)2 * b * b);
-            else
-                rp_factor_kernel<<<1, kFactorThreads, fsm, s>>>(kss, hpart, b, round, p->seed, unif, p->tol,
-                                                                floor_rel, p->k_max, props, rs, minv, minv_f, sacc,
-                                                                piv, hm);
-            KEVD_LAUNCH(ctx);
-        }
-        if (use_tc) {
-            KEVD_TRY(launch_update_tc(ctx, reinterpret_cast<float*>(F), ldF, N, p->k_max, X, d, scale, sacc,
-                                      minv_f, b, rs, dvec, dblk, tc_err, s));
+        if (small) {
+            KEVD_TRY(propose_small(round, b, p->max_rounds));
+            KEVD_TRY(launch_rpchol_small_update(ctx, (double*)F, ldF, X, N, d, scale, sacc, minv, b, rs, dvec, dblk, s));
         } else {
-            ProfScope ps(ctx, "rp_update", s);
-            for (int g = 0; g < n_groups; ++g) {
-                rp_update_kernel<T><<<(int)nblk, 256, usm, s>>>(F, ldF, X, N, d, scale, sacc, minv,
-                                                               minv_f, b, rs, dvec, dblk, g);
+            {
+                ProfScope ps(ctx, "rp_sample", s);
+                rp_sample_kernel<<<1, kSampleThreads, 0, s>>>(dvec, dblk, N, nblk, round, b, p->seed,
+                                                              unif, props, rs, p->k_max, p->max_rounds,
+                                                              p->err_target, floor_rel, err);
                 KEVD_LAUNCH(ctx);
             }
+            {
+                ProfScope ps(ctx, "rp_hgram", s);
+                rp_hgram_kernel<T><<<n_split + n_kss, 256, hsm, s>>>(F, ldF, X, d, scale, props, b,
+                                                                   n_split, rs, hpart, kss);
+                KEVD_LAUNCH(ctx);
+            }
+            {
+                ProfScope ps(ctx, "rp_factor", s);
+                if (big)
+                    rp_factor_big_kernel<<<1, kBigFactorThreads, 0, s>>>(kss, hpart, b, round, p->seed, unif, p->tol,
+                                                                          floor_rel, p->k_max, props, rs, minv, minv_f,
+                                                                          sacc, piv, hm, hbig, hbig + (size_t)b * b,
+                                                                          hbig + (size_t)2 * b * b);
+                else
+                    rp_factor_kernel<<<1, kFactorThreads, fsm, s>>>(kss, hpart, b, round, p->seed, unif, p->tol,
+                                                                    floor_rel, p->k_max, props, rs, minv, minv_f, sacc,
+                                                                    piv, hm);
+                KEVD_LAUNCH(ctx);
+            }
+            if (use_tc) {
+                KEVD_TRY(launch_update_tc(ctx, reinterpret_cast<float*>(F), ldF, N, p->k_max, X, d, scale, sacc,
+                                          minv_f, b, rs, dvec, dblk, tc_err, s));
+            } else {
+                ProfScope ps(ctx, "rp_update", s);
+                for (int g = 0; g < n_groups; ++g) {
+                    rp_update_kernel<T><<<(int)nblk, 256, usm, s>>>(F, ldF, X, N, d, scale, sacc, minv,
+                                                                   minv_f, b, rs, dvec, dblk, g);
+                    KEVD_LAUNCH(ctx);
+                }
+            }
         }
-        if (!defer && (round & 3) == 3) {
+        if (!defer && round % poll == poll - 1) {
             KEVD_CUDA(ctx, cudaMemcpyAsync(done_h, &rs->done, sizeof(int), cudaMemcpyDeviceToHost, s));
             KEVD_CUDA(ctx, cudaStreamSynchronize(s));
             if (*done_h) break;
         }
     }
     // closing sampler call: records the last round's error and the stop
-    rp_sample_kernel<<<1, kSampleThreads, 0, s>>>(dvec, dblk, N, nblk, std::min(round, p->max_rounds),
-                                                  0, p->seed, unif, props, rs, p->k_max,
-                                                  std::min(round, p->max_rounds), p->err_target, floor_rel, err);
-    KEVD_LAUNCH(ctx);
+    if (small) {
+        KEVD_TRY(propose_small(std::min(round, p->max_rounds), 0, std::min(round, p->max_rounds)));
+    } else {
+        rp_sample_kernel<<<1, kSampleThreads, 0, s>>>(dvec, dblk, N, nblk, std::min(round, p->max_rounds),
+                                                      0, p->seed, unif, props, rs, p->k_max,
+                                                      std::min(round, p->max_rounds), p->err_target, floor_rel, err);
+        KEVD_LAUNCH(ctx);
+    }
     if (defer) {
         // capture-safe: results go to pinned host memory, read after the stream completes
         KEVD_CUDA(ctx, cudaMemcpyAsync(defer->state_h, rs, sizeof(RoundState), cudaMemcpyDeviceToHost, s));
