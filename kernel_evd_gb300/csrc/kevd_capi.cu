@@ -1,6 +1,7 @@
 // The extern "C" boundary (include/kevd.h): argument checks, context and
 // workspace management, and the host orchestration that is not a kernel.
 #include "kevd_internal.cuh"
+#include "kevd_nystrom.cuh"
 
 #include <map>
 #include <mutex>
@@ -65,17 +66,6 @@ void Arena::release() {
         if (kv.second.p) cudaFree(kv.second.p);
     bufs_.clear();
 }
-
-// Nystrom model: landmark rows, Z' = L^{-T} Z and p1' = L^{-T} c1 packed as
-// the r x (k_out + 1) column-major matrix [Z' | p1'].
-struct Model {
-    int64_t r = 0;
-    int d = 0;
-    int k_out = 0;
-    double scale = 0.0;
-    float* xs = nullptr;   // r x d
-    double* zp = nullptr;  // r x (k_out + 1), column-major
-};
 
 }  // namespace kevd
 
@@ -450,6 +440,7 @@ int kevd_nystrom_prepare(kevd_ctx* ctx, const float* X, int64_t N, int32_t d, do
     // L = F(S, :) on the device; [Z' | p1'] = L^{-T} [Z | c1]
     int64_t* idx = arena_get<int64_t>(ctx, "ny.idx", r, &st);
     double* L = arena_get<double>(ctx, "ny.L", (size_t)r * r, &st);
+    double* zpd = arena_get<double>(ctx, "ny.zp", (size_t)r * (k_out + 1), &st);
     if (st != KEVD_OK) return set_error(ctx, st, "nystrom_prepare: out of device memory");
     kevd_model* m = new kevd_model();
     m->m.r = r;
@@ -457,7 +448,8 @@ int kevd_nystrom_prepare(kevd_ctx* ctx, const float* X, int64_t N, int32_t d, do
     m->m.k_out = k_out;
     m->m.scale = scale;
     if (cudaMalloc(&m->m.xs, (size_t)r * d * sizeof(float)) != cudaSuccess ||
-        cudaMalloc(&m->m.zp, (size_t)r * (k_out + 1) * sizeof(double)) != cudaSuccess) {
+        cudaMalloc(&m->m.w, (size_t)r * (k_out + 1) * sizeof(float2)) != cudaSuccess ||
+        cudaMalloc(&m->m.ex, (size_t)(k_out + 1) * sizeof(int)) != cudaSuccess) {
         cudaGetLastError();
         kevd_model_destroy(m);
         return set_error(ctx, KEVD_ERR_NOMEM, "nystrom_prepare: out of device memory");
@@ -468,7 +460,7 @@ int kevd_nystrom_prepare(kevd_ctx* ctx, const float* X, int64_t N, int32_t d, do
     int rc = KEVD_OK;
     do {
         if (cudaMemcpyAsync(idx, piv, r * sizeof(int64_t), cudaMemcpyHostToDevice, s) != cudaSuccess ||
-            cudaMemcpyAsync(m->m.zp, zp.data(), zp.size() * sizeof(double), cudaMemcpyHostToDevice, s) !=
+            cudaMemcpyAsync(zpd, zp.data(), zp.size() * sizeof(double), cudaMemcpyHostToDevice, s) !=
                 cudaSuccess) {
             rc = set_error(ctx, KEVD_ERR_CUDA, "nystrom_prepare: copy failed");
             break;
@@ -478,11 +470,13 @@ int kevd_nystrom_prepare(kevd_ctx* ctx, const float* X, int64_t N, int32_t d, do
         const double one = 1.0;
         if (cublasSetStream(ctx->blas, s) != CUBLAS_STATUS_SUCCESS ||
             cublasDtrsm(ctx->blas, CUBLAS_SIDE_LEFT, CUBLAS_FILL_MODE_LOWER, CUBLAS_OP_T,
-                        CUBLAS_DIAG_NON_UNIT, (int)r, k_out + 1, &one, L, (int)r, m->m.zp,
+                        CUBLAS_DIAG_NON_UNIT, (int)r, k_out + 1, &one, L, (int)r, zpd,
                         (int)r) != CUBLAS_STATUS_SUCCESS) {
             rc = set_error(ctx, KEVD_ERR_CUDA, "nystrom_prepare: trsm failed");
             break;
         }
+        rc = launch_nystrom_pack(ctx, zpd, m->m, s);
+        if (rc != KEVD_OK) break;
         // landmark rows X[piv]
         landmark_gather_kernel<<<(unsigned)std::min<int64_t>((r * d + 255) / 256, (int64_t)ctx->num_sms * 8), 256, 0,
                                  s>>>(X, idx, r, d, m->m.xs);
@@ -501,133 +495,19 @@ int kevd_nystrom_prepare(kevd_ctx* ctx, const float* X, int64_t N, int32_t d, do
     return KEVD_OK;
 }
 
-// Fused out-of-sample evaluation.  One CTA serves 32 query rows: for each
-// chunk of 32 landmarks it forms K(y, s_j) from FP32 direct differences summed
-// over the feature index in increasing order and an FP32 exp (relative error
-// about 1e-7 in K, far below the FP32 output's), and accumulates
-// P[row][c] = sum_j K(y, s_j) [Z'|p1'][j][c] in FP64 with j ascending in one
-// register per output: [Z'|p1'] = L^{-T}[Z|c1] has large entries of both
-// signs, so the sum stays FP64.  No thread ever combines two query rows, so a
-// row's result is bit-identical whatever batch it is evaluated in and wherever
-// it sits in the batch.
-constexpr int kNyRows = 32;
-constexpr int kNyLm = 32;
-constexpr int kNyMaxOut = 9;   // ceil(32 * 65 / 256) outputs per thread
-constexpr int kNyFeat = 128;   // features staged at a time
-
-__global__ void __launch_bounds__(256) nystrom_eval_kernel(const float* __restrict__ Y, int64_t n,
-                                                           const float* __restrict__ xs, const double* __restrict__ zp,
-                                                           int64_t r, int d, int k_out, double scale,
-                                                           float* __restrict__ Uy) {
-    extern __shared__ __align__(16) unsigned char ny_smem[];
-    constexpr int dp = kNyFeat + 1;
-    const int kc = k_out + 1;
-    double* kv = reinterpret_cast<double*>(ny_smem);     // 32 x 33
-    double* zc = kv + kNyRows * (kNyLm + 1);             // 32 landmarks x kc
-    float* ys = reinterpret_cast<float*>(zc + kNyLm * kc);  // 32 x dp (one feature chunk)
-    float* xc = ys + kNyRows * dp;                       // 32 x dp
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    const ScalePair fscale = split_scale(scale);
-    const int64_t row0 = (int64_t)blockIdx.x * kNyRows;
-    // with one feature chunk the query rows are staged once for all landmarks
-    const bool one_chunk = d <= kNyFeat;
-    if (one_chunk)
-        for (int e = threadIdx.x; e < kNyRows * d; e += 256) {
-            const int rr = e / d, kk = e - rr * d;
-            ys[rr * dp + kk] = (row0 + rr < n) ? Y[(row0 + rr) * d + kk] : 0.f;
-        }
-    double acc[kNyMaxOut];
-#pragma unroll
-    for (int q = 0; q < kNyMaxOut; ++q) acc[q] = 0.0;
-    const int n_out = kNyRows * kc;
-    for (int64_t j0 = 0; j0 < r; j0 += kNyLm) {
-        __syncthreads();
-        for (int e = threadIdx.x; e < kNyLm * kc; e += 256) {
-            const int jj = e / kc, c = e - jj * kc;
-            zc[jj * kc + c] = (j0 + jj < r) ? zp[(int64_t)c * r + j0 + jj] : 0.0;
-        }
-        // K(row ty + 8i, landmark tx): features kNyFeat at a time, in increasing order
-        float dist[4] = {0.f, 0.f, 0.f, 0.f};
-        for (int f0 = 0; f0 < d; f0 += kNyFeat) {
-            const int w = min(kNyFeat, d - f0);
-            __syncthreads();
-            if (!one_chunk)
-                for (int e = threadIdx.x; e < kNyRows * w; e += 256) {
-                    const int rr = e / w, kk = e - rr * w;
-                    ys[rr * dp + kk] = (row0 + rr < n) ? Y[(row0 + rr) * d + f0 + kk] : 0.f;
-                }
-            for (int e = threadIdx.x; e < kNyLm * w; e += 256) {
-                const int jj = e / w, kk = e - jj * w;
-                xc[jj * dp + kk] = (j0 + jj < r) ? xs[(j0 + jj) * d + f0 + kk] : 0.f;
-            }
-            __syncthreads();
-            for (int kk = 0; kk < w; ++kk) {
-                const float c = xc[tx * dp + kk];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const float t = ys[(ty + 8 * i) * dp + kk] - c;
-                    dist[i] = fmaf(t, t, dist[i]);
-                }
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-            kv[(ty + 8 * i) * (kNyLm + 1) + tx] = (j0 + tx < r) ? (double)kexp_scaled(dist[i], fscale) : 0.0;
-        __syncthreads();
-#pragma unroll
-        for (int q = 0; q < kNyMaxOut; ++q) {
-            const int o = threadIdx.x + 256 * q;
-            if (o < n_out) {
-                const int rr = o / kc, c = o - rr * kc;
-                double a = acc[q];
-#pragma unroll 8
-                for (int jj = 0; jj < kNyLm; ++jj) a += kv[rr * (kNyLm + 1) + jj] * zc[jj * kc + c];
-                acc[q] = a;
-            }
-        }
-    }
-    __syncthreads();
-    double* P = kv;   // reuse: 32 x kc doubles fit in kv + zc
-#pragma unroll
-    for (int q = 0; q < kNyMaxOut; ++q) {
-        const int o = threadIdx.x + 256 * q;
-        if (o < n_out) P[o] = acc[q];
-    }
-    __syncthreads();
-    for (int e = threadIdx.x; e < kNyRows * k_out; e += 256) {
-        const int rr = e / k_out, c = e - rr * k_out;
-        if (row0 + rr < n) Uy[(row0 + rr) * k_out + c] = (float)(P[rr * kc + c] / P[rr * kc + k_out]);
-    }
-}
-
-static size_t nystrom_smem(int d, int k_out) {
-    (void)d;
-    return (size_t)kNyRows * (kNyLm + 1) * 8 + (size_t)kNyLm * (k_out + 1) * 8 + 2 * (size_t)kNyRows * (kNyFeat + 1) * 4;
-}
-
 int kevd_nystrom_eval(kevd_ctx* ctx, const kevd_model* model, const float* Y, int64_t n, float* Uy,
                       void* stream) {
     KEVD_CHECK_CTX(ctx);
     if (!model || !Y || !Uy || n < 0) return set_error(ctx, KEVD_ERR_ARG, "nystrom_eval: bad arguments");
     if (n == 0) return KEVD_OK;
-    const Model& m = model->m;
-    const int64_t n_blocks = (n + kNyRows - 1) / kNyRows;
-    const size_t smem = nystrom_smem(m.d, m.k_out);
-    if (smem > 227 * 1024 || n_blocks > (int64_t)INT32_MAX)
-        return set_error(ctx, KEVD_ERR_ARG, "nystrom_eval: unsupported size (d=%d, n=%lld)", m.d, (long long)n);
-    cudaStream_t s = as_stream(stream);
-    if (smem > 48 * 1024)
-        KEVD_CUDA(ctx, raise_smem_limit(reinterpret_cast<const void*>(&nystrom_eval_kernel), (int)smem));
-    nystrom_eval_kernel<<<(unsigned)n_blocks, 256, smem, s>>>(Y, n, m.xs, m.zp, m.r, m.d, m.k_out,
-                                                                         m.scale, Uy);
-    KEVD_LAUNCH(ctx);
-    return KEVD_OK;
+    return launch_nystrom_eval(ctx, model->m, Y, n, Uy, as_stream(stream));
 }
 
 void kevd_model_destroy(kevd_model* model) {
     if (!model) return;
     if (model->m.xs) cudaFree(model->m.xs);
-    if (model->m.zp) cudaFree(model->m.zp);
+    if (model->m.w) cudaFree(model->m.w);
+    if (model->m.ex) cudaFree(model->m.ex);
     delete model;
 }
 
