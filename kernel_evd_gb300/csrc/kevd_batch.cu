@@ -2,7 +2,7 @@
 //
 // A batch of datasets (each its own X, N, d and eps sweep) is flattened into a
 // device work queue of (dataset, tile range) items covering every dataset's
-// lower-triangle 128 x 128 pair tiles.  One persistent grid (two CTAs per SM)
+// lower-triangle 128 x 128 pair tiles.  One persistent grid (four groups per SM)
 // takes items with an atomic counter, so the large datasets' items and the
 // small datasets' items share the GPU without one launch per dataset and
 // without idle SMs at the tail of a small dataset.  Each item writes its own
@@ -47,76 +47,44 @@ struct Item {
     int64_t t0, t1;      // tile range [t0, t1)
 };
 
-__device__ __forceinline__ float ex2f(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-
-__device__ __forceinline__ void tile_ij(int64_t t, int64_t& ti, int64_t& tj) {
-    int64_t i = (int64_t)((sqrt(8.0 * (double)t + 1.0) - 1.0) * 0.5);
-    while (i * (i + 1) / 2 > t) --i;
-    while ((i + 1) * (i + 2) / 2 <= t) ++i;
-    ti = i;
-    tj = t - i * (i + 1) / 2;
-}
-
-__global__ void __launch_bounds__(256, 2)
+// Each group of a CTA takes items of its own.
+__global__ void __launch_bounds__(kPtThreads, 1)
 calibrate_queue_kernel(const JobDesc* __restrict__ jobs, const Item* __restrict__ items, int item_base,
                        int n_items, const float* __restrict__ c2all, int* __restrict__ counter,
                        double* __restrict__ partial) {
-    extern __shared__ __align__(16) float sm[];
-    float* xi = sm;
-    float* xj = sm + kPtTile * kPtPitch;
-    float* cs = xj + kPtTile * kPtPitch;     // kMaxScalesB
-    float* red = cs + kMaxScalesB;           // 8 warps x kMaxScalesB
-    __shared__ int cur;
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    extern __shared__ __align__(16) float smem[];
+    __shared__ int cur[kPtGroups];
+    static_assert(kMaxScalesB <= kPtGroup, "one thread per scale");
+    const int g = pt_group(), gt = pt_tid();
+    float* sm = smem + g * kPtSmemFloats;
+    float* cs = smem + kPtGroups * kPtSmemFloats + g * (1 + kPtWarps) * kMaxScalesB;   // kMaxScalesB
+    float* red = cs + kMaxScalesB;                                                    // 4 warps x kMaxScalesB
     while (true) {
-        __syncthreads();
-        if (threadIdx.x == 0) cur = atomicAdd(counter, 1);
-        __syncthreads();
-        if (cur >= n_items) break;
-        const int it = item_base + cur;
+        pt_sync();
+        if (gt == 0) cur[g] = atomicAdd(counter, 1);
+        pt_sync();
+        if (cur[g] >= n_items) break;
+        const int it = item_base + cur[g];
         const Item item = items[it];
         const JobDesc jb = jobs[item.job];
-        const int d = jb.d, ns = jb.n_scales;
-        for (int j = threadIdx.x; j < ns; j += blockDim.x) cs[j] = c2all[jb.scale_off + j];
-        double acc = 0.0;   // thread j < ns owns eps j
-        for (int64_t t = item.t0; t < item.t1; ++t) {
-            int64_t ti, tj;
-            tile_ij(t, ti, tj);
-            float D[8][8];
-            pt_dist(jb.X, jb.N, d, ti * kTile, tj * kTile, xi, xj, ty, tx, D);
-            const int64_t gi0 = ti * kTile + ty, gj0 = tj * kTile + tx;
-#pragma unroll
-            for (int a = 0; a < 8; ++a)
-#pragma unroll
-                for (int b = 0; b < 8; ++b) {
-                    const int64_t gi = gi0 + 16 * a, gj = gj0 + 16 * b;
-                    if (!(gi < jb.N && gi > gj)) D[a][b] = __int_as_float(0x7f800000);
-                }
-            for (int j = 0; j < ns; ++j) {
-                const float c = -cs[j];
-                float s = 0.f;
-#pragma unroll
-                for (int a = 0; a < 8; ++a)
-#pragma unroll
-                    for (int b = 0; b < 8; ++b) s += ex2f(D[a][b] * c);
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-                if (lane == 0) red[warp * kMaxScalesB + j] = s;
-            }
-            __syncthreads();
-            if (threadIdx.x < ns) {
+        if (gt < jb.n_scales) cs[gt] = c2all[jb.scale_off + gt];
+        double acc = 0.0;   // thread j < n_scales of the group owns eps j
+        PtUnit unit = pt_unit(2 * item.t0);
+        int64_t staged = -1;
+        for (int64_t u = 2 * item.t0; u < 2 * item.t1; ++u, pt_next(unit)) {
+            f32x2 D[8][4];
+            pt_dist(jb.X, jb.N, jb.d, unit, sm, staged, D);
+            pt_mask(jb.N, unit, D);
+            pt_exp_sums(D, cs, jb.n_scales, red, kMaxScalesB);
+            pt_sync();
+            if (gt < jb.n_scales) {
                 double w = 0.0;
 #pragma unroll
-                for (int q = 0; q < 8; ++q) w += (double)red[q * kMaxScalesB + threadIdx.x];
+                for (int q = 0; q < kPtWarps; ++q) w += (double)red[q * kMaxScalesB + gt];
                 acc += w;
             }
         }
-        if (threadIdx.x < ns) partial[(int64_t)it * kMaxScalesB + threadIdx.x] = acc;
+        if (gt < jb.n_scales) partial[(int64_t)it * kMaxScalesB + gt] = acc;
     }
 }
 
@@ -133,7 +101,7 @@ __global__ void calibrate_queue_reduce_kernel(const JobDesc* __restrict__ jobs, 
 }
 
 size_t queue_smem() {
-    return (2 * kPtTile * (size_t)kPtPitch + kMaxScalesB + 8 * kMaxScalesB) * sizeof(float);
+    return (size_t)kPtGroups * (kPtSmemFloats + (1 + kPtWarps) * kMaxScalesB) * sizeof(float);
 }
 
 }  // namespace
@@ -155,9 +123,9 @@ int run_calibrate_batched(kevd_ctx* ctx, const kevd_calib_job* jobs, int n_jobs,
         const int64_t nt = (j.N + kTile - 1) / kTile;
         total_tiles += nt * (nt + 1) / 2;
     }
-    // item size: about 16 items per SM over the whole batch unless given
+    // item size: about 16 items per group of threads over the whole batch unless given
     int64_t per = tiles_per_item > 0 ? tiles_per_item
-                                     : std::max<int64_t>(1, total_tiles / ((int64_t)ctx->num_sms * 16));
+                                     : std::max<int64_t>(1, total_tiles / ((int64_t)ctx->num_sms * kPtGroups * 16));
     // features are staged kPtChunk at a time, so shared memory does not depend on d
     // and one persistent launch serves every dataset of the batch
     std::vector<int> order(n_jobs);
@@ -201,7 +169,7 @@ int run_calibrate_batched(kevd_ctx* ctx, const kevd_calib_job* jobs, int n_jobs,
     KEVD_CUDA(ctx, raise_smem_limit(reinterpret_cast<const void*>(&calibrate_queue_kernel), (int)smem));
     {
         ProfScope ps(ctx, "calibrate_queue", s);
-        calibrate_queue_kernel<<<ctx->num_sms * 2, 256, smem, s>>>(dj, di, 0, n_items, dc, counter, partial);
+        calibrate_queue_kernel<<<ctx->num_sms, kPtThreads, smem, s>>>(dj, di, 0, n_items, dc, counter, partial);
         KEVD_LAUNCH(ctx);
     }
     calibrate_queue_reduce_kernel<<<n_jobs, 64, 0, s>>>(dj, n_jobs, partial, out);

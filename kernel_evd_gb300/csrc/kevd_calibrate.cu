@@ -9,7 +9,7 @@
 //
 // Tiles cover the lower triangle ti >= tj of the 128-row tile grid; pairs with
 // i <= l, or outside [0, N), are masked to D = +inf (exp2(-inf) = 0).  Each
-// CTA is persistent over a static stride of tiles and keeps one FP64
+// CTA is persistent over a contiguous range of tiles and keeps one FP64
 // accumulator per scale; warp partials are FP32 (<= 2048 terms of <= 1).  The
 // per-CTA FP64 partials go to a scratch array and a second kernel reduces them
 // in a fixed order, so the result is deterministic.
@@ -31,12 +31,6 @@ constexpr int kCalMaxD = 1024;
 constexpr int kFC = 64;            // feature chunk staged in shared memory
 constexpr int kFP = kFC + 1;       // its row pitch (bank-conflict padding)
 
-__device__ __forceinline__ float ex2_approx(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-
 // Tile index t of the lower-triangular tile grid -> (ti, tj), ti >= tj.
 __device__ __forceinline__ void tri_tile(int64_t t, int64_t& ti, int64_t& tj) {
     int64_t i = (int64_t)((sqrt(8.0 * (double)t + 1.0) - 1.0) * 0.5);
@@ -57,52 +51,53 @@ __device__ __forceinline__ void load_chunk(const float* __restrict__ X, int64_t 
     }
 }
 
-__global__ void __launch_bounds__(256, 2)
+// Group p of the grid (four per CTA) takes a contiguous range of half tiles, so
+// that its i rows stay staged along a row of tiles.
+__global__ void __launch_bounds__(kPtThreads, 1)
 calibrate_tiles_kernel(const float* __restrict__ X, int64_t N, int d,
                        const float* __restrict__ c2, int n_scales, int64_t n_tiles,
                        double* __restrict__ partial) {
-    extern __shared__ __align__(16) float sm[];
-    float* xi = sm;
-    float* xj = sm + kPtTile * kPtPitch;
-    float* cs = xj + kPtTile * kPtPitch;                 // n_scales
-    float* red = cs + kCalMaxScales;                     // 8 warps x n_scales
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int j = threadIdx.x; j < n_scales; j += blockDim.x) cs[j] = c2[j];
-    double acc = 0.0;  // thread j < n_scales owns scale j
-    for (int64_t t = blockIdx.x; t < n_tiles; t += gridDim.x) {
-        int64_t ti, tj;
-        tri_tile(t, ti, tj);
-        float D[8][8];
-        pt_dist(X, N, d, ti * kCalTile, tj * kCalTile, xi, xj, ty, tx, D);
-        const int64_t gi0 = ti * kCalTile + ty, gj0 = tj * kCalTile + tx;
+    extern __shared__ __align__(16) float smem[];
+    const int g = pt_group();
+    float* sm = smem + g * kPtSmemFloats;
+    float* cs = smem + kPtGroups * kPtSmemFloats;                 // n_scales
+    float* red = cs + kCalMaxScales + g * kPtWarps * kCalMaxScales;   // 4 warps x n_scales
+    for (int j = threadIdx.x; j < n_scales; j += kPtThreads) cs[j] = c2[j];
+    __syncthreads();
+    constexpr int kPer = kCalMaxScales / kPtGroup;
+    double acc[kPer] = {};   // thread t of a group owns scales t, t + 128
+    const int64_t part = (int64_t)blockIdx.x * kPtGroups + g, parts = (int64_t)gridDim.x * kPtGroups;
+    const int64_t u0 = 2 * n_tiles * part / parts, u1 = 2 * n_tiles * (part + 1) / parts;
+    PtUnit unit = pt_unit(u0);
+    int64_t staged = -1;
+    for (int64_t u = u0; u < u1; ++u, pt_next(unit)) {
+        f32x2 D[8][4];
+        pt_dist(X, N, d, unit, sm, staged, D);
+        pt_mask(N, unit, D);
+        pt_exp_sums(D, cs, n_scales, red, kCalMaxScales);
+        pt_sync();
 #pragma unroll
-        for (int a = 0; a < 8; ++a)
+        for (int i = 0; i < kPer; ++i) {
+            const int j = pt_tid() + i * kPtGroup;
+            if (j < n_scales) {
+                double w = 0.0;
 #pragma unroll
-            for (int b = 0; b < 8; ++b) {
-                const int64_t gi = gi0 + 16 * a, gj = gj0 + 16 * b;
-                if (!(gi < N && gi > gj)) D[a][b] = __int_as_float(0x7f800000);  // +inf
+                for (int q = 0; q < kPtWarps; ++q) w += (double)red[q * kCalMaxScales + j];
+                acc[i] += w;
             }
-        for (int j = 0; j < n_scales; ++j) {
-            const float c = -cs[j];
-            float s = 0.f;
-#pragma unroll
-            for (int a = 0; a < 8; ++a)
-#pragma unroll
-                for (int b = 0; b < 8; ++b) s += ex2_approx(D[a][b] * c);
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-            if (lane == 0) red[warp * kCalMaxScales + j] = s;
-        }
-        __syncthreads();
-        if (threadIdx.x < n_scales) {
-            double w = 0.0;
-#pragma unroll
-            for (int q = 0; q < 8; ++q) w += (double)red[q * kCalMaxScales + threadIdx.x];
-            acc += w;
         }
     }
-    if (threadIdx.x < n_scales) partial[(int64_t)blockIdx.x * n_scales + threadIdx.x] = acc;
+    __syncthreads();
+    double* accs = reinterpret_cast<double*>(smem);   // over the tiles
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) accs[g * kCalMaxScales + pt_tid() + i * kPtGroup] = acc[i];
+    __syncthreads();
+    for (int j = threadIdx.x; j < n_scales; j += kPtThreads) {
+        double w = 0.0;
+#pragma unroll
+        for (int q = 0; q < kPtGroups; ++q) w += accs[q * kCalMaxScales + j];
+        partial[(int64_t)blockIdx.x * n_scales + j] = w;
+    }
 }
 
 __global__ void reduce_partials_kernel(const double* __restrict__ partial, int n_parts,
@@ -225,7 +220,7 @@ int run_calibrate_fp64(kevd_ctx* ctx, const float* X, int64_t N, int d, const do
 
 static size_t calib_smem(int d) {
     (void)d;
-    return (2 * kPtTile * (size_t)kPtPitch + kCalMaxScales + 8 * kCalMaxScales) * sizeof(float);
+    return ((size_t)kPtGroups * kPtSmemFloats + (1 + kPtGroups * kPtWarps) * kCalMaxScales) * sizeof(float);
 }
 
 int run_calibrate(kevd_ctx* ctx, const float* X, int64_t N, int d, const double* scales,
@@ -237,7 +232,7 @@ int run_calibrate(kevd_ctx* ctx, const float* X, int64_t N, int d, const double*
                          kCalMaxScales);
     const int64_t nt = (N + kCalTile - 1) / kCalTile;
     const int64_t n_tiles = nt * (nt + 1) / 2;
-    const int grid = (int)std::min<int64_t>(n_tiles, (int64_t)ctx->num_sms * 2);
+    const int grid = (int)std::min<int64_t>((2 * n_tiles + kPtGroups - 1) / kPtGroups, ctx->num_sms);
     int st = KEVD_OK;
     float* c2 = arena_get<float>(ctx, "cal.c2", kCalMaxScales, &st);
     double* partial = arena_get<double>(ctx, "cal.partial", (size_t)grid * n_scales, &st);
@@ -255,7 +250,7 @@ int run_calibrate(kevd_ctx* ctx, const float* X, int64_t N, int d, const double*
     KEVD_CUDA(ctx, raise_smem_limit(reinterpret_cast<const void*>(&calibrate_tiles_kernel), (int)smem));
     {
         ProfScope ps(ctx, "calibrate_tiles", s);
-        calibrate_tiles_kernel<<<grid, 256, smem, s>>>(X, N, d, c2, n_scales, n_tiles, partial);
+        calibrate_tiles_kernel<<<grid, kPtThreads, smem, s>>>(X, N, d, c2, n_scales, n_tiles, partial);
         KEVD_LAUNCH(ctx);
     }
     reduce_partials_kernel<<<1, kCalMaxScales, 0, s>>>(partial, grid, n_scales, out);
@@ -356,7 +351,7 @@ int run_calibrate_noalloc(const float* X, int64_t N, int d, const double* scales
     for (int j = 0; j < n_scales; ++j) hc[j] = (float)(scales[j] * 1.4426950408889634);
     const int64_t nt = (N + kCalTile - 1) / kCalTile;
     const int64_t n_tiles = nt * (nt + 1) / 2;
-    const int grid = (int)std::min<int64_t>(n_tiles, kNaGrid);
+    const int grid = (int)std::min<int64_t>((2 * n_tiles + kPtGroups - 1) / kPtGroups, kNaGrid / 2);   // one CTA per SM
     const size_t smem = calib_smem(d);
     // hc lives on this stack frame: the copy is complete (pageable source) or
     // staged before cudaMemcpyAsync returns, and the stream is synchronised
@@ -367,7 +362,7 @@ int run_calibrate_noalloc(const float* X, int64_t N, int d, const double* scales
         cudaGetLastError();
         return KEVD_ERR_CUDA;
     }
-    calibrate_tiles_kernel<<<grid, 256, smem, s>>>(X, N, d, sc.scales, n_scales, n_tiles, sc.partial);
+    calibrate_tiles_kernel<<<grid, kPtThreads, smem, s>>>(X, N, d, sc.scales, n_scales, n_tiles, sc.partial);
     reduce_partials_kernel<<<1, kCalMaxScales, 0, s>>>(sc.partial, grid, n_scales, sc.sums);
     if (cudaPeekAtLastError() != cudaSuccess ||
         cudaMemcpyAsync(sums, sc.sums, n_scales * sizeof(double), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
@@ -395,27 +390,32 @@ __device__ __forceinline__ void hist_add(unsigned* h, float D, int shift, unsign
     if (match) atomicAdd(&h[(u >> shift) & mask], 1u);
 }
 
-__global__ void __launch_bounds__(256, 2)
+__global__ void __launch_bounds__(kPtThreads, 1)
 median_tiles_kernel(const float* __restrict__ X, int64_t N, int d, int64_t n_tiles, int shift,
                     unsigned mask, unsigned prefix, int hi_shift, unsigned* __restrict__ hist) {
-    extern __shared__ __align__(16) float sm[];
-    float* xi = sm;
-    float* xj = sm + kPtTile * kPtPitch;
-    unsigned* h = reinterpret_cast<unsigned*>(xj + kPtTile * kPtPitch);
+    extern __shared__ __align__(16) float smem[];
+    float* sm = smem + pt_group() * kPtSmemFloats;
+    unsigned* h = reinterpret_cast<unsigned*>(smem + kPtGroups * kPtSmemFloats);
     for (int e = threadIdx.x; e < kHistBins; e += blockDim.x) h[e] = 0u;
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    for (int64_t t = blockIdx.x; t < n_tiles; t += gridDim.x) {
-        int64_t ti, tj;
-        tri_tile(t, ti, tj);
-        float D[8][8];
-        pt_dist(X, N, d, ti * kCalTile, tj * kCalTile, xi, xj, ty, tx, D);
-        const int64_t gi0 = ti * kCalTile + ty, gj0 = tj * kCalTile + tx;
+    __syncthreads();
+    const int64_t part = (int64_t)blockIdx.x * kPtGroups + pt_group(), parts = (int64_t)gridDim.x * kPtGroups;
+    const int64_t u0 = 2 * n_tiles * part / parts, u1 = 2 * n_tiles * (part + 1) / parts;
+    PtUnit unit = pt_unit(u0);
+    int64_t staged = -1;
+    for (int64_t u = u0; u < u1; ++u, pt_next(unit)) {
+        f32x2 D[8][4];
+        pt_dist(X, N, d, unit, sm, staged, D);
+        const int64_t gi0 = unit.ti * kPtTile + 8 * unit.h + (pt_tid() >> 4);
+        const int64_t gj0 = unit.tj * kPtTile + (pt_tid() & 15);
 #pragma unroll
         for (int a = 0; a < 8; ++a)
 #pragma unroll
-            for (int b = 0; b < 8; ++b) {
-                const int64_t gi = gi0 + 16 * a, gj = gj0 + 16 * b;
-                if (gi < N && gi > gj) hist_add(h, D[a][b], shift, mask, prefix, hi_shift);
+            for (int p = 0; p < 4; ++p) {
+                const int64_t gi = gi0 + 16 * a, gj = gj0 + 32 * p;
+                float x, y;
+                unpack2(D[a][p], x, y);
+                if (gi < N && gi > gj) hist_add(h, x, shift, mask, prefix, hi_shift);
+                if (gi < N && gi > gj + 16) hist_add(h, y, shift, mask, prefix, hi_shift);
             }
     }
     __syncthreads();
@@ -459,7 +459,7 @@ int run_pair_median(kevd_ctx* ctx, const float* X, int64_t N, int d, const int64
     int st = KEVD_OK;
     unsigned* hist = arena_get<unsigned>(ctx, "med.hist", kHistBins, &st);
     if (st != KEVD_OK) return st;
-    const size_t smem = 2 * kPtTile * (size_t)kPtPitch * sizeof(float) + kHistBins * sizeof(unsigned);
+    const size_t smem = (size_t)kPtGroups * kPtSmemFloats * sizeof(float) + kHistBins * sizeof(unsigned);
     KEVD_CUDA(ctx, raise_smem_limit(reinterpret_cast<const void*>(&median_tiles_kernel), (int)smem));
     const int shifts[3] = {20, 8, 0};
     const unsigned masks[3] = {0xfffu, 0xfffu, 0xffu};
@@ -469,8 +469,8 @@ int run_pair_median(kevd_ctx* ctx, const float* X, int64_t N, int d, const int64
     for (int pass = 0; pass < 3; ++pass) {
         KEVD_CUDA(ctx, cudaMemsetAsync(hist, 0, kHistBins * sizeof(unsigned), s));
         if (exact) {
-            const int grid = (int)std::min<int64_t>(n_tiles, (int64_t)ctx->num_sms * 2);
-            median_tiles_kernel<<<grid, 256, smem, s>>>(X, N, d, n_tiles, shifts[pass],
+            const int grid = (int)std::min<int64_t>((2 * n_tiles + kPtGroups - 1) / kPtGroups, ctx->num_sms);
+            median_tiles_kernel<<<grid, kPtThreads, smem, s>>>(X, N, d, n_tiles, shifts[pass],
                                                         masks[pass], prefix, hi_shift, hist);
         } else {
             const int grid = (int)std::min<int64_t>((n_pairs + 255) / 256, (int64_t)ctx->num_sms * 4);
