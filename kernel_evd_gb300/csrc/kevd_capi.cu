@@ -1,5 +1,6 @@
 // The extern "C" boundary (include/kevd.h): argument checks, context and
 // workspace management, and the host orchestration that is not a kernel.
+#include "kevd_f64_tc.cuh"
 #include "kevd_internal.cuh"
 #include "kevd_nystrom.cuh"
 
@@ -337,17 +338,77 @@ int kevd_factor_from_linv(kevd_ctx* ctx, const float* X, int64_t N, int32_t d, d
     int64_t* idx = arena_get<int64_t>(ctx, "fl.idx", r, &st);
     double* Li = arena_get<double>(ctx, "fl.Linv", (size_t)r * r, &st);
     double* Kp = arena_get<double>(ctx, "fl.K", (size_t)rows * r, &st);
-    double* Fp = precision == KEVD_MIXED ? arena_get<double>(ctx, "fl.F", (size_t)rows * r, &st) : nullptr;
     if (st != KEVD_OK) return set_error(ctx, st, "factor_from_linv: out of device memory");
     KEVD_CUDA(ctx, cudaMemcpyAsync(idx, piv, r * sizeof(int64_t), cudaMemcpyHostToDevice, s));
     KEVD_CUDA(ctx, cudaMemcpyAsync(Li, Linv, (size_t)r * r * sizeof(double), cudaMemcpyHostToDevice, s));
+    // F panel = (K panel) Linv^T, Linv lower triangular (its upper part is never
+    // read).  In exact slices on the tensor cores (N = 100,000, r = 1,024, d = 64:
+    // 13.9 ms the call, 8.2 of them this product and 5.0 the kernel panels; relative
+    // error against extended precision 1.2e-15); on the FP64 pipe (a triangular
+    // multiply, half the work of a GEMM; 146 ms, 8.3e-15) where the product is
+    // smaller than the slices' launches, has no room, or Linv is not finite.
+    uint64_t *Kq = nullptr, *Lq = nullptr;
+    int *ek = nullptr, *el = nullptr, *pre = nullptr, *flags = nullptr;
+    bool tc = (double)N * (double)r * (double)r >= 1e8;
+    if (tc) {
+        int st2 = KEVD_OK;
+        Kq = arena_get<uint64_t>(ctx, "fl.Kq", (size_t)rows * digits_ld(r), &st2);
+        Lq = arena_get<uint64_t>(ctx, "fl.Lq", (size_t)r * digits_ld(r), &st2);
+        ek = arena_get<int>(ctx, "fl.ek", (size_t)rows, &st2);
+        el = arena_get<int>(ctx, "fl.el", (size_t)r + 1, &st2);
+        pre = arena_get<int>(ctx, "fl.pre", (size_t)rows * ((r + 63) / 64), &st2);
+        tc = st2 == KEVD_OK && (rows + 127) / 128 <= 65535;
+    }
+    if (tc) {
+        flags = el + r;
+        KEVD_CUDA(ctx, cudaMemsetAsync(flags, 0, sizeof(int), s));
+        KEVD_TRY(launch_digits_rows(ctx, Li, r, r, r, true, true, Lq, el, nullptr, s));
+        std::vector<int> hel(r);
+        KEVD_CUDA(ctx, cudaMemcpyAsync(hel.data(), el, r * sizeof(int), cudaMemcpyDeviceToHost, s));
+        KEVD_CUDA(ctx, cudaStreamSynchronize(s));
+        for (int e : hel) tc = tc && e != kDigitsNotFinite;
+    }
+    // the kernel panels from exact distances as well, where the states allow it
+    StateDigits xd = {}, sd = {};
+    int xe = 0;
+    bool ktc = false;
+    if (tc) {
+        if (d >= 1 && d <= kMaxFeatures) KEVD_TRY(states_exp(ctx, X, N, d, scale, &xe, &ktc, s));
+        int st2 = KEVD_OK;
+        xd.q = arena_get<uint64_t>(ctx, "fl.xq", (size_t)rows * digits_ld(d), &st2);
+        xd.norm = arena_get<int64_t>(ctx, "fl.xn", (size_t)rows * 2, &st2);
+        sd.q = arena_get<uint64_t>(ctx, "fl.sq", (size_t)r * digits_ld(d), &st2);
+        sd.norm = arena_get<int64_t>(ctx, "fl.sn", (size_t)r * 2, &st2);
+        ktc = ktc && st2 == KEVD_OK && (rows + 127) / 128 <= 65535;
+        if (ktc) KEVD_TRY(launch_digits_states(ctx, X, 0, idx, r, d, xe, sd, s));
+    }
+    double* Fp = nullptr;
+    if (!tc && precision == KEVD_MIXED) {
+        Fp = arena_get<double>(ctx, "fl.F", (size_t)rows * r, &st);
+        if (st != KEVD_OK) return set_error(ctx, st, "factor_from_linv: out of device memory");
+    }
     KEVD_BLAS(ctx, cublasSetStream(ctx->blas, s));
     const double one = 1.0;
     for (int64_t r0 = 0; r0 < N; r0 += rows) {
         const int64_t nr = std::min(rows, N - r0);
-        KEVD_TRY(launch_kernel_block(ctx, X, N, d, scale, nullptr, r0, nr, idx, r, KEVD_FP64, Kp, r, s));
-        // (F panel)^T = Linv * (K panel)^T  in column-major terms; Linv is lower
-        // triangular (its upper part is never read), half the FP64 work of a GEMM
+        {
+            ProfScope ps(ctx, "linv_kernel_block", s);
+            if (ktc) {
+                KEVD_TRY(launch_digits_states(ctx, X, r0, nullptr, nr, d, xe, xd, s));
+                KEVD_TRY(launch_kernel_f64_tc(ctx, xd, nr, sd, r, d, xe, scale, Kp, r, flags, s));
+            } else {
+                KEVD_TRY(launch_kernel_block(ctx, X, N, d, scale, nullptr, r0, nr, idx, r, KEVD_FP64, Kp, r, s));
+            }
+        }
+        ProfScope ps(ctx, "linv_multiply", s);
+        if (tc) {
+            KEVD_TRY(launch_digits_rows(ctx, Kp, nr, r, r, false, false, Kq, ek, pre, s));
+            KEVD_TRY(launch_tri_f64_tc(ctx, TriOperands{Kp, Li, Kq, Lq, ek, el, pre}, nr, r,
+                                       precision == KEVD_FP64 ? (double*)F + r0 * ldF : nullptr,
+                                       precision == KEVD_FP64 ? nullptr : (float*)F + r0 * ldF, ldF, flags, s));
+            continue;
+        }
+        // (F panel)^T = Linv * (K panel)^T  in column-major terms
         double* dst = precision == KEVD_FP64 ? (double*)F + r0 * ldF : Fp;
         const int64_t ldd = precision == KEVD_FP64 ? ldF : r;
         KEVD_BLAS(ctx, cublasDtrmm(ctx->blas, CUBLAS_SIDE_LEFT, CUBLAS_FILL_MODE_LOWER, CUBLAS_OP_N,
@@ -359,7 +420,10 @@ int kevd_factor_from_linv(kevd_ctx* ctx, const float* X, int64_t N, int32_t d, d
             KEVD_LAUNCH(ctx);
         }
     }
+    int herr = 0;
+    if (tc) KEVD_CUDA(ctx, cudaMemcpyAsync(&herr, flags, sizeof(int), cudaMemcpyDeviceToHost, s));
     KEVD_CUDA(ctx, cudaStreamSynchronize(s));
+    if (herr != 0) return set_error(ctx, KEVD_ERR_TIMEOUT, "factor_from_linv: pipeline wait timed out (code %d)", herr);
     return KEVD_OK;
 }
 

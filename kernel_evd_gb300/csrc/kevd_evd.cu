@@ -17,6 +17,7 @@
 // uses cuSOLVERMp / cuBLASMp for the same dense steps).  Cross-row sums are
 // FP64; FP32 factors accumulate FP32 partials over 1024-row chunks that are
 // then added in FP64.
+#include "kevd_f64_tc.cuh"
 #include "kevd_internal.cuh"
 #include "kevd_tc.cuh"
 
@@ -870,6 +871,56 @@ static int gram(kevd_ctx* ctx, const T* F, int64_t ldF, int64_t N, int64_t k, co
     return KEVD_OK;
 }
 
+// G = F^T diag(s)^2 F of an FP64 factor.  From kTcGramWork products N k^2 on, in
+// exact slices on the tensor cores (kevd_f64_tc.cu), else, or when that form does
+// not suit the call, on the FP64 pipe with the weights w = s^2 (formed in wbuf).
+// Call times, FP64 pipe / slices: 3,000 x 60 396 / 315 us, 10,000 x 150 725 / 313,
+// 20,000 x 500 5,141 / 615, 1,000,000 x 15 7,502 / 2,467; below that the slices'
+// five launches and the wait for their flags are most of the call.
+constexpr double kTcGramWork = 1e7;
+constexpr double kTcUWork = 5e7;   // N k, times the 64 columns either form computes
+static int gram_f64(kevd_ctx* ctx, const double* F, int64_t ldF, int64_t N, int64_t k, const double* s, double* wbuf,
+                    double* G, cudaStream_t st) {
+    if ((double)N * (double)k * (double)k >= kTcGramWork) {
+        bool done = false;
+        KEVD_TRY(run_gram_f64_tc(ctx, F, N, k, ldF, s, G, &done, st));
+        if (done) return KEVD_OK;
+    }
+    ev_square_kernel<<<ctx->num_sms * 4, 256, 0, st>>>(s, wbuf, N);
+    KEVD_LAUNCH(ctx);
+    return gram<double>(ctx, F, ldF, N, k, wbuf, G, st);
+}
+
+// U = Dtil^{-1} F Z (row-major float) of an FP64 factor, in exact slices on the
+// tensor cores, row panels of at most 2 GiB of digits at a time; *done = false
+// when there is no room for them.
+static int u_f64_tc(kevd_ctx* ctx, const double* F, int64_t ldF, int64_t N, int64_t k, const double* Z, int k_out,
+                    const double* dinv, float* U, bool* done, cudaStream_t st) {
+    *done = false;
+    const int64_t ld = digits_ld(k);
+    const int64_t panel = std::min(N, std::max<int64_t>(4096, ((int64_t)2 << 30) / (8 * ld)));
+    int rc = KEVD_OK;
+    uint64_t* q = arena_get<uint64_t>(ctx, "f64.q", (size_t)panel * ld, &rc);
+    uint64_t* zq = arena_get<uint64_t>(ctx, "f64.zq", (size_t)k_out * ld, &rc);
+    int* ea = arena_get<int>(ctx, "f64.ea", (size_t)panel, &rc);
+    int* ez = arena_get<int>(ctx, "f64.ez", (size_t)k_out + 1, &rc);
+    if (rc != KEVD_OK) return KEVD_OK;
+    int* err = ez + k_out;
+    KEVD_CUDA(ctx, cudaMemsetAsync(err, 0, sizeof(int), st));
+    KEVD_TRY(launch_digits_rows(ctx, Z, k_out, k, k, false, false, zq, ez, nullptr, st));
+    for (int64_t r = 0; r < N; r += panel) {
+        const int64_t rows = std::min(panel, N - r);
+        KEVD_TRY(launch_digits_rows(ctx, F + r * ldF, rows, k, ldF, false, false, q, ea, nullptr, st));
+        KEVD_TRY(launch_rows_f64_tc(ctx, q, ea, rows, zq, ez, k_out, k, dinv + r, U + r * k_out, k_out, err, st));
+    }
+    int h = 0;
+    KEVD_CUDA(ctx, cudaMemcpyAsync(&h, err, sizeof(int), cudaMemcpyDeviceToHost, st));
+    KEVD_CUDA(ctx, cudaStreamSynchronize(st));
+    if (h != 0) return set_error(ctx, KEVD_ERR_TIMEOUT, "bistochastic_evd: U pass timed out (code %d)", h);
+    *done = true;
+    return KEVD_OK;
+}
+
 static int d2h(kevd_ctx* ctx, double* host, const double* dev, size_t n, cudaStream_t s) {
     if (!host) return KEVD_OK;
     KEVD_CUDA(ctx, cudaMemcpyAsync(host, dev, n * sizeof(double), cudaMemcpyDeviceToHost, s));
@@ -1018,10 +1069,12 @@ static int evd_impl(kevd_ctx* ctx, const T* F, int64_t N, int64_t k, int64_t ldF
         KEVD_LAUNCH(ctx);
         KEVD_TRY(run_gram2_tc(ctx, FT, ldT, N, k, colmax, dinv, w2, A, B, s));
     } else {
-        ev_square_kernel<<<ctx->num_sms * 4, 256, 0, s>>>(dinv, w2, N);
+        KEVD_TRY(gram_f64(ctx, (const double*)F, ldF, N, k, dinv, w2, A, s));
+        double* qs = arena_get<double>(ctx, "ev.qs", N, &st);
+        if (st != KEVD_OK) return st;
+        ev_rsqrt_kernel<<<ctx->num_sms * 4, 256, 0, s>>>(qtil, qs, N);
         KEVD_LAUNCH(ctx);
-        KEVD_TRY(gram<T>(ctx, F, ldF, N, k, w2, A, s));
-        KEVD_TRY(gram<T>(ctx, F, ldF, N, k, qinv, B, s));
+        KEVD_TRY(gram_f64(ctx, (const double*)F, ldF, N, k, qs, w2, B, s));
     }
     if (dump) {
         KEVD_TRY(d2h(ctx, dump->c1, c1, k, s));
@@ -1149,7 +1202,12 @@ static int evd_impl(kevd_ctx* ctx, const T* F, int64_t N, int64_t k, int64_t ldF
             evt_u_kernel<<<ceil_div(N, 256), 256, 0, s>>>(FT, ldT, N, k, Z, k_out, dinv, U, Yrr);
             Urr = U;
         } else {
-            ev_u_kernel<T><<<dim3(ceil_div(N, 64), ceil_div(k_out, 64)), 256, 0, s>>>(F, ldF, N, k, Z, k_out, dinv, U);
+            bool u_done = false;
+            if (sizeof(T) == 8 && (double)N * (double)k * 64.0 >= kTcUWork)
+                KEVD_TRY(u_f64_tc(ctx, (const double*)F, ldF, N, k, Z, k_out, dinv, U, &u_done, s));
+            if (!u_done)
+                ev_u_kernel<T><<<dim3(ceil_div(N, 64), ceil_div(k_out, 64)), 256, 0, s>>>(F, ldF, N, k, Z, k_out, dinv,
+                                                                                      U);
             if (sizeof(T) == 4) {
                 // FP32 factor with k_out > 32: the leading 32 columns once more, with
                 // Y, for their refinement (Z's last 32 columns)
@@ -1206,9 +1264,7 @@ int run_weighted_gram(kevd_ctx* ctx, const void* F, int precision, int64_t N, in
     int rc = KEVD_OK;
     double* w2 = arena_get<double>(ctx, "wg.w2", N, &rc);
     if (rc != KEVD_OK) return set_error(ctx, rc, "weighted_gram: out of device memory");
-    ev_square_kernel<<<ctx->num_sms * 4, 256, 0, st>>>(s_dev, w2, N);
-    KEVD_LAUNCH(ctx);
-    KEVD_TRY(gram<double>(ctx, (const double*)F, ldF, N, k, w2, G, st));
+    KEVD_TRY(gram_f64(ctx, (const double*)F, ldF, N, k, s_dev, w2, G, st));
     KEVD_CUDA(ctx, cudaStreamSynchronize(st));
     return KEVD_OK;
 }
