@@ -44,7 +44,7 @@ struct JobDesc {
 struct Item {
     int32_t job;
     int32_t pad;
-    int64_t t0, t1;      // tile range [t0, t1)
+    int64_t u0, u1;      // range [u0, u1) of half tiles (pt_unit)
 };
 
 // Each group of a CTA takes items of its own.
@@ -69,9 +69,9 @@ calibrate_queue_kernel(const JobDesc* __restrict__ jobs, const Item* __restrict_
         const JobDesc jb = jobs[item.job];
         if (gt < jb.n_scales) cs[gt] = c2all[jb.scale_off + gt];
         double acc = 0.0;   // thread j < n_scales of the group owns eps j
-        PtUnit unit = pt_unit(2 * item.t0);
+        PtUnit unit = pt_unit(item.u0);
         int64_t staged = -1;
-        for (int64_t u = 2 * item.t0; u < 2 * item.t1; ++u, pt_next(unit)) {
+        for (int64_t u = item.u0; u < item.u1; ++u, pt_next(unit)) {
             f32x2 D[8][4];
             pt_dist(jb.X, jb.N, jb.d, unit, sm, staged, D);
             pt_mask(jb.N, unit, D);
@@ -88,14 +88,24 @@ calibrate_queue_kernel(const JobDesc* __restrict__ jobs, const Item* __restrict_
     }
 }
 
-__global__ void calibrate_queue_reduce_kernel(const JobDesc* __restrict__ jobs, int n_jobs,
-                                              const double* __restrict__ partial, double* __restrict__ out) {
-    const int job = blockIdx.x;
-    if (job >= n_jobs) return;
-    const JobDesc jb = jobs[job];
-    for (int j = threadIdx.x; j < jb.n_scales; j += blockDim.x) {
-        double s = 0.0;
-        for (int q = 0; q < jb.n_items; ++q) s += partial[(int64_t)(jb.item0 + q) * kMaxScalesB + j];
+// One CTA per job: 16 slices of its items in item order, then the slices in order.
+constexpr int kReduceSlices = 16;
+__global__ void __launch_bounds__(kReduceSlices * kMaxScalesB)
+calibrate_queue_reduce_kernel(const JobDesc* __restrict__ jobs, const double* __restrict__ partial,
+                              double* __restrict__ out) {
+    __shared__ double part[kReduceSlices][kMaxScalesB];
+    const int job = blockIdx.x, j = threadIdx.x % kMaxScalesB, sl = threadIdx.x / kMaxScalesB;
+    const JobDesc& jb = jobs[job];
+    const int n = jb.n_items, q0 = (int)((int64_t)n * sl / kReduceSlices), q1 = (int)((int64_t)n * (sl + 1) / kReduceSlices);
+    double s = 0.0;
+    if (j < jb.n_scales) {
+#pragma unroll 8
+        for (int q = q0; q < q1; ++q) s += partial[(int64_t)(jb.item0 + q) * kMaxScalesB + j];
+    }
+    part[sl][j] = s;
+    __syncthreads();
+    if (sl == 0 && j < jb.n_scales) {
+        for (int t = 1; t < kReduceSlices; ++t) s += part[t][j];
         out[job * kMaxScalesB + j] = s;
     }
 }
@@ -123,9 +133,11 @@ int run_calibrate_batched(kevd_ctx* ctx, const kevd_calib_job* jobs, int n_jobs,
         const int64_t nt = (j.N + kTile - 1) / kTile;
         total_tiles += nt * (nt + 1) / 2;
     }
-    // item size: about 16 items per group of threads over the whole batch unless given
-    int64_t per = tiles_per_item > 0 ? tiles_per_item
-                                     : std::max<int64_t>(1, total_tiles / ((int64_t)ctx->num_sms * kPtGroups * 16));
+    // item size in half tiles: about 8 items per group of threads over the whole
+    // batch unless given
+    const int64_t per = tiles_per_item > 0
+                            ? 2 * (int64_t)tiles_per_item
+                            : std::max<int64_t>(1, 2 * total_tiles / ((int64_t)ctx->num_sms * kPtGroups * 8));
     // features are staged kPtChunk at a time, so shared memory does not depend on d
     // and one persistent launch serves every dataset of the batch
     std::vector<int> order(n_jobs);
@@ -147,7 +159,7 @@ int run_calibrate_batched(kevd_ctx* ctx, const kevd_calib_job* jobs, int n_jobs,
             if (!(j.scales[e] > 0.0)) return set_error(ctx, KEVD_ERR_ARG, "calibrate_batched: scales must be positive");
             hc.push_back((float)(j.scales[e] * 1.4426950408889634));
         }
-        for (int64_t t0 = 0; t0 < tiles; t0 += per) hi.push_back(Item{q, 0, t0, std::min(tiles, t0 + per)});
+        for (int64_t u0 = 0; u0 < 2 * tiles; u0 += per) hi.push_back(Item{q, 0, u0, std::min(2 * tiles, u0 + per)});
         d.n_items = (int32_t)hi.size() - d.item0;
         d.pad = 0;
     }
@@ -172,7 +184,7 @@ int run_calibrate_batched(kevd_ctx* ctx, const kevd_calib_job* jobs, int n_jobs,
         calibrate_queue_kernel<<<ctx->num_sms, kPtThreads, smem, s>>>(dj, di, 0, n_items, dc, counter, partial);
         KEVD_LAUNCH(ctx);
     }
-    calibrate_queue_reduce_kernel<<<n_jobs, 64, 0, s>>>(dj, n_jobs, partial, out);
+    calibrate_queue_reduce_kernel<<<n_jobs, kReduceSlices * kMaxScalesB, 0, s>>>(dj, partial, out);
     KEVD_LAUNCH(ctx);
     std::vector<double> hout((size_t)n_jobs * kMaxScalesB);
     KEVD_CUDA(ctx, cudaMemcpyAsync(hout.data(), out, hout.size() * sizeof(double), cudaMemcpyDeviceToHost, s));

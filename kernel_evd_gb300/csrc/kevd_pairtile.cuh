@@ -112,7 +112,7 @@ __device__ __forceinline__ void pt_stage(const float* __restrict__ X, int64_t N,
     const float* src = X + r * d + c0;
     const bool vec = (d & 3) == 0 && ((uintptr_t)X & 15) == 0;
     const int nq = (w + 3) >> 2;
-#pragma unroll 4
+#pragma unroll 8
     for (int q = warp / kSets; q < nq; q += kPar) {
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
         if (in) {
