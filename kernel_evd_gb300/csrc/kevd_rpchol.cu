@@ -35,6 +35,10 @@ int launch_update_tc(kevd_ctx* ctx, float* F, int64_t ldF, int64_t N, int64_t k_
                      double scale, const int64_t* sacc, const float* minv_f, int b, const void* round_state,
                      double* dvec, double* dblk, int* err, cudaStream_t s);
 
+int launch_update_f32(kevd_ctx* ctx, float* F, int64_t ldF, const float* X, int64_t N, int d, double scale,
+                      const int64_t* sacc, const float* minv_f, int b, const RoundState* st, double* dvec, double* dblk,
+                      cudaStream_t s);
+
 bool rpchol_small_supported(int b);
 int64_t rpchol_small_blocks(int64_t N);
 int launch_rpchol_small_init(kevd_ctx* ctx, double* dvec, double* dsub, int64_t N, RoundState* st, cudaStream_t s);
@@ -866,6 +870,9 @@ static int rpchol_impl(kevd_ctx* ctx, const float* X, int64_t N, int d, double s
             if (use_tc) {
                 KEVD_TRY(launch_update_tc(ctx, reinterpret_cast<float*>(F), ldF, N, p->k_max, X, d, scale, sacc,
                                           minv_f, b, rs, dvec, dblk, tc_err, s));
+            } else if constexpr (sizeof(T) == 4) {
+                ProfScope ps(ctx, "rp_update", s);
+                KEVD_TRY(launch_update_f32(ctx, (float*)F, ldF, X, N, d, scale, sacc, minv_f, b, rs, dvec, dblk, s));
             } else {
                 ProfScope ps(ctx, "rp_update", s);
                 for (int g = 0; g < n_groups; ++g) {
