@@ -54,10 +54,9 @@ int launch_rpchol_small_update(kevd_ctx* ctx, double* F, int64_t ldF, const floa
 constexpr int kRowBlock = 128;   // rows per update CTA (= rows per d partial sum)
 constexpr int kMaxBlock = 512;   // proposals per round (the reference's default BLK, ks_arpclm.cu:38)
 constexpr int kGroup = 64;       // accepted columns per update pass: a round with more runs several passes
-constexpr int kSmallBlock = 64;  // rounds up to this size factor their block in shared memory
-constexpr int kFactorThreads = 256;   // rp_factor_kernel: 16 x 16 threads over the trailing update
+constexpr int kSmallBlock = 128; // rounds up to this size factor their block in shared memory
+constexpr int kFactorThreads = 512;   // rp_factor_kernel: warp 0 decides, 15 warps update rows
 constexpr int kBigFactorThreads = 1024;   // rp_factor_big_kernel: 32 x 32 threads
-static_assert(kFactorThreads == 256 && kSmallBlock * kSmallBlock % kFactorThreads == 0, "factor thread layout");
 constexpr int kColChunk = 32;    // F columns per hgram CTA
 constexpr int kFeat = 64;        // features staged at a time by the SIMT update
 constexpr int kSampleThreads = 1024;
@@ -342,10 +341,27 @@ rp_hgram_kernel(const T* __restrict__ F, int64_t ldF, const float* __restrict__ 
 }
 
 // ---- accept / reject, Cholesky, inverse of the compacted factor ------------
-// ks_arpclm.cu:305-408.  H lives in shared memory; accepted columns are
-// overwritten in place by the Cholesky column (only accepted columns are
-// read back).  Minv (b x b, row-major [a][e], zeros above the diagonal).
-__global__ void __launch_bounds__(256)
+// ks_arpclm.cu:305-408.  One CTA; the b x b matrix lives in shared memory (b <=
+// 32 Q).  An accepted proposal i (the m-th) with f = 1 / sqrt(H_ii) makes the
+// scaled column l_j = H_ji f; right of it the trailing update is H_jk -= l_j l_k,
+// and left of it, where the columns of accepted proposals have been used up, the
+// same matrix collects S_jp = sum_e L_je Minv_ep, the sums of the forward
+// substitution: row i of S gives row m of the inverse, Minv_mp = -f S_ip,
+// Minv_mi = f, and S_jp += l_j Minv_mp.  So a step is one rank-1 update of the
+// rows below i by v = (Minv_m, f, -l), with two barriers.
+//
+// What bounds a step is the FP64 pipe (2 lanes per clock on the one SM) and the
+// chain decision -> 1 / sqrt -> scaled column.  Warp 0 keeps the diagonal in
+// registers, tests all proposals at once (a rejected one costs nothing), and
+// forms the next step's f while the other warps update; with every warp taking
+// every decision and square root, one thread per column substituting forward at
+// the end, and one load in flight per element of H, a round took 258 us at b = 64
+// and 100 us at b = 32; now 104 and 38 us (N = 2M, k = 2000).
+//
+// Minv is b x b, row-major [a][e], zeros above the diagonal and beyond the
+// accepted count.
+template <int Q>
+__global__ void __launch_bounds__(kFactorThreads)
 rp_factor_kernel(const double* __restrict__ kss, const double* __restrict__ hpart, int b,
                  int round, uint64_t seed, const double* __restrict__ uniforms, double tol,
                  double floor_rel, int64_t k_max, const int64_t* __restrict__ props, RoundState* st,
@@ -353,115 +369,158 @@ rp_factor_kernel(const double* __restrict__ kss, const double* __restrict__ hpar
                  int64_t* __restrict__ sacc, int64_t* __restrict__ piv,
                  int32_t* __restrict__ hm) {
     if (st->done) return;
-    extern __shared__ double H[];         // b x b, the b x b inverse being formed, the compacted factor
-    double* MS = H + b * b;
-    double* LC = MS + b * b;
-    __shared__ double H0[kSmallBlock];
-    __shared__ double us[kSmallBlock];    // the round's acceptance uniforms
-    __shared__ double kfl[kSmallBlock];   // acceptance floor per proposal (0 in the FP64 form)
-    __shared__ int accpos[kSmallBlock];
-    const int tid = threadIdx.x;
+    constexpr int B = 32 * Q;
+    extern __shared__ double A[];     // b x (b + 1)
+    __shared__ double thr[B], l[B], v[B];
+    __shared__ int accpos[B];
+    __shared__ double s_f;
+    __shared__ int s_i;
+    const int P = b + 1;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int64_t r = st->rank;
     const int nz = (int)((r + kColChunk - 1) / kColChunk);
-    {
-        // 256 threads x 16 elements (b <= 64): the 16 chains of a thread advance
-        // together over the column chunks, so 16 loads are in flight per step;
-        // each element still subtracts its chunks in increasing order
-        constexpr int kPer = kSmallBlock * kSmallBlock / 256;
-        double v[kPer];
+    // H = K(S',S') - sum of the column chunks' products, each element in chunk
+    // order; kPer elements per thread and four chunks ahead keep 32 loads in flight
+    constexpr int kPer = 8;
+    for (int e0 = tid; e0 < b * b; e0 += kPer * kFactorThreads) {
+        double x[kPer];
 #pragma unroll
         for (int j = 0; j < kPer; ++j) {
-            const int e = tid + 256 * j;
-            v[j] = (e < b * b) ? kss[e] : 0.0;
+            const int e = e0 + j * kFactorThreads;
+            x[j] = (e < b * b) ? kss[e] : 0.0;
         }
-        for (int z = 0; z < nz; ++z) {
-            const double* hz = hpart + (int64_t)z * b * b;
+        int z = 0;
+        for (; z + 4 <= nz; z += 4) {
+            double y[4][kPer];
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+#pragma unroll
+                for (int j = 0; j < kPer; ++j) {
+                    const int e = e0 + j * kFactorThreads;
+                    y[q][j] = (e < b * b) ? hpart[(int64_t)(z + q) * b * b + e] : 0.0;
+                }
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+#pragma unroll
+                for (int j = 0; j < kPer; ++j) x[j] -= y[q][j];
+        }
+        for (; z < nz; ++z)
 #pragma unroll
             for (int j = 0; j < kPer; ++j) {
-                const int e = tid + 256 * j;
-                if (e < b * b) v[j] -= hz[e];
+                const int e = e0 + j * kFactorThreads;
+                if (e < b * b) x[j] -= hpart[(int64_t)z * b * b + e];
             }
-        }
 #pragma unroll
         for (int j = 0; j < kPer; ++j) {
-            const int e = tid + 256 * j;
-            if (e < b * b) H[e] = v[j];
+            const int e = e0 + j * kFactorThreads;
+            if (e < b * b) {
+                A[(e / b) * P + e % b] = x[j];
+                minv[e] = 0.0;
+                minv_f[e] = 0.f;
+            }
         }
     }
     __syncthreads();
-    for (int p = tid; p < b; p += blockDim.x) {
-        H0[p] = H[p * b + p];
-        kfl[p] = floor_rel * kss[p * b + p];
-        us[p] = uniforms ? uniforms[((int64_t)round * 2 + 1) * b + p] : philox_uniform(seed, (uint32_t)round, 1u, (uint32_t)p);
+    // accepted iff H0_ii u < H_ii, H_ii > tol and H_ii above the rounding floor
+    if (tid < b) {
+        const double u = uniforms ? uniforms[((int64_t)round * 2 + 1) * b + tid]
+                                  : philox_uniform(seed, (uint32_t)round, 1u, (uint32_t)tid);
+        thr[tid] = fmax(fmax(A[tid * P + tid] * u, tol), floor_rel * kss[tid * b + tid]);
     }
-    const int64_t cap = k_max - r;
-    // Every thread takes the same decisions (H_ii is final once the previous
-    // accepted step's trailing update has passed its barrier), so a rejected
-    // proposal costs no barrier and an accepted one a single barrier.  The
-    // trailing update forms the scaled column l_j = H_ji f in registers, the
-    // same product that is stored into column i after the barrier (the next
-    // steps never touch column i, so that write overlaps them).
-    int m = 0;
     __syncthreads();
-    for (int i = 0; i < b; ++i) {
-        const double hii = H[i * b + i];
-        const bool acc = (m < cap) && (H0[i] * us[i] < hii) && (hii > tol) && (hii > kfl[i]);
-        if (!acc) continue;
+    const int cap = (int)min((int64_t)b, k_max - r);
+    int m = 0;
+    unsigned acc[Q];    // accepted proposals so far, 32 per word
+    double dg[Q];       // warp 0: the diagonal, proposal lane + 32 q
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+        acc[q] = 0u;
+        dg[q] = (warp == 0 && lane + 32 * q < b) ? A[(lane + 32 * q) * P + lane + 32 * q] : 0.0;
+    }
+    // warp 0: the first acceptable proposal from i0 on (mm accepted before it)
+    auto decide = [&](int i0, int mm) {
+        int i = -1;
+        double hii = 1.0;
+#pragma unroll
+        for (int q = Q - 1; q >= 0; --q) {
+            const int p = lane + 32 * q;
+            const unsigned ok = __ballot_sync(0xffffffffu, p >= i0 && p < b && mm < cap && dg[q] > thr[min(p, b - 1)]);
+            if (ok) {
+                i = 32 * q + __ffs(ok) - 1;
+                hii = __shfl_sync(0xffffffffu, dg[q], __ffs(ok) - 1);
+            }
+        }
+        const double f = rsqrt(hii);
+        if (lane == 0) {
+            s_i = i;
+            s_f = f;
+        }
+    };
+    if (warp == 0) decide(0, 0);
+    __syncthreads();
+    while (s_i >= 0) {
+        const int i = s_i;
+        const double f = s_f;
+        if (tid < b) {
+            const int c = tid;
+            double vc = 0.0;
+            if (c > i) {
+                vc = -(A[c * P + i] * f);
+            } else if (c == i || (acc[Q == 1 ? 0 : c >> 5] >> (c & 31) & 1u)) {
+                vc = c == i ? f : -(f * A[i * P + c]);
+                int t = 0;   // accepted before c
+#pragma unroll
+                for (int q = 0; q < Q; ++q)
+                    t += __popc(q < (c >> 5) ? acc[q] : q == (c >> 5) ? acc[q] & ((1u << (c & 31)) - 1u) : 0u);
+                minv[m * b + t] = vc;
+                minv_f[m * b + t] = (float)vc;
+            }
+            l[c] = c > i ? -vc : 0.0;
+            v[c] = vc;
+        }
         if (tid == 0) accpos[m] = i;
         ++m;
-        const double f = 1.0 / sqrt(hii);
-        // trailing update of the lower triangle, 16 x 16 threads over (jj, kk)
-        for (int jj = i + 1 + (tid >> 4); jj < b; jj += 16) {
-            const double lj = H[jj * b + i] * f;
-            for (int kk = i + 1 + (tid & 15); kk <= jj; kk += 16) {
-                const double lk = H[kk * b + i] * f;
-                H[jj * b + kk] -= lj * lk;
+#pragma unroll
+        for (int q = 0; q < Q; ++q)
+            if (q == i >> 5) acc[q] |= 1u << (i & 31);
+        __syncthreads();
+        if (warp == 0) {
+#pragma unroll
+            for (int q = 0; q < Q; ++q) {
+                const int p = lane + 32 * q;
+                if (p > i && p < b) dg[q] = fma(-l[p], l[p], dg[q]);
+            }
+            decide(i + 1, m);
+        } else {
+            double vq[Q];
+#pragma unroll
+            for (int q = 0; q < Q; ++q) vq[q] = lane + 32 * q < b ? v[lane + 32 * q] : 0.0;
+            for (int jj = i + warp; jj < b; jj += kFactorThreads / 32 - 1) {
+                const double lj = l[jj];
+#pragma unroll
+                for (int q = 0; q < Q; ++q) {
+                    const int c = lane + 32 * q;
+                    if (32 * q < jj && c < b)   // columns past jj are never read
+                        A[jj * P + c] = fma(lj, vq[q], c == i ? 0.0 : A[jj * P + c]);
+                }
             }
         }
         __syncthreads();
-        for (int j = i + tid; j < b; j += blockDim.x) H[j * b + i] *= f;
     }
-    __syncthreads();   // the last scaled column is written
-    const int nacc = m;
-    // forward substitution, one column per thread, in shared memory (the
-    // sequential dot products read what the same thread wrote a step earlier)
-    // on the compacted factor LC (no index indirection inside the chains)
-    for (int e = tid; e < b * b; e += blockDim.x) {
-        MS[e] = 0.0;
-        const int a = e / b, c = e - a * b;
-        LC[e] = (a < nacc && c < nacc) ? H[accpos[a] * b + accpos[c]] : 0.0;
-    }
-    __syncthreads();
-    if (tid < nacc) {
-        const int t = tid;
-        MS[t * b + t] = 1.0 / LC[t * b + t];
-        for (int a = t + 1; a < nacc; ++a) {
-            const double* la = LC + a * b;
-            double s = 0.0;
-            for (int e = t; e < a; ++e) s += la[e] * MS[e * b + t];
-            MS[a * b + t] = -s / la[a];
-        }
-    }
-    __syncthreads();
-    for (int e = tid; e < b * b; e += blockDim.x) {
-        minv[e] = MS[e];
-        minv_f[e] = (float)MS[e];
-    }
-    if (tid < nacc) {
+    if (tid < m) {
         const int64_t sp = props[accpos[tid]];
         sacc[tid] = sp;
         piv[r + tid] = sp;
     }
     if (tid == 0) {
         st->r_old = r;
-        st->nacc = nacc;
-        st->rank = r + nacc;
-        hm[round] = nacc;
+        st->nacc = m;
+        st->rank = r + m;
+        hm[round] = m;
     }
 }
 
-// Accept / reject, Cholesky and inverse for 64 < b <= kMaxBlock: the steps and
-// the per-element operation order of rp_factor_kernel, with H, the compacted
+// Accept / reject, Cholesky and inverse for kSmallBlock < b <= kMaxBlock: with H, the compacted
 // factor LC and the inverse MS in a global workspace (b^2 doubles each,
 // L2-resident) instead of shared memory, and 32 x 32 threads over the
 // trailing update.  __syncthreads orders the CTA's global accesses as it does
@@ -806,19 +865,21 @@ static int rpchol_impl(kevd_ctx* ctx, const float* X, int64_t N, int d, double s
     }
 
     const bool big = b > kSmallBlock;
-    const size_t fsm = big ? 0 : (size_t)3 * b * b * sizeof(double);
+    const size_t fsm = big ? 0 : (size_t)b * (b + 1) * sizeof(double);
+    auto factor = b <= 32 ? &rp_factor_kernel<1> : b <= 64 ? &rp_factor_kernel<2> : &rp_factor_kernel<4>;
     double* hbig = nullptr;   // H, the compacted factor and the inverse of a large block
     if (big) {
         hbig = arena_get<double>(ctx, "rp.hbig", (size_t)3 * b * b, &st);
         if (st != KEVD_OK) return st;
     } else {
-        KEVD_CUDA(ctx, raise_smem_limit(reinterpret_cast<const void*>(&rp_factor_kernel), (int)std::max(fsm, (size_t)1024)));
+        KEVD_CUDA(ctx, raise_smem_limit(reinterpret_cast<const void*>(factor), (int)std::max(fsm, (size_t)1024)));
     }
     const size_t hsm = hgram_smem<T>(b);
     KEVD_CUDA(ctx, raise_smem_limit(reinterpret_cast<const void*>(&rp_hgram_kernel<T>), (int)hsm));
     const int n_groups = (b + kGroup - 1) / kGroup;
     const size_t usm = update_smem<T>(d);
-    KEVD_CUDA(ctx, raise_smem_limit(reinterpret_cast<const void*>(&rp_update_kernel<T>), (int)usm));
+    if constexpr (sizeof(T) == 8)
+        KEVD_CUDA(ctx, raise_smem_limit(reinterpret_cast<const void*>(&rp_update_kernel<T>), (int)usm));
     int* done_h = static_cast<int*>(ctx->pinned);
     // FP32 factors take the tensor-core residual update when the layout allows
     // TMA and the kernel is not nearly diagonal (kernel_density_kernel)
@@ -862,7 +923,7 @@ static int rpchol_impl(kevd_ctx* ctx, const float* X, int64_t N, int d, double s
                                                                           sacc, piv, hm, hbig, hbig + (size_t)b * b,
                                                                           hbig + (size_t)2 * b * b);
                 else
-                    rp_factor_kernel<<<1, kFactorThreads, fsm, s>>>(kss, hpart, b, round, p->seed, unif, p->tol,
+                    factor<<<1, kFactorThreads, fsm, s>>>(kss, hpart, b, round, p->seed, unif, p->tol,
                                                                     floor_rel, p->k_max, props, rs, minv, minv_f, sacc,
                                                                     piv, hm);
                 KEVD_LAUNCH(ctx);
