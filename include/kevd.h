@@ -217,11 +217,11 @@ int kevd_rpchol(kevd_ctx* ctx, const float* X, int64_t N, int32_t d,
 /* Many mixed-precision factorisations at once (no reference counterpart).
  * Each job has its own X (device), FP32 factor F (device, N x ldF) and seed;
  * piv (host, k_max entries) receives the pivots and result the rank, rounds
- * and trace error.  use_graph != 0: the round loops of all jobs are captured
- * as parallel branches of one CUDA graph (forked from stream, joined back)
- * and launched once; every job runs max_rounds rounds on the device (kernels
- * return at once after the stop).  use_graph == 0: the same work is issued on
- * one stream per job. */
+ * and trace error.  use_graph != 0: four rounds of every job are captured as
+ * parallel branches of one CUDA graph, which is launched on stream until all
+ * jobs have stopped (kernels of a stopped job return at once).  use_graph == 0:
+ * the same rounds are issued on one stream per job.  The jobs' workspaces stay
+ * with ctx when they hold at most 1 GiB. */
 typedef struct {
     const float* X;
     int64_t N;

@@ -276,9 +276,9 @@ def factor_from_linv(ctx: Context, X: torch.Tensor, scale: float, piv, Linv: np.
 def rpcholesky_batched(ctx: Context, Xs, scales, k_max, block=32, seeds=None, max_rounds=None,
                        use_graph: bool = True) -> list:
     """Mixed-precision block RPCholesky of many datasets at once
-    (``kevd_rpchol_batched``): with ``use_graph`` every job's round loop is a
-    branch of one captured CUDA graph launched once.  Returns one
-    Factorization per job (FP32 factor)."""
+    (``kevd_rpchol_batched``): with ``use_graph`` four rounds of every job are
+    branches of one captured CUDA graph, launched until all jobs have stopped.
+    Returns one Factorization per job (FP32 factor)."""
     n = len(Xs)
     k_max = list(k_max) if hasattr(k_max, "__len__") else [int(k_max)] * n
     block = list(block) if hasattr(block, "__len__") else [int(block)] * n

@@ -144,6 +144,7 @@ void kevd_ctx_destroy(kevd_ctx* ctx) {
     cudaSetDevice(ctx->device);
     resolve_profile(ctx);
     for (cudaEvent_t e : ctx->pool) cudaEventDestroy(e);
+    free_batch_pool(ctx);
     ctx->arena.release();
     if (ctx->blas) cublasDestroy(ctx->blas);
     if (ctx->solver) cusolverDnDestroy(ctx->solver);

@@ -57,6 +57,7 @@ struct kevd_ctx {
     cublasHandle_t blas = nullptr;
     cusolverDnHandle_t solver = nullptr;
     kevd::Arena arena;
+    void* batch_pool = nullptr;  // workspaces of batched factorisations (kevd_rpchol.cu)
     void* pinned = nullptr;  // small pinned host staging area
     size_t pinned_bytes = 0;
     std::string last_error;
@@ -157,9 +158,18 @@ class ProfScope {
     cudaEvent_t a_ = nullptr;
 };
 
+void free_batch_pool(kevd_ctx* ctx);   // kevd_rpchol.cu
+
 template <typename T>
 T* arena_get(kevd_ctx* ctx, const char* name, size_t count, int* st) {
-    return static_cast<T*>(ctx->arena.get(name, count * sizeof(T), st));
+    const int before = *st;
+    T* p = static_cast<T*>(ctx->arena.get(name, count * sizeof(T), st));
+    if (!p && ctx->batch_pool) {   // out of memory: give the batch's workspaces back first
+        *st = before;
+        free_batch_pool(ctx);
+        p = static_cast<T*>(ctx->arena.get(name, count * sizeof(T), st));
+    }
+    return p;
 }
 
 inline cudaStream_t as_stream(void* s) { return static_cast<cudaStream_t>(s); }

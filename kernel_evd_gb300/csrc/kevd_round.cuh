@@ -11,7 +11,7 @@ struct RoundState {
     int32_t nacc;    // accepted this round
     int32_t done;    // set once the factorisation has stopped
     int32_t rounds;  // rounds executed
-    int32_t pad;
+    int32_t cur;     // index of the round being worked on
     double total;    // sum of d after the last update
 };
 

@@ -31,6 +31,7 @@
 namespace kevd {
 
 bool update_tc_supported(const float* F, int64_t ldF, int d);
+int reserve_update_tc(kevd_ctx* ctx, int64_t N, int64_t k_max);
 int launch_update_tc(kevd_ctx* ctx, float* F, int64_t ldF, int64_t N, int64_t k_max, const float* X, int d,
                      double scale, const int64_t* sacc, const float* minv_f, int b, const void* round_state,
                      double* dvec, double* dblk, int* err, cudaStream_t s);
@@ -70,15 +71,6 @@ constexpr int kSampleThreads = 1024;
 // error, the mean residual diagonal, has fallen below the same level.  The
 // FP64 form keeps the reference's tolerance alone (ks_arpclm.cu:329-331).
 constexpr double kMixedFloor = 16.0 / 16777216.0;
-
-// Host side of a capture-safe factorisation: no host read inside the round
-// loop (all max_rounds rounds are enqueued; the kernels return at once after
-// the stop), results copied to these pinned buffers at the end.
-struct RpcholDeferred {
-    RoundState* state_h;
-    int* tcerr_h;
-    int64_t* piv_h;
-};
 
 // Kernel values of a fixed pseudo-random sample of kDensityPairs pairs (i, j),
 // i != j, counted when K(i, j) >= 2^-24.  A factorisation whose kernel is
@@ -150,6 +142,7 @@ __global__ void rp_init_kernel(double* __restrict__ d, double* __restrict__ dblk
         st->nacc = 0;
         st->done = 0;
         st->rounds = 0;
+        st->cur = 0;
         st->total = (double)N;
     }
 }
@@ -159,16 +152,18 @@ __global__ void rp_init_kernel(double* __restrict__ d, double* __restrict__ dblk
 // cumsum(d)[i] >= u * sum(d), else N - 1.  The prefix is hierarchical: a scan
 // over per-thread chunks of the block sums, a sequential walk over the chunk,
 // then a warp scan inside the 128-row block.  Also records the trace error of
-// the previous round and decides the stop.
+// the previous round and decides the stop (the closing call, after the last
+// round, always stops).
 __global__ void __launch_bounds__(kSampleThreads)
 rp_sample_kernel(const double* __restrict__ d, const double* __restrict__ dblk, int64_t N,
-                 int64_t nblk, int round, int b, uint64_t seed,
+                 int64_t nblk, int closing, int b, uint64_t seed,
                  const double* __restrict__ uniforms, int64_t* __restrict__ props,
                  RoundState* st, int64_t k_max, int max_rounds, double err_target,
                  double err_floor, double* __restrict__ err) {
     __shared__ double incl[kSampleThreads];
     __shared__ int s_stop;
     if (st->done) return;
+    const int round = st->cur;
     const int tid = threadIdx.x;
     const int64_t chunk = (nblk + kSampleThreads - 1) / kSampleThreads;
     const int64_t c0 = min(nblk, (int64_t)tid * chunk), c1 = min(nblk, c0 + chunk);
@@ -187,7 +182,7 @@ rp_sample_kernel(const double* __restrict__ d, const double* __restrict__ dblk, 
         const double e = total / (double)N;
         if (round > 0) err[round - 1] = e;
         st->total = total;
-        const bool stop = (round >= max_rounds) || (st->rank >= k_max) ||
+        const bool stop = closing || (round >= max_rounds) || (st->rank >= k_max) ||
                           (err_target > 0.0 && round > 0 && e <= err_target) ||
                           (err_floor > 0.0 && round > 0 && e <= err_floor);
         if (stop) {
@@ -363,7 +358,7 @@ rp_hgram_kernel(const T* __restrict__ F, int64_t ldF, const float* __restrict__ 
 template <int Q>
 __global__ void __launch_bounds__(kFactorThreads)
 rp_factor_kernel(const double* __restrict__ kss, const double* __restrict__ hpart, int b,
-                 int round, uint64_t seed, const double* __restrict__ uniforms, double tol,
+                 uint64_t seed, const double* __restrict__ uniforms, double tol,
                  double floor_rel, int64_t k_max, const int64_t* __restrict__ props, RoundState* st,
                  double* __restrict__ minv, float* __restrict__ minv_f,
                  int64_t* __restrict__ sacc, int64_t* __restrict__ piv,
@@ -377,6 +372,7 @@ rp_factor_kernel(const double* __restrict__ kss, const double* __restrict__ hpar
     __shared__ int s_i;
     const int P = b + 1;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int round = st->cur;
     const int64_t r = st->rank;
     const int nz = (int)((r + kColChunk - 1) / kColChunk);
     // H = K(S',S') - sum of the column chunks' products, each element in chunk
@@ -516,6 +512,7 @@ rp_factor_kernel(const double* __restrict__ kss, const double* __restrict__ hpar
         st->r_old = r;
         st->nacc = m;
         st->rank = r + m;
+        st->cur = round + 1;
         hm[round] = m;
     }
 }
@@ -527,7 +524,7 @@ rp_factor_kernel(const double* __restrict__ kss, const double* __restrict__ hpar
 // its shared ones.
 __global__ void __launch_bounds__(kBigFactorThreads)
 rp_factor_big_kernel(const double* __restrict__ kss, const double* __restrict__ hpart, int b,
-                     int round, uint64_t seed, const double* __restrict__ uniforms, double tol,
+                     uint64_t seed, const double* __restrict__ uniforms, double tol,
                      double floor_rel, int64_t k_max, const int64_t* __restrict__ props, RoundState* st,
                      double* __restrict__ minv, float* __restrict__ minv_f,
                      int64_t* __restrict__ sacc, int64_t* __restrict__ piv,
@@ -540,6 +537,7 @@ rp_factor_big_kernel(const double* __restrict__ kss, const double* __restrict__ 
     __shared__ int s_dec, s_m;
     const int tid = threadIdx.x;
     const int nt = blockDim.x;
+    const int round = st->cur;
     const int64_t r = st->rank;
     const int nz = (int)((r + kColChunk - 1) / kColChunk);
     for (int e = tid; e < b * b; e += nt) {
@@ -607,6 +605,7 @@ rp_factor_big_kernel(const double* __restrict__ kss, const double* __restrict__ 
         st->r_old = r;
         st->nacc = nacc;
         st->rank = r + nacc;
+        st->cur = round + 1;
         hm[round] = nacc;
     }
 }
@@ -822,160 +821,185 @@ static size_t update_smem(int d) {
            (size_t)kGroup * (kGroup + 1) * sizeof(T);
 }
 
+// One factorisation's buffers and launches.  setup() allocates (the sizes do not
+// depend on the round count), init() starts the round state, round() enqueues one
+// round (its index is in the round state, so the launches of every round are the
+// same), closing() records the last round's error.
+template <typename T>
+struct RpRun {
+    kevd_ctx* ctx;
+    const float* X;
+    int64_t N;
+    int d;
+    double scale;
+    kevd_rpchol_params p;
+    T* F;
+    int64_t ldF;
+    bool tc_allowed;
+
+    int b = 0, n_split = 0;
+    int64_t nblk = 0;
+    bool small = false, use_tc = false;
+    double floor_rel = 0.0;
+    double *dvec = nullptr, *dblk = nullptr, *hpart = nullptr, *kss = nullptr, *minv = nullptr, *err = nullptr,
+           *unif = nullptr, *hbig = nullptr;
+    RoundState* rs = nullptr;
+    int64_t *props = nullptr, *sacc = nullptr, *piv = nullptr;
+    float* minv_f = nullptr;
+    int32_t* hm = nullptr;
+    int* tc_err = nullptr;
+    size_t fsm = 0, hsm = 0, usm = 0;
+
+    int setup() {
+        b = p.block;
+        floor_rel = sizeof(T) == 4 ? kMixedFloor : 0.0;
+        nblk = (N + kRowBlock - 1) / kRowBlock;
+        n_split = (int)((p.k_max + kColChunk - 1) / kColChunk);
+        // few proposals in FP64: two kernels a round that touch the accepted columns
+        // only (kevd_rpchol_small.cu).  The FP32 form keeps the general kernels: a
+        // pivot sequence follows every rounding of its residual diagonal.
+        small = sizeof(T) == 8 && rpchol_small_supported(b);
+        int st = KEVD_OK;
+        dvec = arena_get<double>(ctx, "rp.d", N, &st);
+        dblk = arena_get<double>(ctx, "rp.dblk", small ? rpchol_small_blocks(N) : nblk, &st);
+        rs = arena_get<RoundState>(ctx, "rp.state", 1, &st);
+        props = arena_get<int64_t>(ctx, "rp.props", kMaxBlock, &st);
+        sacc = arena_get<int64_t>(ctx, "rp.sacc", kMaxBlock, &st);
+        piv = arena_get<int64_t>(ctx, "rp.piv", p.k_max, &st);
+        hpart = arena_get<double>(ctx, "rp.hpart", (size_t)std::max(n_split, 1) * b * b, &st);
+        kss = arena_get<double>(ctx, "rp.kss", (size_t)b * b, &st);
+        minv = arena_get<double>(ctx, "rp.minv", (size_t)b * b, &st);
+        minv_f = arena_get<float>(ctx, "rp.minvf", (size_t)b * b, &st);
+        err = arena_get<double>(ctx, "rp.err", p.max_rounds, &st);
+        hm = arena_get<int32_t>(ctx, "rp.hm", p.max_rounds, &st);
+        tc_err = arena_get<int>(ctx, "rp.tcerr", 1, &st);
+        if (p.uniforms) unif = arena_get<double>(ctx, "rp.unif", (size_t)p.max_rounds * 2 * b, &st);
+        // H, the compacted factor and the inverse of a large block
+        if (b > kSmallBlock) hbig = arena_get<double>(ctx, "rp.hbig", (size_t)3 * b * b, &st);
+        if (st != KEVD_OK) return st;
+        fsm = b > kSmallBlock ? 0 : (size_t)b * (b + 1) * sizeof(double);
+        if (b <= kSmallBlock)
+            KEVD_CUDA(ctx, raise_smem_limit(reinterpret_cast<const void*>(factor()), std::max(fsm, (size_t)1024)));
+        hsm = hgram_smem<T>(b);
+        KEVD_CUDA(ctx, raise_smem_limit(reinterpret_cast<const void*>(&rp_hgram_kernel<T>), (int)hsm));
+        usm = update_smem<T>(d);
+        if constexpr (sizeof(T) == 8)
+            KEVD_CUDA(ctx, raise_smem_limit(reinterpret_cast<const void*>(&rp_update_kernel<T>), (int)usm));
+        // FP32 factors take the tensor-core residual update when the layout allows
+        // TMA and the kernel is not nearly diagonal (kernel_density_kernel)
+        use_tc = sizeof(T) == 4 && tc_allowed && update_tc_supported(reinterpret_cast<const float*>(F), ldF, d);
+        if (use_tc) KEVD_TRY(reserve_update_tc(ctx, N, p.k_max));
+        return KEVD_OK;
+    }
+
+    int init(cudaStream_t s) {
+        if (unif)
+            KEVD_CUDA(ctx, cudaMemcpyAsync(unif, p.uniforms, (size_t)p.max_rounds * 2 * b * sizeof(double),
+                                           cudaMemcpyHostToDevice, s));
+        KEVD_CUDA(ctx, cudaMemsetAsync(err, 0, p.max_rounds * sizeof(double), s));
+        KEVD_CUDA(ctx, cudaMemsetAsync(hm, 0, p.max_rounds * sizeof(int32_t), s));
+        KEVD_CUDA(ctx, cudaMemsetAsync(tc_err, 0, sizeof(int), s));
+        if (small) return launch_rpchol_small_init(ctx, dvec, dblk, N, rs, s);
+        rp_init_kernel<<<ctx->num_sms * 4, 256, 0, s>>>(dvec, dblk, N, nblk, rs);
+        KEVD_LAUNCH(ctx);
+        return KEVD_OK;
+    }
+
+    // `index` is read by the two-kernel round alone
+    int round(int index, cudaStream_t s) {
+        if (small) {
+            KEVD_TRY(propose_small(index, b, p.max_rounds, s));
+            return launch_rpchol_small_update(ctx, (double*)F, ldF, X, N, d, scale, sacc, minv, b, rs, dvec, dblk, s);
+        }
+        {
+            ProfScope ps(ctx, "rp_sample", s);
+            sample(0, b, s);
+            KEVD_LAUNCH(ctx);
+        }
+        {
+            ProfScope ps(ctx, "rp_hgram", s);
+            const int n_kss = 32;   // CTAs sharing the FP64 K(S', S') block
+            rp_hgram_kernel<T><<<n_split + n_kss, 256, hsm, s>>>(F, ldF, X, d, scale, props, b, n_split, rs, hpart, kss);
+            KEVD_LAUNCH(ctx);
+        }
+        {
+            ProfScope ps(ctx, "rp_factor", s);
+            if (hbig)
+                rp_factor_big_kernel<<<1, kBigFactorThreads, 0, s>>>(kss, hpart, b, p.seed, unif, p.tol, floor_rel,
+                                                                      p.k_max, props, rs, minv, minv_f, sacc, piv, hm,
+                                                                      hbig, hbig + (size_t)b * b,
+                                                                      hbig + (size_t)2 * b * b);
+            else
+                factor()<<<1, kFactorThreads, fsm, s>>>(kss, hpart, b, p.seed, unif, p.tol, floor_rel, p.k_max, props,
+                                                        rs, minv, minv_f, sacc, piv, hm);
+            KEVD_LAUNCH(ctx);
+        }
+        if (use_tc)
+            return launch_update_tc(ctx, reinterpret_cast<float*>(F), ldF, N, p.k_max, X, d, scale, sacc, minv_f, b, rs,
+                                    dvec, dblk, tc_err, s);
+        ProfScope ps(ctx, "rp_update", s);
+        if constexpr (sizeof(T) == 4) {
+            KEVD_TRY(launch_update_f32(ctx, (float*)F, ldF, X, N, d, scale, sacc, minv_f, b, rs, dvec, dblk, s));
+        } else {
+            for (int g = 0; g < (b + kGroup - 1) / kGroup; ++g) {
+                rp_update_kernel<T><<<(int)nblk, 256, usm, s>>>(F, ldF, X, N, d, scale, sacc, minv, minv_f, b, rs, dvec,
+                                                               dblk, g);
+                KEVD_LAUNCH(ctx);
+            }
+        }
+        return KEVD_OK;
+    }
+
+    int closing(int rounds, cudaStream_t s) {
+        if (small) return propose_small(rounds, 0, rounds, s);
+        sample(1, 0, s);
+        KEVD_LAUNCH(ctx);
+        return KEVD_OK;
+    }
+
+    auto factor() const { return b <= 32 ? &rp_factor_kernel<1> : b <= 64 ? &rp_factor_kernel<2> : &rp_factor_kernel<4>; }
+    void sample(int closing, int nb, cudaStream_t s) {
+        rp_sample_kernel<<<1, kSampleThreads, 0, s>>>(dvec, dblk, N, nblk, closing, nb, p.seed, unif, props, rs, p.k_max,
+                                                      p.max_rounds, p.err_target, floor_rel, err);
+    }
+    int propose_small(int round, int nb, int limit, cudaStream_t s) {
+        return launch_rpchol_small_propose(ctx, (const double*)F, ldF, X, N, d, scale, dvec, dblk, round, nb, p.seed, unif,
+                                           p.tol, p.k_max, limit, p.err_target, rs, minv, sacc, piv, err, hm, s);
+    }
+};
+
 template <typename T>
 static int rpchol_impl(kevd_ctx* ctx, const float* X, int64_t N, int d, double scale,
                        const kevd_rpchol_params* p, T* F, int64_t ldF, int64_t* piv_h,
-                       double* err_h, int32_t* hm_h, kevd_rpchol_result* res, cudaStream_t s,
-                       RpcholDeferred* defer = nullptr, bool tc_allowed = true) {
-    const int b = p->block;
-    const double floor_rel = sizeof(T) == 4 ? kMixedFloor : 0.0;
-    const int64_t nblk = (N + kRowBlock - 1) / kRowBlock;
-    const int n_split = (int)((p->k_max + kColChunk - 1) / kColChunk);
-    const int n_kss = 32;   // CTAs sharing the FP64 K(S', S') block (one element per thread, same order)
-    int st = KEVD_OK;
-    // few proposals in FP64: two kernels a round that touch the accepted columns
-    // only (kevd_rpchol_small.cu).  The FP32 form keeps the general kernels: a
-    // pivot sequence follows every rounding of its residual diagonal.
-    const bool small = sizeof(T) == 8 && rpchol_small_supported(b);
-    double* dvec = arena_get<double>(ctx, "rp.d", N, &st);
-    double* dblk = arena_get<double>(ctx, "rp.dblk", small ? rpchol_small_blocks(N) : nblk, &st);
-    RoundState* rs = arena_get<RoundState>(ctx, "rp.state", 1, &st);
-    int64_t* props = arena_get<int64_t>(ctx, "rp.props", kMaxBlock, &st);
-    int64_t* sacc = arena_get<int64_t>(ctx, "rp.sacc", kMaxBlock, &st);
-    int64_t* piv = arena_get<int64_t>(ctx, "rp.piv", p->k_max, &st);
-    double* hpart = arena_get<double>(ctx, "rp.hpart", (size_t)std::max(n_split, 1) * b * b, &st);
-    double* kss = arena_get<double>(ctx, "rp.kss", (size_t)b * b, &st);
-    double* minv = arena_get<double>(ctx, "rp.minv", (size_t)b * b, &st);
-    float* minv_f = arena_get<float>(ctx, "rp.minvf", (size_t)b * b, &st);
-    double* err = arena_get<double>(ctx, "rp.err", p->max_rounds, &st);
-    int32_t* hm = arena_get<int32_t>(ctx, "rp.hm", p->max_rounds, &st);
-    double* unif = nullptr;
-    if (p->uniforms) unif = arena_get<double>(ctx, "rp.unif", (size_t)p->max_rounds * 2 * b, &st);
-    if (st != KEVD_OK) return st;
-    if (unif)
-        KEVD_CUDA(ctx, cudaMemcpyAsync(unif, p->uniforms, (size_t)p->max_rounds * 2 * b * sizeof(double),
-                                       cudaMemcpyHostToDevice, s));
-    KEVD_CUDA(ctx, cudaMemsetAsync(err, 0, p->max_rounds * sizeof(double), s));
-    KEVD_CUDA(ctx, cudaMemsetAsync(hm, 0, p->max_rounds * sizeof(int32_t), s));
-    if (small) {
-        KEVD_TRY(launch_rpchol_small_init(ctx, dvec, dblk, N, rs, s));
-    } else {
-        rp_init_kernel<<<ctx->num_sms * 4, 256, 0, s>>>(dvec, dblk, N, nblk, rs);
-        KEVD_LAUNCH(ctx);
-    }
-
-    const bool big = b > kSmallBlock;
-    const size_t fsm = big ? 0 : (size_t)b * (b + 1) * sizeof(double);
-    auto factor = b <= 32 ? &rp_factor_kernel<1> : b <= 64 ? &rp_factor_kernel<2> : &rp_factor_kernel<4>;
-    double* hbig = nullptr;   // H, the compacted factor and the inverse of a large block
-    if (big) {
-        hbig = arena_get<double>(ctx, "rp.hbig", (size_t)3 * b * b, &st);
-        if (st != KEVD_OK) return st;
-    } else {
-        KEVD_CUDA(ctx, raise_smem_limit(reinterpret_cast<const void*>(factor), (int)std::max(fsm, (size_t)1024)));
-    }
-    const size_t hsm = hgram_smem<T>(b);
-    KEVD_CUDA(ctx, raise_smem_limit(reinterpret_cast<const void*>(&rp_hgram_kernel<T>), (int)hsm));
-    const int n_groups = (b + kGroup - 1) / kGroup;
-    const size_t usm = update_smem<T>(d);
-    if constexpr (sizeof(T) == 8)
-        KEVD_CUDA(ctx, raise_smem_limit(reinterpret_cast<const void*>(&rp_update_kernel<T>), (int)usm));
+                       double* err_h, int32_t* hm_h, kevd_rpchol_result* res, cudaStream_t s, bool tc_allowed = true) {
+    RpRun<T> run{ctx, X, N, d, scale, *p, F, ldF, tc_allowed};
+    KEVD_TRY(run.setup());
+    KEVD_TRY(run.init(s));
     int* done_h = static_cast<int*>(ctx->pinned);
-    // FP32 factors take the tensor-core residual update when the layout allows
-    // TMA and the kernel is not nearly diagonal (kernel_density_kernel)
-    const bool use_tc =
-        sizeof(T) == 4 && tc_allowed && update_tc_supported(reinterpret_cast<const float*>(F), ldF, d);
-    int* tc_err = arena_get<int>(ctx, "rp.tcerr", 1, &st);
-    if (st != KEVD_OK) return st;
-    KEVD_CUDA(ctx, cudaMemsetAsync(tc_err, 0, sizeof(int), s));
-    int round = 0;
-    auto propose_small = [&](int rnd, int nb, int limit) {
-        return launch_rpchol_small_propose(ctx, (const double*)F, ldF, X, N, d, scale, dvec, dblk, rnd, nb, p->seed,
-                                           unif, p->tol, p->k_max, limit, p->err_target, rs, minv, sacc, piv, err, hm,
-                                           s);
-    };
     // rounds between two reads of the done flag (each read waits for the stream):
     // a small round is short, and the rounds after the stop return at once
-    const int poll = small ? 16 : 4;
+    const int poll = run.small ? 16 : 4;
+    int round = 0;
     for (; round < p->max_rounds; ++round) {
-        if (small) {
-            KEVD_TRY(propose_small(round, b, p->max_rounds));
-            KEVD_TRY(launch_rpchol_small_update(ctx, (double*)F, ldF, X, N, d, scale, sacc, minv, b, rs, dvec, dblk, s));
-        } else {
-            {
-                ProfScope ps(ctx, "rp_sample", s);
-                rp_sample_kernel<<<1, kSampleThreads, 0, s>>>(dvec, dblk, N, nblk, round, b, p->seed,
-                                                              unif, props, rs, p->k_max, p->max_rounds,
-                                                              p->err_target, floor_rel, err);
-                KEVD_LAUNCH(ctx);
-            }
-            {
-                ProfScope ps(ctx, "rp_hgram", s);
-                rp_hgram_kernel<T><<<n_split + n_kss, 256, hsm, s>>>(F, ldF, X, d, scale, props, b,
-                                                                   n_split, rs, hpart, kss);
-                KEVD_LAUNCH(ctx);
-            }
-            {
-                ProfScope ps(ctx, "rp_factor", s);
-                if (big)
-                    rp_factor_big_kernel<<<1, kBigFactorThreads, 0, s>>>(kss, hpart, b, round, p->seed, unif, p->tol,
-                                                                          floor_rel, p->k_max, props, rs, minv, minv_f,
-                                                                          sacc, piv, hm, hbig, hbig + (size_t)b * b,
-                                                                          hbig + (size_t)2 * b * b);
-                else
-                    factor<<<1, kFactorThreads, fsm, s>>>(kss, hpart, b, round, p->seed, unif, p->tol,
-                                                                    floor_rel, p->k_max, props, rs, minv, minv_f, sacc,
-                                                                    piv, hm);
-                KEVD_LAUNCH(ctx);
-            }
-            if (use_tc) {
-                KEVD_TRY(launch_update_tc(ctx, reinterpret_cast<float*>(F), ldF, N, p->k_max, X, d, scale, sacc,
-                                          minv_f, b, rs, dvec, dblk, tc_err, s));
-            } else if constexpr (sizeof(T) == 4) {
-                ProfScope ps(ctx, "rp_update", s);
-                KEVD_TRY(launch_update_f32(ctx, (float*)F, ldF, X, N, d, scale, sacc, minv_f, b, rs, dvec, dblk, s));
-            } else {
-                ProfScope ps(ctx, "rp_update", s);
-                for (int g = 0; g < n_groups; ++g) {
-                    rp_update_kernel<T><<<(int)nblk, 256, usm, s>>>(F, ldF, X, N, d, scale, sacc, minv,
-                                                                   minv_f, b, rs, dvec, dblk, g);
-                    KEVD_LAUNCH(ctx);
-                }
-            }
-        }
-        if (!defer && round % poll == poll - 1) {
-            KEVD_CUDA(ctx, cudaMemcpyAsync(done_h, &rs->done, sizeof(int), cudaMemcpyDeviceToHost, s));
+        KEVD_TRY(run.round(round, s));
+        if (round % poll == poll - 1) {
+            KEVD_CUDA(ctx, cudaMemcpyAsync(done_h, &run.rs->done, sizeof(int), cudaMemcpyDeviceToHost, s));
             KEVD_CUDA(ctx, cudaStreamSynchronize(s));
             if (*done_h) break;
         }
     }
-    // closing sampler call: records the last round's error and the stop
-    if (small) {
-        KEVD_TRY(propose_small(std::min(round, p->max_rounds), 0, std::min(round, p->max_rounds)));
-    } else {
-        rp_sample_kernel<<<1, kSampleThreads, 0, s>>>(dvec, dblk, N, nblk, std::min(round, p->max_rounds),
-                                                      0, p->seed, unif, props, rs, p->k_max,
-                                                      std::min(round, p->max_rounds), p->err_target, floor_rel, err);
-        KEVD_LAUNCH(ctx);
-    }
-    if (defer) {
-        // capture-safe: results go to pinned host memory, read after the stream completes
-        KEVD_CUDA(ctx, cudaMemcpyAsync(defer->state_h, rs, sizeof(RoundState), cudaMemcpyDeviceToHost, s));
-        KEVD_CUDA(ctx, cudaMemcpyAsync(defer->tcerr_h, tc_err, sizeof(int), cudaMemcpyDeviceToHost, s));
-        KEVD_CUDA(ctx, cudaMemcpyAsync(defer->piv_h, piv, p->k_max * sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-        return KEVD_OK;
-    }
+    KEVD_TRY(run.closing(std::min(round, p->max_rounds), s));
     RoundState hs;
     int herr = 0;
-    KEVD_CUDA(ctx, cudaMemcpyAsync(&hs, rs, sizeof(RoundState), cudaMemcpyDeviceToHost, s));
-    KEVD_CUDA(ctx, cudaMemcpyAsync(&herr, tc_err, sizeof(int), cudaMemcpyDeviceToHost, s));
+    KEVD_CUDA(ctx, cudaMemcpyAsync(&hs, run.rs, sizeof(RoundState), cudaMemcpyDeviceToHost, s));
+    KEVD_CUDA(ctx, cudaMemcpyAsync(&herr, run.tc_err, sizeof(int), cudaMemcpyDeviceToHost, s));
     KEVD_CUDA(ctx, cudaStreamSynchronize(s));
     if (herr != 0)
         return set_error(ctx, KEVD_ERR_TIMEOUT, "rpchol: tensor-core update pipeline timed out (code %d)", herr);
     if (hs.rank > 0 && piv_h)
-        KEVD_CUDA(ctx, cudaMemcpy(piv_h, piv, hs.rank * sizeof(int64_t), cudaMemcpyDeviceToHost));
-    if (err_h) KEVD_CUDA(ctx, cudaMemcpy(err_h, err, hs.rounds * sizeof(double), cudaMemcpyDeviceToHost));
-    if (hm_h) KEVD_CUDA(ctx, cudaMemcpy(hm_h, hm, hs.rounds * sizeof(int32_t), cudaMemcpyDeviceToHost));
+        KEVD_CUDA(ctx, cudaMemcpy(piv_h, run.piv, hs.rank * sizeof(int64_t), cudaMemcpyDeviceToHost));
+    if (err_h) KEVD_CUDA(ctx, cudaMemcpy(err_h, run.err, hs.rounds * sizeof(double), cudaMemcpyDeviceToHost));
+    if (hm_h) KEVD_CUDA(ctx, cudaMemcpy(hm_h, run.hm, hs.rounds * sizeof(int32_t), cudaMemcpyDeviceToHost));
     if (res) {
         res->rank = hs.rank;
         res->rounds = hs.rounds;
@@ -998,17 +1022,232 @@ int run_rpchol(kevd_ctx* ctx, const float* X, int64_t N, int d, double scale,
     if (p->precision == KEVD_MIXED) {
         bool diag = false;
         if (update_tc_supported((const float*)F, ldF, d)) KEVD_TRY(kernel_nearly_diagonal(ctx, X, N, d, scale, s, &diag));
-        return rpchol_impl<float>(ctx, X, N, d, scale, p, (float*)F, ldF, piv, err, accepted, res, s, nullptr, !diag);
+        return rpchol_impl<float>(ctx, X, N, d, scale, p, (float*)F, ldF, piv, err, accepted, res, s, !diag);
     }
     return set_error(ctx, KEVD_ERR_ARG, "rpchol: unknown precision %d", p->precision);
 }
 
-// Many factorisations at once.  Each job gets its own workspace context and
-// stream; with use_graph the whole set of round loops is captured as parallel
-// branches of one CUDA graph (fork from the caller's stream, join back) and
-// launched once, so the GPU overlaps the jobs' small launches without a host
-// thread per job.  Without use_graph the same work is issued directly on the
-// per-job streams.
+// Many factorisations at once, each with a workspace and a stream of its own.
+// With use_graph, kGraphRounds rounds of every job are captured as parallel
+// branches of one CUDA graph (a round's launches do not depend on its index) and
+// the graph is launched until every job has stopped; without, the same rounds are
+// issued directly on the jobs' streams.  The host looks at a chunk's results while
+// the next one runs.  Eight jobs of N = 14,000 .. 91,000 to rank 113 .. 981, b =
+// 32: 13.6 ms a call, with and without the graph (31.3 ms with one graph of all
+// max_rounds rounds, 136 for rank 1,000 of which about 35 do work: allocation,
+// capture and instantiation took longer than the rounds).
+//
+// The jobs' workspaces, streams and pinned buffers stay with the context (grown to
+// the largest batch seen) while they are at most kBatchKeepJobs and hold at most
+// kBatchKeepBytes; beyond, and after an error, they are freed at the end of the call.
+constexpr int kGraphRounds = 4;
+constexpr size_t kBatchKeepBytes = (size_t)1 << 30;
+constexpr int kBatchKeepJobs = 64;
+
+struct BatchSlot {
+    kevd_ctx* c = nullptr;
+    cudaStream_t st = nullptr;
+    cudaEvent_t ev = nullptr;            // joins the job's branch
+    cudaEvent_t seen[2] = {};            // chunk's results copied (direct launches)
+    RoundState* state_h = nullptr;       // pinned: two chunks' states, the error flag, the pivots
+    int* tcerr_h = nullptr;
+    int64_t* piv_h = nullptr;
+    size_t pinned = 0;
+};
+struct BatchPool {
+    std::vector<BatchSlot> slots;
+    cudaStream_t cs = nullptr;           // capture stream
+    cudaEvent_t fork = nullptr, seen[2] = {};
+};
+
+static void free_batch_slot(BatchSlot& x) {
+    if (x.ev) cudaEventDestroy(x.ev);
+    for (cudaEvent_t e : x.seen)
+        if (e) cudaEventDestroy(e);
+    if (x.st) cudaStreamDestroy(x.st);
+    if (x.state_h) cudaFreeHost(x.state_h);
+    if (x.c) {
+        x.c->arena.release();
+        delete x.c;
+    }
+    x = BatchSlot();
+}
+
+void free_batch_pool(kevd_ctx* ctx) {
+    BatchPool* pool = static_cast<BatchPool*>(ctx->batch_pool);
+    if (!pool) return;
+    for (auto& x : pool->slots) free_batch_slot(x);
+    if (pool->cs) cudaStreamDestroy(pool->cs);
+    if (pool->fork) cudaEventDestroy(pool->fork);
+    for (cudaEvent_t e : pool->seen)
+        if (e) cudaEventDestroy(e);
+    delete pool;
+    ctx->batch_pool = nullptr;
+}
+
+// The pool with n ready slots, each with pinned room for its job's pivots.
+static int batch_pool(kevd_ctx* ctx, const kevd_rpchol_job* jobs, int n, BatchPool** out) {
+    if (!ctx->batch_pool) ctx->batch_pool = new BatchPool();
+    BatchPool& pool = *static_cast<BatchPool*>(ctx->batch_pool);
+    *out = &pool;
+    auto event = [&](cudaEvent_t* e) { return *e ? cudaSuccess : cudaEventCreateWithFlags(e, cudaEventDisableTiming); };
+    // the capture runs on a stream of its own (the caller's stream may be the
+    // legacy default stream, which cannot be captured)
+    if (!pool.cs) KEVD_CUDA(ctx, cudaStreamCreateWithFlags(&pool.cs, cudaStreamNonBlocking));
+    KEVD_CUDA(ctx, event(&pool.fork));
+    for (cudaEvent_t& e : pool.seen) KEVD_CUDA(ctx, event(&e));
+    if ((int)pool.slots.size() < n) pool.slots.resize(n);
+    for (int q = 0; q < n; ++q) {
+        BatchSlot& x = pool.slots[q];
+        if (!x.c) {
+            x.c = new kevd_ctx();
+            x.c->device = ctx->device;
+            x.c->num_sms = ctx->num_sms;
+        }
+        if (!x.st) KEVD_CUDA(ctx, cudaStreamCreateWithFlags(&x.st, cudaStreamNonBlocking));
+        KEVD_CUDA(ctx, event(&x.ev));
+        for (cudaEvent_t& e : x.seen) KEVD_CUDA(ctx, event(&e));
+        const size_t head = 2 * sizeof(RoundState) + 16, want = head + (size_t)jobs[q].k_max * sizeof(int64_t);
+        if (x.pinned < want) {
+            if (x.state_h) cudaFreeHost(x.state_h);
+            x.state_h = nullptr;
+            x.pinned = 0;
+            KEVD_CUDA(ctx, cudaMallocHost(&x.state_h, want));
+            x.pinned = want;
+            x.tcerr_h = reinterpret_cast<int*>(x.state_h + 2);
+            x.piv_h = reinterpret_cast<int64_t*>(reinterpret_cast<uint8_t*>(x.state_h) + head);
+        }
+    }
+    return KEVD_OK;
+}
+
+static int rpchol_batched(kevd_ctx* ctx, kevd_rpchol_job* jobs, int n_jobs, bool use_graph, BatchPool& pool,
+                          int* cnt, cudaGraph_t* graph, cudaGraphExec_t* exec, cudaStream_t s) {
+    // the residual-update form of every job, decided before any capture
+    KEVD_CUDA(ctx, cudaMemsetAsync(cnt, 0, n_jobs * sizeof(int), s));
+    for (int q = 0; q < n_jobs; ++q) {
+        const kevd_rpchol_job& j = jobs[q];
+        if (j.N < 2 || !update_tc_supported((const float*)j.F, j.ldF, j.d)) continue;
+        kernel_density_kernel<<<1, 256, 0, s>>>(j.X, j.N, j.d, j.scale, cnt + q);
+        KEVD_LAUNCH(ctx);
+    }
+    std::vector<int> hcnt(n_jobs);
+    KEVD_CUDA(ctx, cudaMemcpyAsync(hcnt.data(), cnt, n_jobs * sizeof(int), cudaMemcpyDeviceToHost, s));
+    KEVD_CUDA(ctx, cudaStreamSynchronize(s));
+    std::vector<RpRun<float>> runs;
+    runs.reserve(n_jobs);
+    auto job_error = [&](int q, int rc) {
+        return set_error(ctx, rc, "rpchol_batched: job %d: %s", q, pool.slots[q].c->last_error.c_str());
+    };
+    for (int q = 0; q < n_jobs; ++q) {
+        const kevd_rpchol_job& j = jobs[q];
+        kevd_rpchol_params p;
+        std::memset(&p, 0, sizeof(p));
+        p.k_max = j.k_max;
+        p.block = j.block;
+        p.max_rounds = j.max_rounds;
+        p.tol = 1e-10;
+        p.seed = j.seed;
+        p.precision = KEVD_MIXED;
+        runs.push_back(RpRun<float>{pool.slots[q].c, j.X, j.N, j.d, j.scale, p, (float*)j.F, j.ldF,
+                                    j.N < 2 || 2 * hcnt[q] >= kDensityPairs});
+        int rc = runs[q].setup();
+        if (rc == KEVD_OK) rc = runs[q].init(s);
+        if (rc != KEVD_OK) return job_error(q, rc);
+    }
+    // one chunk of job q on its stream: kGraphRounds rounds and the state behind them
+    auto chunk = [&](int q, int buf) -> int {
+        BatchSlot& x = pool.slots[q];
+        for (int i = 0; i < kGraphRounds; ++i) {
+            const int rc = runs[q].round(0, x.st);
+            if (rc != KEVD_OK) return job_error(q, rc);
+        }
+        ctx->launches += x.c->launches;
+        x.c->launches = 0;
+        KEVD_CUDA(ctx, cudaMemcpyAsync(x.state_h + buf, runs[q].rs, sizeof(RoundState), cudaMemcpyDeviceToHost, x.st));
+        return KEVD_OK;
+    };
+    auto fork_from = [&](cudaStream_t root) -> int {
+        KEVD_CUDA(ctx, cudaEventRecord(pool.fork, root));
+        for (int q = 0; q < n_jobs; ++q) KEVD_CUDA(ctx, cudaStreamWaitEvent(pool.slots[q].st, pool.fork, 0));
+        return KEVD_OK;
+    };
+    auto join_to = [&](cudaStream_t root) -> int {
+        for (int q = 0; q < n_jobs; ++q) {
+            KEVD_CUDA(ctx, cudaEventRecord(pool.slots[q].ev, pool.slots[q].st));
+            KEVD_CUDA(ctx, cudaStreamWaitEvent(root, pool.slots[q].ev, 0));
+        }
+        return KEVD_OK;
+    };
+    // every job stops by itself in the round after its last one
+    int max_rounds = 0;
+    for (int q = 0; q < n_jobs; ++q) max_rounds = std::max(max_rounds, jobs[q].max_rounds);
+    const int max_chunks = max_rounds / kGraphRounds + 1;
+    if (use_graph) {
+        const int64_t launched = ctx->launches;
+        KEVD_CUDA(ctx, cudaStreamBeginCapture(pool.cs, cudaStreamCaptureModeRelaxed));
+        int rc = fork_from(pool.cs);
+        for (int q = 0; q < n_jobs && rc == KEVD_OK; ++q) rc = chunk(q, 0);
+        if (rc == KEVD_OK) rc = join_to(pool.cs);
+        const cudaError_t ce = cudaStreamEndCapture(pool.cs, graph);
+        const int64_t captured = ctx->launches - launched;
+        ctx->launches = launched;
+        if (rc != KEVD_OK) return rc;
+        if (ce != cudaSuccess) return set_error(ctx, KEVD_ERR_CUDA, "rpchol_batched: end capture: %s", cudaGetErrorString(ce));
+        KEVD_CUDA(ctx, cudaGraphInstantiate(exec, *graph, 0));
+        // launches alternate between two events; the states a launch copied are read
+        // while the next one runs (a later copy can only show more jobs stopped)
+        for (int c = 0; c < max_chunks; ++c) {
+            KEVD_CUDA(ctx, cudaGraphLaunch(*exec, s));
+            ctx->launches += captured;
+            KEVD_CUDA(ctx, cudaEventRecord(pool.seen[c & 1], s));
+            if (c == 0) continue;
+            KEVD_CUDA(ctx, cudaEventSynchronize(pool.seen[(c - 1) & 1]));
+            bool all = true;
+            for (int q = 0; q < n_jobs; ++q)
+                all = all && *reinterpret_cast<volatile int32_t*>(&pool.slots[q].state_h[0].done) != 0;
+            if (all) break;
+        }
+    } else {
+        KEVD_TRY(fork_from(s));
+        std::vector<char> live(n_jobs, 1);
+        int n_live = n_jobs;
+        for (int c = 0; c < max_chunks && n_live > 0; ++c)
+            for (int q = 0; q < n_jobs; ++q) {
+                if (!live[q]) continue;
+                BatchSlot& x = pool.slots[q];
+                KEVD_TRY(chunk(q, c & 1));
+                KEVD_CUDA(ctx, cudaEventRecord(x.seen[c & 1], x.st));
+                if (c == 0) continue;
+                KEVD_CUDA(ctx, cudaEventSynchronize(x.seen[(c - 1) & 1]));
+                if (x.state_h[(c - 1) & 1].done) {
+                    live[q] = 0;
+                    --n_live;
+                }
+            }
+        KEVD_TRY(join_to(s));
+    }
+    for (int q = 0; q < n_jobs; ++q) {
+        BatchSlot& x = pool.slots[q];
+        KEVD_CUDA(ctx, cudaMemcpyAsync(x.state_h, runs[q].rs, sizeof(RoundState), cudaMemcpyDeviceToHost, s));
+        KEVD_CUDA(ctx, cudaMemcpyAsync(x.tcerr_h, runs[q].tc_err, sizeof(int), cudaMemcpyDeviceToHost, s));
+        KEVD_CUDA(ctx, cudaMemcpyAsync(x.piv_h, runs[q].piv, jobs[q].k_max * sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+    }
+    KEVD_CUDA(ctx, cudaStreamSynchronize(s));
+    int rc = KEVD_OK;
+    for (int q = 0; q < n_jobs; ++q) {
+        const BatchSlot& x = pool.slots[q];
+        kevd_rpchol_job& j = jobs[q];
+        if (*x.tcerr_h != 0 && rc == KEVD_OK)
+            rc = set_error(ctx, KEVD_ERR_TIMEOUT, "rpchol_batched: job %d tensor-core pipeline timed out", q);
+        j.result.rank = x.state_h->rank;
+        j.result.rounds = x.state_h->rounds;
+        j.result.trace_error = x.state_h->total / (double)j.N;
+        std::memcpy(j.piv, x.piv_h, (size_t)x.state_h->rank * sizeof(int64_t));
+    }
+    return rc;
+}
+
 int run_rpchol_batched(kevd_ctx* ctx, kevd_rpchol_job* jobs, int n_jobs, int use_graph, cudaStream_t s) {
     if (!jobs || n_jobs < 1 || n_jobs > 1024) return set_error(ctx, KEVD_ERR_ARG, "rpchol_batched: 1..1024 jobs");
     for (int q = 0; q < n_jobs; ++q) {
@@ -1017,131 +1256,27 @@ int run_rpchol_batched(kevd_ctx* ctx, kevd_rpchol_job* jobs, int n_jobs, int use
             j.k_max < 1 || j.ldF < j.k_max || j.max_rounds < 1 || !(j.scale > 0.0))
             return set_error(ctx, KEVD_ERR_ARG, "rpchol_batched: bad job %d", q);
     }
-    struct Slot {
-        kevd_ctx* c = nullptr;
-        cudaStream_t st = nullptr;
-        cudaEvent_t ev = nullptr;
-        RoundState* state_h = nullptr;
-        int* tcerr_h = nullptr;
-        int64_t* piv_h = nullptr;
-    };
-    std::vector<Slot> sl(n_jobs);
-    int rc = KEVD_OK;
-    cudaEvent_t fork = nullptr;
+    BatchPool* pool = nullptr;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
-    auto cleanup = [&]() {
-        if (exec) cudaGraphExecDestroy(exec);
-        if (graph) cudaGraphDestroy(graph);
-        if (fork) cudaEventDestroy(fork);
-        for (auto& x : sl) {
-            if (x.ev) cudaEventDestroy(x.ev);
-            if (x.st) cudaStreamDestroy(x.st);
-            if (x.state_h) cudaFreeHost(x.state_h);
-            if (x.tcerr_h) cudaFreeHost(x.tcerr_h);
-            if (x.piv_h) cudaFreeHost(x.piv_h);
-            if (x.c) {
-                x.c->arena.release();
-                delete x.c;
-            }
-        }
-    };
-    for (int q = 0; q < n_jobs && rc == KEVD_OK; ++q) {
-        Slot& x = sl[q];
-        x.c = new kevd_ctx();
-        x.c->device = ctx->device;
-        x.c->num_sms = ctx->num_sms;
-        if (cudaStreamCreateWithFlags(&x.st, cudaStreamNonBlocking) != cudaSuccess ||
-            cudaEventCreateWithFlags(&x.ev, cudaEventDisableTiming) != cudaSuccess ||
-            cudaMallocHost(&x.state_h, sizeof(RoundState)) != cudaSuccess ||
-            cudaMallocHost(&x.tcerr_h, sizeof(int)) != cudaSuccess ||
-            cudaMallocHost(&x.piv_h, jobs[q].k_max * sizeof(int64_t)) != cudaSuccess)
-            rc = set_error(ctx, KEVD_ERR_CUDA, "rpchol_batched: stream / pinned buffer setup failed");
+    int rc = KEVD_OK;
+    // before the pool is taken: an allocation of ctx may give the pool back
+    int* cnt = arena_get<int>(ctx, "rp.density", n_jobs, &rc);
+    if (rc != KEVD_OK) return set_error(ctx, rc, "rpchol_batched: out of device memory");
+    rc = batch_pool(ctx, jobs, n_jobs, &pool);
+    if (rc == KEVD_OK) rc = rpchol_batched(ctx, jobs, n_jobs, use_graph != 0, *pool, cnt, &graph, &exec, s);
+    if (rc != KEVD_OK) {
+        // work may still be in flight on the caller's or the jobs' streams
+        cudaStreamSynchronize(s);
+        for (auto& x : pool->slots)
+            if (x.st) cudaStreamSynchronize(x.st);
+        cudaGetLastError();
     }
-    if (rc == KEVD_OK && cudaEventCreateWithFlags(&fork, cudaEventDisableTiming) != cudaSuccess)
-        rc = set_error(ctx, KEVD_ERR_CUDA, "rpchol_batched: event setup failed");
-    // the residual-update form of every job, decided before any capture
-    std::vector<char> tc_ok(n_jobs, 1);
-    for (int q = 0; q < n_jobs && rc == KEVD_OK; ++q) {
-        const kevd_rpchol_job& j = jobs[q];
-        bool diag = false;
-        if (update_tc_supported((const float*)j.F, j.ldF, j.d)) rc = kernel_nearly_diagonal(ctx, j.X, j.N, j.d, j.scale, s, &diag);
-        tc_ok[q] = diag ? 0 : 1;
-    }
-    // the capture runs on a stream of its own (the caller's stream may be the
-    // legacy default stream, which cannot be captured); it is ordered after the
-    // caller's work and the graph is launched on the caller's stream
-    cudaStream_t cs = nullptr;
-    if (rc == KEVD_OK && cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking) != cudaSuccess)
-        rc = set_error(ctx, KEVD_ERR_CUDA, "rpchol_batched: capture stream setup failed");
-    auto enqueue_all = [&](int rounds_override, cudaStream_t root) -> int {
-        if (cudaEventRecord(fork, root) != cudaSuccess) return set_error(ctx, KEVD_ERR_CUDA, "rpchol_batched: fork");
-        for (int q = 0; q < n_jobs; ++q) {
-            const kevd_rpchol_job& j = jobs[q];
-            Slot& x = sl[q];
-            if (cudaStreamWaitEvent(x.st, fork, 0) != cudaSuccess)
-                return set_error(ctx, KEVD_ERR_CUDA, "rpchol_batched: fork wait");
-            kevd_rpchol_params p;
-            std::memset(&p, 0, sizeof(p));
-            p.k_max = j.k_max;
-            p.block = j.block;
-            p.max_rounds = rounds_override > 0 ? rounds_override : j.max_rounds;
-            p.tol = 1e-10;
-            p.seed = j.seed;
-            p.precision = KEVD_MIXED;
-            RpcholDeferred df{x.state_h, x.tcerr_h, x.piv_h};
-            const int r = rpchol_impl<float>(x.c, j.X, j.N, j.d, j.scale, &p, (float*)j.F, j.ldF, nullptr, nullptr,
-                                             nullptr, nullptr, x.st, &df, tc_ok[q] != 0);
-            ctx->launches += x.c->launches;
-            x.c->launches = 0;
-            if (r != KEVD_OK) return set_error(ctx, r, "rpchol_batched: job %d: %s", q, x.c->last_error.c_str());
-            if (cudaEventRecord(x.ev, x.st) != cudaSuccess || cudaStreamWaitEvent(root, x.ev, 0) != cudaSuccess)
-                return set_error(ctx, KEVD_ERR_CUDA, "rpchol_batched: join");
-        }
-        return KEVD_OK;
-    };
-    if (rc == KEVD_OK) {
-        if (use_graph) {
-            // one uncaptured round per job allocates every workspace buffer (their
-            // sizes do not depend on the round count), so nothing is allocated
-            // inside the capture; the captured run starts again from rp_init
-            rc = enqueue_all(1, s);
-            if (rc == KEVD_OK && cudaStreamSynchronize(s) != cudaSuccess)
-                rc = set_error(ctx, KEVD_ERR_CUDA, "rpchol_batched: workspace pass failed");
-            if (rc == KEVD_OK) {
-                if (cudaStreamBeginCapture(cs, cudaStreamCaptureModeRelaxed) != cudaSuccess) {
-                    rc = set_error(ctx, KEVD_ERR_CUDA, "rpchol_batched: begin capture");
-                } else {
-                    rc = enqueue_all(0, cs);
-                    const cudaError_t ce = cudaStreamEndCapture(cs, &graph);
-                    if (rc == KEVD_OK && ce != cudaSuccess)
-                        rc = set_error(ctx, KEVD_ERR_CUDA, "rpchol_batched: end capture: %s", cudaGetErrorString(ce));
-                }
-            }
-            if (rc == KEVD_OK && cudaGraphInstantiate(&exec, graph, 0) != cudaSuccess)
-                rc = set_error(ctx, KEVD_ERR_CUDA, "rpchol_batched: graph instantiate");
-            if (rc == KEVD_OK && cudaGraphLaunch(exec, s) != cudaSuccess)
-                rc = set_error(ctx, KEVD_ERR_CUDA, "rpchol_batched: graph launch");
-        } else {
-            rc = enqueue_all(0, s);
-        }
-    }
-    if (rc == KEVD_OK && cudaStreamSynchronize(s) != cudaSuccess)
-        rc = set_error(ctx, KEVD_ERR_CUDA, "rpchol_batched: %s", cudaGetErrorString(cudaGetLastError()));
-    if (rc == KEVD_OK) {
-        for (int q = 0; q < n_jobs; ++q) {
-            const Slot& x = sl[q];
-            kevd_rpchol_job& j = jobs[q];
-            if (*x.tcerr_h != 0 && rc == KEVD_OK)
-                rc = set_error(ctx, KEVD_ERR_TIMEOUT, "rpchol_batched: job %d tensor-core pipeline timed out", q);
-            j.result.rank = x.state_h->rank;
-            j.result.rounds = x.state_h->rounds;
-            j.result.trace_error = x.state_h->total / (double)j.N;
-            std::memcpy(j.piv, x.piv_h, (size_t)x.state_h->rank * sizeof(int64_t));
-        }
-    }
-    cleanup();
-    if (cs) cudaStreamDestroy(cs);
+    if (exec) cudaGraphExecDestroy(exec);
+    if (graph) cudaGraphDestroy(graph);
+    size_t held = 0;
+    for (auto& x : pool->slots) held += x.c ? x.c->arena.total() : 0;
+    if (held > kBatchKeepBytes || (int)pool->slots.size() > kBatchKeepJobs || rc != KEVD_OK) free_batch_pool(ctx);
     return rc;
 }
 

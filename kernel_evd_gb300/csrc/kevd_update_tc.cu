@@ -123,7 +123,7 @@ struct RoundView {   // must match the RoundState layout of kevd_rpchol.cu
     int32_t nacc;
     int32_t done;
     int32_t rounds;
-    int32_t pad;
+    int32_t cur;
     double total;
 };
 
@@ -654,6 +654,15 @@ static_assert(kUpdSmem <= 227 * 1024, "shared memory per CTA");
 bool update_tc_supported(const float* F, int64_t ldF, int d) {
     return get_encode() != nullptr && (ldF % 4) == 0 && ((uintptr_t)F % 16) == 0 && d <= kMaxD &&
            ldF * 4 < (1ll << 40);
+}
+
+// The workspace of launch_update_tc, so that it allocates nothing later (inside a
+// stream capture).
+int reserve_update_tc(kevd_ctx* ctx, int64_t N, int64_t k_max) {
+    int rc = KEVD_OK;
+    arena_get<uint8_t>(ctx, "utc.bprep", (size_t)std::max<int64_t>(1, (k_max + kKs - 1) / kKs) * 2 * kBTile, &rc);
+    arena_get<float>(ctx, "utc.kc", (size_t)N * kCols, &rc);
+    return rc == KEVD_OK ? rc : set_error(ctx, rc, "update_tc: out of device memory");
 }
 
 // Enqueue one round's residual update (reads nacc / r_old from the device
