@@ -19,6 +19,7 @@
 // then added in FP64.
 #include "kevd_f64_tc.cuh"
 #include "kevd_internal.cuh"
+#include "kevd_pairtile.cuh"
 #include "kevd_tc.cuh"
 
 #include <algorithm>
@@ -292,11 +293,10 @@ ev_u_kernel(const T* __restrict__ F, int64_t ldF, int64_t N, int64_t k, const do
     }
 }
 
-// Compensated (Kahan) FP32 accumulation: the running sum is s - c.
-__device__ __forceinline__ void kahan_add(float& s, float& c, float x) {
-    const float y = x - c;
-    const float t = s + y;
-    c = (t - s) - y;
+// Compensated (Kahan) FP32 accumulation of packed pairs: the running sum is s + nc.
+__device__ __forceinline__ void kahan_add2(f32x2& s, f32x2& nc, f32x2 y) {   // y = term + nc
+    const f32x2 t = add2(s, y);
+    nc = add2(fma2(t, pack2(-1.f, -1.f), s), y);
     s = t;
 }
 
@@ -393,182 +393,207 @@ evt_rowdot_kernel(const float* __restrict__ FT, int64_t ldT, int64_t N, int64_t 
     if (!(acc > 0.0)) atomicOr(bad, 1);
 }
 
-// U[i][:] = dinv_i * sum_j FT[j][i] Z[j][:]  (Z: k x m column-major FP64, m <= 32).
-// CTA = 256 rows; thread t forms columns 16 h .. 16 h + 15 (h = t & 1) of rows
-// p and p + 128 (p = t >> 1), so every broadcast load of a Z row feeds twice as
-// many FMAs as with one full row per thread (there the shared-memory loads
-// and the FMAs each filled their pipe) at the same 32 accumulators.
-__global__ void __launch_bounds__(256)
-evt_u_kernel(const float* __restrict__ FT, int64_t ldT, int64_t N, int64_t k, const double* __restrict__ Z, int m,
+// Zf[j][q] = Z(j, q) in FP32 (Z: k x m column-major FP64; zero past m and past k,
+// up to len rows), so that every CTA below stages it by 16-byte copies.
+__global__ void evt_zf_kernel(const double* __restrict__ Z, int64_t k, int m, int64_t len, float* __restrict__ Zf) {
+    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < len * 32;
+         e += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t j = e >> 5;
+        const int q = (int)(e & 31);
+        Zf[e] = (j < k && q < m) ? (float)Z[(int64_t)q * k + j] : 0.f;
+    }
+}
+
+// U[i][:] = dinv_i * sum_j FT[j][i] Z[j][:]  (Zf: Z in FP32, 32 columns, rows up to
+// a multiple of kUChunk; m <= 32).  FP32 pipe: 32 FMA per element of F, one chain
+// per entry of U in increasing j.
+// CTA = 128 threads on 256 rows; thread t forms columns 16 h .. 16 h + 15 (h = t & 1)
+// of the four rows 4 (t >> 1) .. +3 as packed pairs of columns: a 16-byte read of F
+// (the next four columns' are in flight) and four of Z for 32 packed FMA.
+// N = 2M, k = 2000: U_FIG
+constexpr int kUChunk = 64;
+__global__ void __launch_bounds__(128, 4)
+evt_u_kernel(const float* __restrict__ FT, int64_t ldT, int64_t N, int64_t k, const float* __restrict__ Zf, int m,
              const double* __restrict__ dinv, float* __restrict__ U, float* __restrict__ Y) {
-    __shared__ __align__(16) float Zs[128][32];
-    const int h = threadIdx.x & 1, p = threadIdx.x >> 1;
-    const int64_t i0 = (int64_t)blockIdx.x * 256 + p, i1 = i0 + 128;
-    const bool v0 = i0 < N, v1 = i1 < N;
-    float acc0[16], acc1[16];
+    __shared__ __align__(16) float Zs[2][kUChunk][32];
+    const int tid = threadIdx.x, h = tid & 1;
+    const int64_t i0 = (int64_t)blockIdx.x * 256 + 4 * (tid >> 1);
+    const bool valid = i0 < N;   // rows N .. ldT - 1 of FT are zeros
+    const float* col = FT + (valid ? i0 : 0);
+    const int64_t n_ch = (k + kUChunk - 1) / kUChunk;
+    auto stage = [&](int64_t c) {
+        const float* src = Zf + c * kUChunk * 32;
+        float* dst = &Zs[c & 1][0][0];
+        for (int e = tid; e < kUChunk * 8; e += 128) tc::cp_async16(dst + 4 * e, src + 4 * e, 16u);
+        tc::cp_async_commit();
+    };
+    f32x2 acc[4][8];
 #pragma unroll
-    for (int q = 0; q < 16; ++q) acc0[q] = acc1[q] = 0.f;
-    for (int64_t j0 = 0; j0 < k; j0 += 128) {
-        __syncthreads();
-        for (int e = threadIdx.x; e < 128 * 32; e += blockDim.x) {
-            const int jj = e >> 5, q = e & 31;
-            const int64_t j = j0 + jj;
-            Zs[jj][q] = (j < k && q < m) ? (float)Z[(int64_t)q * k + j] : 0.f;
-        }
-        __syncthreads();
-        if (v0) {
-            const int jn = (int)min((int64_t)128, k - j0);
-            // the F values of the next four columns are loaded before this
-            // step's FMAs (columns past jn read as zero; Zs is zero there too)
-            float g0[4], g1[4];
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int q = 0; q < 8; ++q) acc[r][q] = 0;
+    float4 g[4];
+    auto fetch = [&](int u, int64_t j) {
+        g[u] = (valid && j < k) ? *reinterpret_cast<const float4*>(col + j * ldT) : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+    stage(0);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) fetch(u, u);
+    for (int64_t c = 0; c < n_ch; ++c) {
+        tc::cp_async_wait<0>();
+        __syncthreads();   // chunk c is staged, and chunk c - 1 no longer read
+        if (c + 1 < n_ch) stage(c + 1);
+        const float (*Zc)[32] = Zs[c & 1];
+#pragma unroll 1
+        for (int jj = 0; jj < kUChunk; jj += 4) {
+            float4 f[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
-                g0[u] = (u < jn) ? FT[(j0 + u) * ldT + i0] : 0.f;
-                g1[u] = (u < jn && v1) ? FT[(j0 + u) * ldT + i1] : 0.f;
+                f[u] = g[u];
+                fetch(u, c * kUChunk + jj + 4 + u);
             }
-            for (int jj = 0; jj < jn; jj += 4) {
-                float f0[4], f1[4];
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    f0[u] = g0[u];
-                    f1[u] = g1[u];
-                }
+            for (int u = 0; u < 4; ++u) {
+                const ulonglong2* zr = reinterpret_cast<const ulonglong2*>(Zc[jj + u] + 16 * h);
+                const f32x2 fr[4] = {pack2(f[u].x, f[u].x), pack2(f[u].y, f[u].y), pack2(f[u].z, f[u].z),
+                                     pack2(f[u].w, f[u].w)};
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const bool in = jj + 4 + u < jn;
-                    g0[u] = in ? FT[(j0 + jj + 4 + u) * ldT + i0] : 0.f;
-                    g1[u] = (in && v1) ? FT[(j0 + jj + 4 + u) * ldT + i1] : 0.f;
-                }
+                for (int q4 = 0; q4 < 4; ++q4) {
+                    const ulonglong2 z = zr[q4];
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const float4* zr = reinterpret_cast<const float4*>(Zs[jj + u] + 16 * h);
-#pragma unroll
-                    for (int q4 = 0; q4 < 4; ++q4) {
-                        const float4 z = zr[q4];
-                        acc0[4 * q4 + 0] = fmaf(f0[u], z.x, acc0[4 * q4 + 0]);
-                        acc0[4 * q4 + 1] = fmaf(f0[u], z.y, acc0[4 * q4 + 1]);
-                        acc0[4 * q4 + 2] = fmaf(f0[u], z.z, acc0[4 * q4 + 2]);
-                        acc0[4 * q4 + 3] = fmaf(f0[u], z.w, acc0[4 * q4 + 3]);
-                        acc1[4 * q4 + 0] = fmaf(f1[u], z.x, acc1[4 * q4 + 0]);
-                        acc1[4 * q4 + 1] = fmaf(f1[u], z.y, acc1[4 * q4 + 1]);
-                        acc1[4 * q4 + 2] = fmaf(f1[u], z.z, acc1[4 * q4 + 2]);
-                        acc1[4 * q4 + 3] = fmaf(f1[u], z.w, acc1[4 * q4 + 3]);
+                    for (int r = 0; r < 4; ++r) {
+                        acc[r][2 * q4] = fma2(fr[r], z.x, acc[r][2 * q4]);
+                        acc[r][2 * q4 + 1] = fma2(fr[r], z.y, acc[r][2 * q4 + 1]);
                     }
                 }
             }
         }
     }
+    const bool vec = m == 32 && ((uintptr_t)U % 16) == 0;
 #pragma unroll
-    for (int r = 0; r < 2; ++r) {
-        const int64_t i = r ? i1 : i0;
-        if (i >= N) continue;
+    for (int r = 0; r < 4; ++r) {
+        const int64_t i = i0 + r;
+        if (i >= N) break;
         const double di = dinv[i];
 #pragma unroll
-        for (int qq = 0; qq < 16; ++qq) {
-            const int q = 16 * h + qq;
-            const float u = (float)((double)(r ? acc1[qq] : acc0[qq]) * di);
-            if (q < m) U[i * m + q] = u;
-            // Y = Dtil^{-1} U of the rounded U, 32 columns (zero beyond m), for the
-            // Rayleigh-Ritz T1 pass
-            if (Y) Y[i * 32 + q] = (q < m) ? (float)((double)u * di) : 0.f;
+        for (int q4 = 0; q4 < 4; ++q4) {
+            const int q = 16 * h + 4 * q4;
+            float a[4], u[4], y[4];
+            unpack2(acc[r][2 * q4], a[0], a[1]);
+            unpack2(acc[r][2 * q4 + 1], a[2], a[3]);
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+                u[b] = (float)((double)a[b] * di);
+                // Y = Dtil^{-1} U of the rounded U, 32 columns (zero beyond m), for the
+                // Rayleigh-Ritz T1 pass
+                y[b] = (q + b < m) ? (float)((double)u[b] * di) : 0.f;
+            }
+            if (vec) {
+                *reinterpret_cast<float4*>(U + i * 32 + q) = make_float4(u[0], u[1], u[2], u[3]);
+            } else {
+#pragma unroll
+                for (int b = 0; b < 4; ++b)
+                    if (q + b < m) U[i * m + q + b] = u[b];
+            }
+            *reinterpret_cast<float4*>(Y + i * 32 + q) = make_float4(y[0], y[1], y[2], y[3]);
         }
     }
 }
 
 // Rayleigh-Ritz T1 partials: T1[j][q] = sum_i FT[j][i] Y[i][q] over this CTA's
 // rows, Y = Dtil^{-1} U rounded to FP32 (N x 32, written by evt_u_kernel), for a
-// block of 64 columns j.  128 threads, thread (jg, qg) owns columns 4 jg..4 jg+3
-// and q = 4 qg..4 qg+3.  Tiles of 64 rows are staged with 16-byte cp.async into
-// a double buffer (the next tile is in flight while this one is used): F as
-// [column][row] with the 16-byte chunk index of a column XOR-ed with
-// (column >> 1) & 7 (the four columns a warp reads at once land in four
-// different bank groups), Y as [row][q].  FP32 products and 8-row FP32 partials
-// (round to nearest: their errors are unbiased and average out in H); the
-// partials are added with compensation over the CTA's row range.
-constexpr int kT1Rows = 64;
-constexpr size_t kT1Smem = 2 * (size_t)(64 * kT1Rows + kT1Rows * 32) * sizeof(float);
-__global__ void __launch_bounds__(128)
+// block of 128 columns j.  128 threads, thread (jg, qg) owns columns 4 jg..4 jg+3
+// and q = 8 qg..8 qg+7 as packed pairs of q.  Tiles of 32 rows are staged with
+// 16-byte cp.async into a double buffer (the next tile is in flight while this one
+// is used): F as [column][row] with the 16-byte chunk index of a column XOR-ed with
+// (column >> 2) & 7 (the eight columns a warp reads at once land in eight different
+// bank groups), Y as [row][q].  FP32 products and 8-row FP32 partials (round to
+// nearest: their errors are unbiased and average out in H); the partials are added
+// with compensation over the CTA's row range.
+// FP32 pipe: 32 (1 + 4 / 8) operations per element of F.  N = 2M, k = 2000: T1_FIG
+constexpr int kT1Rows = 32;
+constexpr int kT1Cols = 128;
+constexpr int kT1Buf = kT1Cols * kT1Rows + kT1Rows * 32;   // floats of one buffer
+__global__ void __launch_bounds__(128, 3)
 evt_t1_kernel(const float* __restrict__ FT, int64_t ldT, int64_t N, int64_t k, const float* __restrict__ Y, int m,
               int64_t rows_per, double* __restrict__ partial) {
-    extern __shared__ __align__(16) float t1sm[];
+    __shared__ __align__(16) float t1sm[2 * kT1Buf];
     const int tid = threadIdx.x;
-    const int jg = tid >> 3, qg = tid & 7;
-    const int64_t j0 = (int64_t)blockIdx.x * 64;
+    const int jg = tid >> 2, qg = tid & 3;
+    const int64_t j0 = (int64_t)blockIdx.x * kT1Cols;
     const int64_t r0 = (int64_t)blockIdx.y * rows_per;
     const int64_t r1 = min(N, r0 + rows_per);
     const int64_t n_t = (r1 > r0) ? (r1 - r0 + kT1Rows - 1) / kT1Rows : 0;
-    auto fbuf = [&](int b) { return t1sm + (size_t)b * (64 * kT1Rows + kT1Rows * 32); };
-    auto stage = [&](int64_t t, int b) {
-        float* Fs = fbuf(b);
-        float* Ws = Fs + 64 * kT1Rows;
+    auto stage = [&](int64_t t) {
+        float* Fs = t1sm + (t & 1) * kT1Buf;
+        float* Ws = Fs + kT1Cols * kT1Rows;
         const int64_t i0 = r0 + t * kT1Rows;
-        for (int e = tid; e < 64 * 16 + kT1Rows * 8; e += 128) {
-            if (e < 64 * 16) {
-                const int jj = e >> 4, c = e & 15;   // column jj, rows 4c..4c+3
-                const int64_t j = j0 + jj, i = i0 + 4 * c;
-                const bool ok = (j < k) && (i < r1);
-                const float* src = ok ? FT + j * ldT + i : FT;
-                tc::cp_async16(Fs + jj * kT1Rows + 4 * (c ^ ((jj >> 1) & 7)), src, ok ? 16u : 0u);
-            } else {
-                const int e2 = e - 64 * 16;
-                const int ii = e2 >> 3, c = e2 & 7;   // row ii, q 4c..4c+3
-                const int64_t i = i0 + ii;
-                const bool ok = i < r1;
-                tc::cp_async16(Ws + ii * 32 + 4 * c, ok ? Y + i * 32 + 4 * c : Y, ok ? 16u : 0u);
-            }
+#pragma unroll
+        for (int e = tid; e < kT1Cols * (kT1Rows / 4); e += 128) {
+            const int jj = e >> 3, c = e & 7;   // column jj, rows 4c..4c+3
+            const int64_t j = j0 + jj, i = i0 + 4 * c;
+            const bool ok = (j < k) && (i < r1);   // FT rows are padded to a multiple of 4 with zeros
+            tc::cp_async16(Fs + jj * kT1Rows + 4 * (c ^ ((jj >> 2) & 7)), ok ? FT + j * ldT + i : FT, ok ? 16u : 0u);
+        }
+#pragma unroll
+        for (int e = tid; e < kT1Rows * 8; e += 128) {
+            const int64_t i = i0 + (e >> 3);
+            const bool ok = i < r1;
+            tc::cp_async16(Ws + 4 * e, ok ? Y + i * 32 + 4 * (e & 7) : Y, ok ? 16u : 0u);
         }
     };
-    float ks[4][4], kc[4][4];
+    f32x2 ks[4][4], kc[4][4];
 #pragma unroll
     for (int a = 0; a < 4; ++a)
 #pragma unroll
-        for (int b = 0; b < 4; ++b) ks[a][b] = kc[a][b] = 0.f;
-    if (n_t > 0) stage(0, 0);
+        for (int b = 0; b < 4; ++b) ks[a][b] = kc[a][b] = 0;
+    if (n_t > 0) stage(0);
     tc::cp_async_commit();
     for (int64_t t = 0; t < n_t; ++t) {
         if (t + 1 < n_t) {
-            stage(t + 1, (int)((t + 1) & 1));
+            stage(t + 1);
             tc::cp_async_commit();
             tc::cp_async_wait<1>();
         } else {
             tc::cp_async_wait<0>();
         }
         __syncthreads();
-        const float* Fs = fbuf((int)(t & 1));
-        const float* Ws = Fs + 64 * kT1Rows;
+        const float* Fs = t1sm + (t & 1) * kT1Buf + 4 * jg * kT1Rows;
+        const float* Ws = t1sm + (t & 1) * kT1Buf + kT1Cols * kT1Rows + 8 * qg;
 #pragma unroll 1
         for (int i8 = 0; i8 < kT1Rows; i8 += 8) {
-            float p[4][4];
+            f32x2 p[4][4];
 #pragma unroll
             for (int a = 0; a < 4; ++a)
 #pragma unroll
-                for (int b = 0; b < 4; ++b) p[a][b] = 0.f;
+                for (int b = 0; b < 4; ++b) p[a][b] = 0;
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const int rc = (i8 >> 2) + h;   // 16-byte chunk of rows 4 rc..4 rc+3
-                float fv[4][4], wv[4][4];
+                float fv[4][4];
 #pragma unroll
-                for (int a = 0; a < 4; ++a) {
-                    const int jj = 4 * jg + a;
-                    const float4 f = *reinterpret_cast<const float4*>(Fs + jj * kT1Rows + 4 * (rc ^ ((jj >> 1) & 7)));
+                for (int a = 0; a < 4; ++a) {   // (column >> 2) & 7 = jg & 7
+                    const float4 f = *reinterpret_cast<const float4*>(Fs + a * kT1Rows + 4 * (rc ^ (jg & 7)));
                     fv[a][0] = f.x; fv[a][1] = f.y; fv[a][2] = f.z; fv[a][3] = f.w;
                 }
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
-                    const float4 w = *reinterpret_cast<const float4*>(Ws + (4 * rc + u) * 32 + 4 * qg);
-                    wv[u][0] = w.x; wv[u][1] = w.y; wv[u][2] = w.z; wv[u][3] = w.w;
+                    const ulonglong2* wr = reinterpret_cast<const ulonglong2*>(Ws + (4 * rc + u) * 32);
+                    const ulonglong2 w0 = wr[0], w1 = wr[1];
+#pragma unroll
+                    for (int a = 0; a < 4; ++a) {
+                        const f32x2 f = pack2(fv[a][u], fv[a][u]);
+                        p[a][0] = fma2(f, w0.x, p[a][0]);
+                        p[a][1] = fma2(f, w0.y, p[a][1]);
+                        p[a][2] = fma2(f, w1.x, p[a][2]);
+                        p[a][3] = fma2(f, w1.y, p[a][3]);
+                    }
                 }
-#pragma unroll
-                for (int u = 0; u < 4; ++u)
-#pragma unroll
-                    for (int a = 0; a < 4; ++a)
-#pragma unroll
-                        for (int b = 0; b < 4; ++b) p[a][b] = fmaf(fv[a][u], wv[u][b], p[a][b]);
             }
 #pragma unroll
             for (int a = 0; a < 4; ++a)
 #pragma unroll
-                for (int b = 0; b < 4; ++b) kahan_add(ks[a][b], kc[a][b], p[a][b]);
+                for (int b = 0; b < 4; ++b) kahan_add2(ks[a][b], kc[a][b], add2(p[a][b], kc[a][b]));
         }
         __syncthreads();
     }
@@ -578,31 +603,39 @@ evt_t1_kernel(const float* __restrict__ FT, int64_t ldT, int64_t N, int64_t k, c
         if (j >= k) continue;
 #pragma unroll
         for (int b = 0; b < 4; ++b) {
-            const int q = 4 * qg + b;
-            if (q < m) partial[((int64_t)blockIdx.y * k + j) * m + q] = (double)ks[a][b] - (double)kc[a][b];
+            const int q = 8 * qg + 2 * b;
+            float s0, s1, c0, c1;
+            unpack2(ks[a][b], s0, s1);
+            unpack2(kc[a][b], c0, c1);
+            double* out = partial + ((int64_t)blockIdx.y * k + j) * m + q;
+            if (q < m) out[0] = (double)s0 + (double)c0;
+            if (q + 1 < m) out[1] = (double)s1 + (double)c1;
         }
     }
 }
 
-// Rayleigh-Ritz H and M partials over 64-row tiles: w_i = F_i (T1h + T1l)
+// Rayleigh-Ritz H and M partials over 128-row tiles: w_i = F_i (T1h + T1l)
 // (T1 as an FP32 hi/lo pair, k x 32), H += (w/sqrt(q))(w/sqrt(q))^T, M += u u^T.
 // 128 threads; for w thread (ig, qg) owns rows 4 ig..4 ig+3 and columns
-// 4 qg..4 qg+3 (16-byte loads of F and of the T1 rows from shared memory, 8-term
-// FP32 partials added with compensation); for H and M thread t owns entries
-// t + 128 r of the 32 x 32 matrices, summed over the tile with compensation and
-// across tiles in FP64.
-constexpr int kHmRows = 64;
-__global__ void __launch_bounds__(128)
+// 8 qg..8 qg+7 as packed pairs (16-byte loads of F and of the T1 rows from shared
+// memory, 8-term FP32 partials added with compensation); for H and M thread t owns
+// entries (8 (t >> 5) + r, t & 31), r < 8, of the 32 x 32 matrices, summed over 64
+// rows with compensation and beyond in FP64.
+// FP32 pipe: 32 (2 + 4 / 8) operations per element of F.  N = 2M, k = 2000: HM_FIG
+constexpr int kHmRows = 128;
+constexpr int kHmFChunk = 32 * kHmRows;                 // floats of an F chunk, [column j][row i]
+constexpr int kHmBuf = kHmFChunk + 2 * 32 * 32;         // and the T1 hi and lo chunks
+constexpr int kHmStride = 36;                           // of a row of w
+constexpr size_t kHmSmem = (2 * kHmBuf + kHmRows * kHmStride) * sizeof(float);
+__global__ void __launch_bounds__(128, 3)
 evt_hm_kernel(const float* __restrict__ FT, int64_t ldT, int64_t N, int64_t k, const float* __restrict__ T1hl,
               int m, const float* __restrict__ U, const double* __restrict__ qinv, double* __restrict__ partial) {
-    // double buffer of (F chunk [column j][row i], T1 hi/lo chunk), 16-byte
-    // cp.async copies: the next (tile, column chunk) step is in flight while
-    // this one is used
-    __shared__ __align__(16) float Fsb[2][32][kHmRows];
-    __shared__ __align__(16) float Tsb[2][2][32][32];
-    __shared__ float Ws[kHmRows][33];
+    // double buffer of (F chunk, T1 hi/lo chunk), 16-byte cp.async copies: the
+    // next (tile, column chunk) step is in flight while this one is used
+    extern __shared__ __align__(16) float hmsm[];
+    float* Ws = hmsm + 2 * kHmBuf;
     const int tid = threadIdx.x;
-    const int ig = tid >> 3, qg = tid & 7;
+    const int ig = tid >> 2, qg = tid & 3;
     double h64[8], m64[8];
 #pragma unroll
     for (int r = 0; r < 8; ++r) h64[r] = m64[r] = 0.0;
@@ -610,19 +643,50 @@ evt_hm_kernel(const float* __restrict__ FT, int64_t ldT, int64_t N, int64_t k, c
     const int nch = (int)((k + 31) / 32);
     auto stage = [&](int64_t t, int c, int b) {
         const int64_t i0 = t * kHmRows, j0 = (int64_t)c * 32;
-        for (int e = tid; e < 32 * (kHmRows / 4) + 64 * 8; e += 128) {
-            if (e < 32 * (kHmRows / 4)) {
-                const int jj = e / (kHmRows / 4), rc = e % (kHmRows / 4);   // column jj, rows 4 rc..4 rc+3
-                const int64_t j = j0 + jj, i = i0 + 4 * rc;
-                const bool ok = (j < k) && (i < N);   // FT rows are padded to a multiple of 4 with zeros
-                tc::cp_async16(&Fsb[b][jj][4 * rc], ok ? FT + j * ldT + i : FT, ok ? 16u : 0u);
-            } else {
-                const int e2 = e - 32 * (kHmRows / 4);
-                const int r2 = e2 >> 3, c4 = e2 & 7;   // T1hl row 2 j + (hi, lo), q 4 c4..4 c4+3
-                const int jj = r2 >> 1, hl = r2 & 1;
-                const int64_t j = j0 + jj;
-                const bool ok = j < k;
-                tc::cp_async16(&Tsb[b][hl][jj][4 * c4], ok ? T1hl + (2 * j + hl) * 32 + 4 * c4 : T1hl, ok ? 16u : 0u);
+        float* Fs = hmsm + b * kHmBuf;
+        float* Ts = Fs + kHmFChunk;   // [hi, lo][32][32]
+#pragma unroll
+        for (int e = tid; e < 32 * (kHmRows / 4); e += 128) {
+            const int jj = e / (kHmRows / 4), rc = e % (kHmRows / 4);   // column jj, rows 4 rc..4 rc+3
+            const int64_t j = j0 + jj, i = i0 + 4 * rc;
+            const bool ok = (j < k) && (i < N);   // FT rows are padded to a multiple of 4 with zeros
+            tc::cp_async16(Fs + 4 * e, ok ? FT + j * ldT + i : FT, ok ? 16u : 0u);
+        }
+#pragma unroll
+        for (int e = tid; e < 64 * 8; e += 128) {
+            const int r2 = e >> 3, c4 = e & 7;   // T1hl row 2 j + (hi, lo), q 4 c4..4 c4+3
+            const int jj = r2 >> 1, hl = r2 & 1;
+            const int64_t j = j0 + jj;
+            const bool ok = j < k;
+            tc::cp_async16(Ts + (hl * 32 + jj) * 32 + 4 * c4, ok ? T1hl + (2 * j + hl) * 32 + 4 * c4 : T1hl,
+                           ok ? 16u : 0u);
+        }
+    };
+    // x64[r] += sum over the tile's rows of Ws[row][8 (t >> 5) + r] Ws[row][t & 31]
+    auto outer = [&](double (&x64)[8]) {
+        const float* wa = Ws + 8 * (tid >> 5);
+        const float* wb = Ws + (tid & 31);
+#pragma unroll 1
+        for (int r0 = 0; r0 < kHmRows; r0 += 64) {
+            f32x2 s[4] = {0, 0, 0, 0}, c[4] = {0, 0, 0, 0};
+#pragma unroll 4
+            for (int rr = r0; rr < r0 + 64; ++rr) {
+                const float b = wb[rr * kHmStride];
+                const ulonglong2* ar = reinterpret_cast<const ulonglong2*>(wa + rr * kHmStride);
+                const f32x2 b2 = pack2(b, b);
+                const ulonglong2 a0 = ar[0], a1 = ar[1];
+                kahan_add2(s[0], c[0], fma2(a0.x, b2, c[0]));
+                kahan_add2(s[1], c[1], fma2(a0.y, b2, c[1]));
+                kahan_add2(s[2], c[2], fma2(a1.x, b2, c[2]));
+                kahan_add2(s[3], c[3], fma2(a1.y, b2, c[3]));
+            }
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                float s0, s1, c0, c1;
+                unpack2(s[r], s0, s1);
+                unpack2(c[r], c0, c1);
+                x64[2 * r] += (double)s0 + (double)c0;
+                x64[2 * r + 1] += (double)s1 + (double)c1;
             }
         }
     };
@@ -631,11 +695,11 @@ evt_hm_kernel(const float* __restrict__ FT, int64_t ldT, int64_t N, int64_t k, c
     tc::cp_async_commit();
     for (int64_t t = blockIdx.x; t < n_tiles; t += gridDim.x) {
         const int64_t i0 = t * kHmRows;
-        float ws[4][4], wc[4][4];
+        f32x2 ws[4][4], wc[4][4];
 #pragma unroll
         for (int a = 0; a < 4; ++a)
 #pragma unroll
-            for (int bb = 0; bb < 4; ++bb) ws[a][bb] = wc[a][bb] = 0.f;
+            for (int q = 0; q < 4; ++q) ws[a][q] = wc[a][q] = 0;
         for (int c = 0; c < nch; ++c) {
             const int64_t nt = (c + 1 < nch) ? t : t + gridDim.x;
             const int nc = (c + 1 < nch) ? c + 1 : 0;
@@ -647,76 +711,71 @@ evt_hm_kernel(const float* __restrict__ FT, int64_t ldT, int64_t N, int64_t k, c
                 tc::cp_async_wait<0>();
             }
             __syncthreads();
-            float (*Fs)[kHmRows] = Fsb[b];
-            float (*Ts)[32][32] = Tsb[b];
+            const float* Fs = hmsm + b * kHmBuf + 4 * ig;
+            const float* Ts = hmsm + b * kHmBuf + kHmFChunk + 8 * qg;
 #pragma unroll 1
             for (int j8 = 0; j8 < 32; j8 += 8) {
-                float p[4][4];
+                f32x2 p[4][4];
 #pragma unroll
                 for (int a = 0; a < 4; ++a)
 #pragma unroll
-                    for (int bb = 0; bb < 4; ++bb) p[a][bb] = 0.f;
+                    for (int q = 0; q < 4; ++q) p[a][q] = 0;
 #pragma unroll
                 for (int u = 0; u < 8; ++u) {
-                    const float4 f = *reinterpret_cast<const float4*>(&Fs[j8 + u][4 * ig]);
-                    const float4 th = *reinterpret_cast<const float4*>(&Ts[0][j8 + u][4 * qg]);
-                    const float4 tl = *reinterpret_cast<const float4*>(&Ts[1][j8 + u][4 * qg]);
-                    const float fv[4] = {f.x, f.y, f.z, f.w};
-                    const float hv[4] = {th.x, th.y, th.z, th.w}, lv[4] = {tl.x, tl.y, tl.z, tl.w};
+                    const float4 f = *reinterpret_cast<const float4*>(Fs + (j8 + u) * kHmRows);
+                    const ulonglong2* th = reinterpret_cast<const ulonglong2*>(Ts + (j8 + u) * 32);
+                    const ulonglong2* tl = reinterpret_cast<const ulonglong2*>(Ts + (32 + j8 + u) * 32);
+                    const f32x2 fv[4] = {pack2(f.x, f.x), pack2(f.y, f.y), pack2(f.z, f.z), pack2(f.w, f.w)};
 #pragma unroll
-                    for (int a = 0; a < 4; ++a)
+                    for (int q = 0; q < 2; ++q) {
+                        const ulonglong2 l = tl[q], hi = th[q];
 #pragma unroll
-                        for (int bb = 0; bb < 4; ++bb) p[a][bb] = fmaf(fv[a], hv[bb], fmaf(fv[a], lv[bb], p[a][bb]));
+                        for (int a = 0; a < 4; ++a) {
+                            p[a][2 * q] = fma2(fv[a], hi.x, fma2(fv[a], l.x, p[a][2 * q]));
+                            p[a][2 * q + 1] = fma2(fv[a], hi.y, fma2(fv[a], l.y, p[a][2 * q + 1]));
+                        }
+                    }
                 }
 #pragma unroll
                 for (int a = 0; a < 4; ++a)
 #pragma unroll
-                    for (int bb = 0; bb < 4; ++bb) kahan_add(ws[a][bb], wc[a][bb], p[a][bb]);
+                    for (int q = 0; q < 4; ++q) kahan_add2(ws[a][q], wc[a][q], add2(p[a][q], wc[a][q]));
             }
             __syncthreads();
             b ^= 1;
         }
-        __syncthreads();
 #pragma unroll
         for (int a = 0; a < 4; ++a) {
             const int64_t i = i0 + 4 * ig + a;
             const float sq = (i < N) ? (float)sqrt(qinv[i]) : 0.f;
 #pragma unroll
-            for (int bb = 0; bb < 4; ++bb) {
-                const int q = 4 * qg + bb;
-                Ws[4 * ig + a][q] = (q < m) ? (ws[a][bb] - wc[a][bb]) * sq : 0.f;
+            for (int q = 0; q < 4; ++q) {
+                float s0, s1, c0, c1;
+                unpack2(ws[a][q], s0, s1);
+                unpack2(wc[a][q], c0, c1);
+                const int col = 8 * qg + 2 * q;
+                float* o = Ws + (4 * ig + a) * kHmStride + col;
+                o[0] = (col < m) ? (s0 + c0) * sq : 0.f;
+                o[1] = (col + 1 < m) ? (s1 + c1) * sq : 0.f;
             }
         }
         __syncthreads();
-#pragma unroll
-        for (int r = 0; r < 8; ++r) {
-            const int e = tid + 128 * r;
-            const int ja = e >> 5, jb = e & 31;
-            float hs = 0.f, hc = 0.f;
-            for (int rr = 0; rr < kHmRows; ++rr) kahan_add(hs, hc, Ws[rr][ja] * Ws[rr][jb]);
-            h64[r] += (double)hs - (double)hc;
-        }
+        outer(h64);
         __syncthreads();
         for (int e = tid; e < kHmRows * 32; e += 128) {
             const int rr = e >> 5, q = e & 31;
             const int64_t i = i0 + rr;
-            Ws[rr][q] = (i < N && q < m) ? U[i * m + q] : 0.f;
+            Ws[rr * kHmStride + q] = (i < N && q < m) ? U[i * m + q] : 0.f;
         }
         __syncthreads();
-#pragma unroll
-        for (int r = 0; r < 8; ++r) {
-            const int e = tid + 128 * r;
-            const int ja = e >> 5, jb = e & 31;
-            float ms = 0.f, mc = 0.f;
-            for (int rr = 0; rr < kHmRows; ++rr) kahan_add(ms, mc, Ws[rr][ja] * Ws[rr][jb]);
-            m64[r] += (double)ms - (double)mc;
-        }
+        outer(m64);
+        __syncthreads();   // before Ws is written again
     }
-    double* out = partial + (int64_t)blockIdx.x * 2048;
+    double* out = partial + (int64_t)blockIdx.x * 2048 + 8 * (tid >> 5) * 32 + (tid & 31);
 #pragma unroll
     for (int r = 0; r < 8; ++r) {
-        out[tid + 128 * r] = h64[r];
-        out[1024 + tid + 128 * r] = m64[r];
+        out[32 * r] = h64[r];
+        out[1024 + 32 * r] = m64[r];
     }
 }
 
@@ -778,25 +837,29 @@ static int rayleigh_ritz(kevd_ctx* ctx, const float* FT, int64_t ldT, int64_t N,
                          const float* Y, const double* qinv, double* lam_top, cudaStream_t s) {
     ProfScope ps(ctx, "ev_ritz", s);
     int st = KEVD_OK;
-    const int ny = (int)std::min<int64_t>((N + 8191) / 8192, (int64_t)ctx->num_sms * 2);
+    // T1: row ranges of 8192 rows (at most two a SM), shorter ones, down to 512
+    // rows, where those and the column blocks would leave SMs without a CTA
+    const int t1c = ceil_div(k, kT1Cols);
+    const int64_t fill = std::min<int64_t>((N + 511) / 512, ceil_div((int64_t)ctx->num_sms * 3, t1c));
+    const int ny = (int)std::max<int64_t>(std::min<int64_t>((N + 8191) / 8192, (int64_t)ctx->num_sms * 2), fill);
     const int64_t rows_per = ((N + ny - 1) / ny + 63) / 64 * 64;
     double* tpart = arena_get<double>(ctx, "rr.tpart", (size_t)ny * k * m, &st);
     double* T1 = arena_get<double>(ctx, "rr.T1", (size_t)k * m, &st);
     float* T1hl = arena_get<float>(ctx, "rr.T1hl", (size_t)k * 64, &st);
-    const int nhm = ctx->num_sms * 4;
+    const int nhm = (int)std::min<int64_t>((int64_t)ctx->num_sms * 3, (N + kHmRows - 1) / kHmRows);
     double* hmpart = arena_get<double>(ctx, "rr.hmpart", (size_t)nhm * 2048, &st);
     double* HM = arena_get<double>(ctx, "rr.HM", 2048, &st);
     double* w = arena_get<double>(ctx, "rr.w", 64, &st);
     int* info = arena_get<int>(ctx, "rr.info", 1, &st);
     if (st != KEVD_OK) return set_error(ctx, st, "rayleigh_ritz: out of device memory");
-    KEVD_CUDA(ctx, raise_smem_limit(reinterpret_cast<const void*>(&evt_t1_kernel), kT1Smem));
-    evt_t1_kernel<<<dim3(ceil_div(k, 64), ny), 128, kT1Smem, s>>>(FT, ldT, N, k, Y, m, rows_per, tpart);
+    KEVD_CUDA(ctx, raise_smem_limit(reinterpret_cast<const void*>(&evt_hm_kernel), kHmSmem));
+    evt_t1_kernel<<<dim3(t1c, ny), 128, 0, s>>>(FT, ldT, N, k, Y, m, rows_per, tpart);
     KEVD_LAUNCH(ctx);
     rr_sum_kernel<<<ceil_div(k * m, 256), 256, 0, s>>>(tpart, ny, k * m, T1);
     KEVD_LAUNCH(ctx);
     evt_split_t1_kernel<<<ceil_div(k * 32, 256), 256, 0, s>>>(T1, k, m, T1hl);
     KEVD_LAUNCH(ctx);
-    evt_hm_kernel<<<nhm, 128, 0, s>>>(FT, ldT, N, k, T1hl, m, U, qinv, hmpart);
+    evt_hm_kernel<<<nhm, 128, kHmSmem, s>>>(FT, ldT, N, k, T1hl, m, U, qinv, hmpart);
     KEVD_LAUNCH(ctx);
     rr_sum_kernel<<<8, 256, 0, s>>>(hmpart, nhm, 2048, HM);
     KEVD_LAUNCH(ctx);
@@ -896,6 +959,20 @@ static int gram_f64(kevd_ctx* ctx, const double* F, int64_t ldF, int64_t N, int6
 // U = Dtil^{-1} F Z (row-major float) of an FP64 factor, in exact slices on the
 // tensor cores, row panels of at most 2 GiB of digits at a time; *done = false
 // when there is no room for them.
+// U and Y of at most 32 columns of Z from the column-major FP32 factor.
+static int u_f32(kevd_ctx* ctx, const float* FT, int64_t ldT, int64_t N, int64_t k, const double* Z, int m,
+                 const double* dinv, float* U, float* Y, cudaStream_t s) {
+    const int64_t len = (k + kUChunk - 1) / kUChunk * kUChunk;
+    int st = KEVD_OK;
+    float* Zf = arena_get<float>(ctx, "ev.Zf", (size_t)len * 32, &st);
+    if (st != KEVD_OK) return set_error(ctx, st, "bistochastic_evd: out of device memory");
+    evt_zf_kernel<<<ceil_div(len * 32, 256), 256, 0, s>>>(Z, k, m, len, Zf);
+    KEVD_LAUNCH(ctx);
+    evt_u_kernel<<<ceil_div(N, 256), 128, 0, s>>>(FT, ldT, N, k, Zf, m, dinv, U, Y);
+    KEVD_LAUNCH(ctx);
+    return KEVD_OK;
+}
+
 static int u_f64_tc(kevd_ctx* ctx, const double* F, int64_t ldF, int64_t N, int64_t k, const double* Z, int k_out,
                     const double* dinv, float* U, bool* done, cudaStream_t st) {
     *done = false;
@@ -1201,27 +1278,26 @@ static int evd_impl(kevd_ctx* ctx, const T* F, int64_t N, int64_t k, int64_t ldF
         if (sizeof(T) == 4 && k_out <= 32) {
             Yrr = arena_get<float>(ctx, "ev.Yrr", (size_t)N * 32, &st);
             if (st != KEVD_OK) return set_error(ctx, st, "bistochastic_evd: out of device memory");
-            evt_u_kernel<<<ceil_div(N, 256), 256, 0, s>>>(FT, ldT, N, k, Z, k_out, dinv, U, Yrr);
+            KEVD_TRY(u_f32(ctx, FT, ldT, N, k, Z, k_out, dinv, U, Yrr, s));
             Urr = U;
         } else {
             bool u_done = false;
             if (sizeof(T) == 8 && (double)N * (double)k * 64.0 >= kTcUWork)
                 KEVD_TRY(u_f64_tc(ctx, (const double*)F, ldF, N, k, Z, k_out, dinv, U, &u_done, s));
-            if (!u_done)
+            if (!u_done) {
                 ev_u_kernel<T><<<dim3(ceil_div(N, 64), ceil_div(k_out, 64)), 256, 0, s>>>(F, ldF, N, k, Z, k_out, dinv,
                                                                                       U);
+                KEVD_LAUNCH(ctx);
+            }
             if (sizeof(T) == 4) {
                 // FP32 factor with k_out > 32: the leading 32 columns once more, with
                 // Y, for their refinement (Z's last 32 columns)
-                KEVD_LAUNCH(ctx);
                 Yrr = arena_get<float>(ctx, "ev.Yrr", (size_t)N * 32, &st);
                 Urr = arena_get<float>(ctx, "ev.Urr", (size_t)N * 32, &st);
                 if (st != KEVD_OK) return set_error(ctx, st, "bistochastic_evd: out of device memory");
-                evt_u_kernel<<<ceil_div(N, 256), 256, 0, s>>>(FT, ldT, N, k, Z + (size_t)(k_out - 32) * k, 32, dinv,
-                                                              Urr, Yrr);
+                KEVD_TRY(u_f32(ctx, FT, ldT, N, k, Z + (size_t)(k_out - 32) * k, 32, dinv, Urr, Yrr, s));
             }
         }
-        KEVD_LAUNCH(ctx);
     }
     if (dump) KEVD_TRY(d2h(ctx, dump->Z, Z, (size_t)k * k_out, s));
     double htr[2];
