@@ -98,7 +98,10 @@ constexpr float kSplitUnscale = 1.0f / (16384.f * 16384.f);
 constexpr int kThreads = 576;
 constexpr uint64_t kTimeoutNs = 4000000000ull;
 constexpr int kMaxD = kMaxFeatures;
-constexpr int kGPitch = kCols + 1;  // row pitch of the new-column staging buffer (conflict-free by row and column)
+// T, then G, of a row block, column-major: column c's rows 4 h .. 4 h + 3 are the
+// 16 bytes at chunk h ^ (c & 7), so that reads of one row by consecutive rows and of
+// 16-byte chunks by consecutive chunks or columns are all free of bank conflicts
+__device__ __forceinline__ int g_chunk(int c, int h) { return c * 128 + 4 * (h ^ (c & 7)); }
 
 struct Bars {
     uint64_t tma_full[kStages];
@@ -161,8 +164,8 @@ update_tc_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant
     // K(R, S_i) tile: two 128 x 32 SWIZZLE_128B halves (TMA), then G in place
     uint8_t* ktile = base + (size_t)kStages * kStageBytes;
     float* mv = reinterpret_cast<float*>(ktile + 2 * kAOp);                      // kCols x kCols
-    float* gbuf = mv + kCols * kCols;                                            // kRows x kGPitch: new columns
-    Bars* bar = reinterpret_cast<Bars*>(gbuf + kRows * kGPitch);
+    float* gbuf = mv + kCols * kCols;                                            // kCols x kRows: T, then G (g_chunk)
+    Bars* bar = reinterpret_cast<Bars*>(gbuf + kRows * kCols);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
     // L_i^{-1} (FP32) for the epilogue, transposed: mv[q][a] = L_i^{-1}[a][q]
@@ -415,18 +418,17 @@ update_tc_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant
                 ok = false;
             }
             const bool live = ok && i < N;
-            // T row -> this thread's staging row (pitch kGPitch: the 32 rows of
-            // a warp fall in distinct banks for every column)
-            float* grow = gbuf + rloc * kGPitch;
+            // this thread's T row -> the staging columns
+            float* grow = gbuf + (rloc & 3);
             if (live) {
 #pragma unroll
                 for (int c4 = 0; c4 < kCols / 4; ++c4) {
                     const float4 tv = *reinterpret_cast<const float4*>(
                         ktile + (c4 >> 3) * kAOp + tc::sw128_off((uint32_t)rloc, (uint32_t)(4 * (c4 & 7))));
-                    grow[4 * c4 + 0] = tv.x;
-                    grow[4 * c4 + 1] = tv.y;
-                    grow[4 * c4 + 2] = tv.z;
-                    grow[4 * c4 + 3] = tv.w;
+                    grow[g_chunk(4 * c4 + 0, rloc >> 2)] = tv.x;
+                    grow[g_chunk(4 * c4 + 1, rloc >> 2)] = tv.y;
+                    grow[g_chunk(4 * c4 + 2, rloc >> 2)] = tv.z;
+                    grow[g_chunk(4 * c4 + 3, rloc >> 2)] = tv.w;
                 }
             }
             // every tail thread has copied its T row: the next K tile may land
@@ -438,66 +440,89 @@ update_tc_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant
                 tc::fence_async_smem();
                 load_ktile(&tmk, ktile, &bar->kfull, rb + gridDim.x);
             }
+            // G = T L_i^{-T} in place in the warp's 32 rows, blocks of sixteen outputs
+            // from the last to the first: block a0 reads T[0 .. a0 + 15] and overwrites
+            // T[a0 .. a0 + 15], which no later block needs.  A lane forms four outputs
+            // of four rows as packed pairs, each G[a] one FMA chain over e = 0 .. in
+            // increasing order (the zero terms above the diagonal leave it unchanged):
+            // 32 bytes of shared memory a lane serve 16 FMAs.  The whole tail
+            // of a row block takes 17k clocks (25k with a row's outputs in one thread,
+            // bound by its reads of L_i^{-1}), so updates of r < 600 columns no longer wait
+            // for it: N = 2M, k = 2,000, all updates 58.5 -> 55.8 ms.
+            __syncwarp();   // the warp's rows of T are staged
+            {
+                const int h = 8 * q + (lane & 7), oq = lane >> 3;
+                for (int a0 = (nacc - 1) & ~15; a0 >= 0; a0 -= 16) {
+                    f32x2 gq[4][2];
+#pragma unroll
+                    for (int rr = 0; rr < 4; ++rr) gq[rr][0] = gq[rr][1] = 0;
+                    const float* mcol = mv + a0 + 4 * oq;
+#pragma unroll 1
+                    for (int e8 = 0; e8 < a0 + 16; e8 += 8) {
+#pragma unroll
+                        for (int u = 0; u < 8; ++u) {
+                            const int e = e8 + u;
+                            const float4 te = *reinterpret_cast<const float4*>(gbuf + e8 * 128 + g_chunk(u, h));
+                            const ulonglong2 m = *reinterpret_cast<const ulonglong2*>(mcol + e * kCols);
+                            const float tr[4] = {te.x, te.y, te.z, te.w};
+#pragma unroll
+                            for (int rr = 0; rr < 4; ++rr) {
+                                const f32x2 t2 = pack2(tr[rr], tr[rr]);
+                                gq[rr][0] = fma2(t2, m.x, gq[rr][0]);
+                                gq[rr][1] = fma2(t2, m.y, gq[rr][1]);
+                            }
+                        }
+                    }
+                    __syncwarp();   // T[a0 ..] has been read
+#pragma unroll
+                    for (int c = 0; c < 2; ++c) {
+                        float4 g0, g1;
+                        unpack2(gq[0][c], g0.x, g1.x);
+                        unpack2(gq[1][c], g0.y, g1.y);
+                        unpack2(gq[2][c], g0.z, g1.z);
+                        unpack2(gq[3][c], g0.w, g1.w);
+                        *reinterpret_cast<float4*>(gbuf + g_chunk(a0 + 4 * oq + 2 * c, h)) = g0;
+                        *reinterpret_cast<float4*>(gbuf + g_chunk(a0 + 4 * oq + 2 * c + 1, h)) = g1;
+                    }
+                }
+            }
+            __syncwarp();   // this warp's 32 rows of G are staged
             double nd = d_old;
             if (live) {
-                // G = T L_i^{-T} in place in the staging row, blocks of eight
-                // outputs from the last to the first: block a0 reads T[0 ..
-                // a0+7] and overwrites T[a0 .. a0+7], which no earlier block
-                // needs.  Eight independent FMA chains per block, each G[a]
-                // summing e = 0..a in increasing order (the zero terms above
-                // the diagonal leave it unchanged); runtime loops keep the code
-                // small (fully unrolled, the 2,080 FMAs of a row took 11k cycles
-                // per row block against 2k of FP32 pipe time).
-                const int nb = (nacc + 7) >> 3;
+                // squares of a block of eight in increasing order, blocks from the
+                // last to the first
                 float sq = 0.f;
-                for (int blk = nb - 1; blk >= 0; --blk) {
-                    const int a0 = 8 * blk;
-                    float g8[8];
 #pragma unroll
-                    for (int u = 0; u < 8; ++u) g8[u] = 0.f;
-                    const float* mcol = mv + a0;
-#pragma unroll 4
-                    for (int e = 0; e < a0 + 8; ++e) {
-                        const float te = grow[e];
-                        const float4 m0 = *reinterpret_cast<const float4*>(mcol + e * kCols);
-                        const float4 m1 = *reinterpret_cast<const float4*>(mcol + e * kCols + 4);
-                        g8[0] = fmaf(te, m0.x, g8[0]);
-                        g8[1] = fmaf(te, m0.y, g8[1]);
-                        g8[2] = fmaf(te, m0.z, g8[2]);
-                        g8[3] = fmaf(te, m0.w, g8[3]);
-                        g8[4] = fmaf(te, m1.x, g8[4]);
-                        g8[5] = fmaf(te, m1.y, g8[5]);
-                        g8[6] = fmaf(te, m1.z, g8[6]);
-                        g8[7] = fmaf(te, m1.w, g8[7]);
-                    }
-                    float sb = 0.f;
+                for (int blk = kCols / 8 - 1; blk >= 0; --blk)
+                    if (8 * blk < nacc) {
+                        float sb = 0.f;
 #pragma unroll
-                    for (int u = 0; u < 8; ++u) {
-                        grow[a0 + u] = g8[u];
-                        if (a0 + u < nacc) sb = fmaf(g8[u], g8[u], sb);
+                        for (int u = 0; u < 8; ++u) {
+                            const float gv = grow[g_chunk(8 * blk + u, rloc >> 2)];
+                            if (8 * blk + u < nacc) sb = fmaf(gv, gv, sb);
+                        }
+                        sq += sb;
                     }
-                    sq += sb;
-                }
                 nd = fmax(d_old - (double)sq, 0.0);
                 dvec[i] = nd;
             }
-            __syncwarp();   // this warp's 32 rows of G staged
-            // coalesced store of the new columns: warp q writes its own rows
-            // 32q .. 32q+31, so no other warp has to be waited for
+            // coalesced store of the new columns: warp q writes rows 32q .. 32q+31
             if (ok) {
-                // lane owns columns lane and lane + 32; eight rows per batch so
-                // the shared loads of a batch are in flight together
+                // lane owns columns lane and lane + 32, four rows a read
                 const int nr = (int)min((int64_t)32, N - row0 - 32 * q);
-                float* fbase = F + (row0 + 32 * q) * ldF + r;
+                float* fr = F + (row0 + 32 * q) * ldF + r + lane;
                 const bool c1 = lane < nacc, c2 = lane + 32 < nacc;
-#pragma unroll 8
-                for (int rr = 0; rr < 32; ++rr) {
-                    if (rr < nr) {
-                        const float* grow = gbuf + (32 * q + rr) * kGPitch;
-                        const float v1 = grow[lane], v2 = grow[lane + 32];
-                        if (c1) fbase[(int64_t)rr * ldF + lane] = v1;
-                        if (c2) fbase[(int64_t)rr * ldF + lane + 32] = v2;
-                    }
+#pragma unroll 4
+                for (int h = 0; h < 8; ++h) {
+                    const float4 v1 = *reinterpret_cast<const float4*>(gbuf + g_chunk(lane, 8 * q + h));
+                    const float4 v2 = *reinterpret_cast<const float4*>(gbuf + g_chunk(lane + 32, 8 * q + h));
+                    const float a1[4] = {v1.x, v1.y, v1.z, v1.w}, a2[4] = {v2.x, v2.y, v2.z, v2.w};
+#pragma unroll
+                    for (int rr = 0; rr < 4; ++rr, fr += ldF)
+                        if (4 * h + rr < nr) {
+                            if (c1) fr[0] = a1[rr];
+                            if (c2) fr[32] = a2[rr];
+                        }
                 }
             }
             __syncwarp();
@@ -646,8 +671,7 @@ PFN_cuTensorMapEncodeTiled_v12000 get_encode() {
 }  // namespace
 
 constexpr size_t kUpdSmem =
-    (size_t)kStages * kStageBytes + 2 * kAOp + kCols * kCols * 4 + kRows * kGPitch * 4 + sizeof(Bars) + 1024;
-static_assert(kUpdSmem <= 227 * 1024, "shared memory per CTA");
+    (size_t)kStages * kStageBytes + 2 * kAOp + kCols * kCols * 4 + kRows * kCols * 4 + sizeof(Bars) + 1024;
 static_assert(kUpdSmem <= 227 * 1024, "shared memory per CTA");
 
 // Whether the tensor-core update can run for this factor layout.
