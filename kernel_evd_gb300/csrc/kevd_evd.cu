@@ -410,7 +410,8 @@ __global__ void evt_zf_kernel(const double* __restrict__ Z, int64_t k, int m, in
 // CTA = 128 threads on 256 rows; thread t forms columns 16 h .. 16 h + 15 (h = t & 1)
 // of the four rows 4 (t >> 1) .. +3 as packed pairs of columns: a 16-byte read of F
 // (the next four columns' are in flight) and four of Z for 32 packed FMA.
-// N = 2M, k = 2000: U_FIG
+// N = 2M, k = 2,000: 6.0 ms (8.9 with scalar FMAs, 32 columns by 256 threads; FP32
+// pipe 3.5).
 constexpr int kUChunk = 64;
 __global__ void __launch_bounds__(128, 4)
 evt_u_kernel(const float* __restrict__ FT, int64_t ldT, int64_t N, int64_t k, const float* __restrict__ Zf, int m,
@@ -510,7 +511,7 @@ evt_u_kernel(const float* __restrict__ FT, int64_t ldT, int64_t N, int64_t k, co
 // bank groups), Y as [row][q].  FP32 products and 8-row FP32 partials (round to
 // nearest: their errors are unbiased and average out in H); the partials are added
 // with compensation over the CTA's row range.
-// FP32 pipe: 32 (1 + 4 / 8) operations per element of F.  N = 2M, k = 2000: T1_FIG
+// FP32 pipe: 32 (1 + 4 / 8) operations per element of F.
 constexpr int kT1Rows = 32;
 constexpr int kT1Cols = 128;
 constexpr int kT1Buf = kT1Cols * kT1Rows + kT1Rows * 32;   // floats of one buffer
@@ -621,7 +622,8 @@ evt_t1_kernel(const float* __restrict__ FT, int64_t ldT, int64_t N, int64_t k, c
 // memory, 8-term FP32 partials added with compensation); for H and M thread t owns
 // entries (8 (t >> 5) + r, t & 31), r < 8, of the 32 x 32 matrices, summed over 64
 // rows with compensation and beyond in FP64.
-// FP32 pipe: 32 (2 + 4 / 8) operations per element of F.  N = 2M, k = 2000: HM_FIG
+// FP32 pipe: 32 (2 + 4 / 8) operations per element of F.  N = 2M, k = 2,000: with
+// T1 and the rotation 21.6 ms (26.6 with scalar FMAs and 4 x 4 tiles; FP32 pipe 14.4).
 constexpr int kHmRows = 128;
 constexpr int kHmFChunk = 32 * kHmRows;                 // floats of an F chunk, [column j][row i]
 constexpr int kHmBuf = kHmFChunk + 2 * 32 * 32;         // and the T1 hi and lo chunks

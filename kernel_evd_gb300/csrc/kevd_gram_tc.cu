@@ -108,6 +108,7 @@ struct Barriers {
     uint64_t empty[kMaxStages];
     uint64_t tfree[4];
     uint64_t accf;
+    uint64_t accf2;   // second Gram (pair kernel)
     uint64_t acce[2];
     uint64_t done;
     uint32_t tmem_base;
@@ -185,8 +186,7 @@ __device__ __forceinline__ void store_b_split(uint8_t* breg, int m, const float 
 //     per stage and Gram; the raw b tile is b-hi, b-lo an FP32 tile.
 template <int NG, bool F16>
 __global__ void __launch_bounds__(kThreads, 1)
-gram_tc_kernel(const __grid_constant__ CUtensorMap tmF, const float* __restrict__ w2a, const float* __restrict__ w2b,
-               GramExp ex, int64_t N, int64_t k, int n_tiles, int64_t rows_per,
+gram_tc_kernel(const __grid_constant__ CUtensorMap tmF, const float* __restrict__ w2, GramExp ex, int64_t N, int64_t k, int n_tiles, int64_t rows_per,
                double* __restrict__ partial, float* __restrict__ scratch, int n_scratch, int* __restrict__ err) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* base = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -254,8 +254,7 @@ gram_tc_kernel(const __grid_constant__ CUtensorMap tmF, const float* __restrict_
                 uint8_t* st = base + (size_t)slot * kStageBytes;
                 const int x = (int)(r0 + s * kTK);
                 tc::mbar_arrive_expect_tx(&bar->tma[slot], bytes);
-                tc::bulk_load(bar->w2[slot][0], w2a + x, kTK * 4, &bar->tma[slot]);
-                if (NG == 2) tc::bulk_load(bar->w2[slot][1], w2b + x, kTK * 4, &bar->tma[slot]);
+                tc::bulk_load(bar->w2[slot][0], w2 + (size_t)x * NG, NG * kTK * 4, &bar->tma[slot]);
                 tc::tma_load_2d(st, &tmF, x, (int)a0, &bar->tma[slot]);
                 if (!diag) tc::tma_load_2d(st + kOffB, &tmF, x, (int)b0, &bar->tma[slot]);
             }
@@ -498,6 +497,324 @@ gram_tc_kernel(const __grid_constant__ CUtensorMap tmF, const float* __restrict_
     if (warp == kMmaWarp) tc::tmem_dealloc(tbase, kTmemCols);
 }
 
+// The f16 form on CTA pairs: a cluster of two CTAs forms the tiles (2 I, J) and
+// (2 I + 1, J) as one M = 256 tile (cta_group::2).  Each CTA loads and weights its
+// own a tile, and loads and splits half of the b tile's rows; CTA 0's MMA thread
+// issues for both CTAs.
+//
+// Why: the single-CTA form is bound by its shared memory.  Per stage it writes
+// 32 KB and reads 48 KB by TMA and converters, writes 16 KB of split b, and the
+// tensor core reads the 4 KB of b of each of the 12 MMAs for 128 rows only.  Halving
+// the loads alone took 12 % off its time, no b split another 17 %.  A pair reads each
+// half of b once for 256 rows, and loads, reads and writes half of the b tile.
+// Every accumulator takes the same MMAs in the same order, flushed at the same rows.
+// N = 500,000, k = 2,000: two Grams 12.8 -> 11.1 ms, one 9.1 -> 7.3 ms.  Without loads
+// and converters the MMAs and their hand-over take 7.6 ms.
+//
+// Roles as above, except: an MMA thread per Gram; warps 4-7 and 14-17 convert a in alternate stages (the
+// warps have 96 registers a thread); b converters: two threads a row (16 of the 32 values each);
+// the "converted" barriers and the accumulator hand-back are counted in CTA 0, slot
+// and accumulator releases are multicast to both CTAs.
+constexpr int kPairB = kTT / 2;                        // b rows per CTA
+constexpr int kPairStages = 6;
+constexpr int kPairCvtA1 = 14;                         // warps 14-17: a operand of the odd stages
+constexpr int kPairMma1 = 18;                          // MMA issuer of the second Gram
+template <int NG> constexpr int kPairThreads = (NG == 2 ? 19 : 18) * 32;
+constexpr int kPairStageBytes = kOpBytes + kPairB * kTK * 4;
+static_assert(kFlushStages % kPairStages == 0 && kPairStages <= kMaxStages, "ring shape");
+constexpr size_t kPairSmem = (size_t)kPairStages * kPairStageBytes + sizeof(Barriers) + 1024;
+
+// pair-tile p -> (I, J), J <= 2 I + 1
+__device__ __forceinline__ void pair_of(int64_t p, int64_t nt, int64_t& I, int64_t& J) {
+    I = 0;
+    while (true) {   // at most nt / 2 steps, once per CTA
+        const int64_t n = min(nt, 2 * I + 2);
+        if (p < n) break;
+        p -= n;
+        ++I;
+    }
+    J = p;
+}
+
+template <int NG>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads<NG>, 1)
+gram_tc_pair_kernel(const __grid_constant__ CUtensorMap tmF, const __grid_constant__ CUtensorMap tmB,
+                    const float* __restrict__ w2, GramExp ex, int64_t N, int64_t k, int n_tiles, int n_pairs,
+                    int64_t rows_per, double* __restrict__ partial, float* __restrict__ scratch, int n_scratch,
+                    int* __restrict__ err) {
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* base = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    Barriers* bar = reinterpret_cast<Barriers*>(base + (size_t)kPairStages * kPairStageBytes);
+    using SL = Slots<true>;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t rank = tc::cluster_rank();
+    const int64_t nt = (k + kTT - 1) / kTT;
+    const int64_t cl = blockIdx.x >> 1;
+    const int64_t split = cl / n_pairs;
+    int64_t I, tb;
+    pair_of(cl % n_pairs, nt, I, tb);
+    const int64_t ta = 2 * I + rank;
+    const bool valid = ta < nt && tb <= ta;   // (2 I, 2 I + 1) and a row past the last are not wanted
+    const int64_t a0 = ta * kTT, b0 = tb * kTT;
+    const int64_t r0 = split * rows_per;
+    const int64_t r1 = min(N, r0 + rows_per);
+    const int n_stages = (r1 > r0) ? (int)((r1 - r0 + kTK - 1) / kTK) : 0;
+    const int n_chunks = (n_stages + kFlushStages - 1) / kFlushStages;
+    double* out = partial + (split * n_tiles + (ta * (ta + 1) / 2 + tb)) * NG * kTT * kTT;   // [G][n][m]
+    uint32_t smid, nsmid;
+    asm volatile("mov.u32 %0, %%smid;" : "=r"(smid));
+    asm volatile("mov.u32 %0, %%nsmid;" : "=r"(nsmid));
+    if (nsmid > (uint32_t)n_scratch) {   // both CTAs alike
+        if (threadIdx.x == 0) atomicExch(err, 7);
+        return;
+    }
+    float* scr = scratch + (size_t)smid * NG * kTT * kTT;   // [G][n][m]
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < kPairStages; ++s) {
+            tc::mbar_init(&bar->tma[s], 1);
+            tc::mbar_init(&bar->full[s], 2 * kCvtWarps);
+            tc::mbar_init(&bar->empty[s], NG);
+        }
+        for (int t = 0; t < SL::n; ++t) tc::mbar_init(&bar->tfree[t], NG);
+        tc::mbar_init(&bar->accf, 1);
+        tc::mbar_init(&bar->accf2, 1);
+        tc::mbar_init(&bar->acce[0], 2 * kEpiWarps);
+        tc::mbar_init(&bar->acce[1], 2 * kEpiWarps);
+        tc::mbar_init(&bar->done, NG);
+        tc::mbar_fence_init();
+    }
+    if (warp == kMmaWarp) tc::tmem_alloc_pair(&bar->tmem_base, kTmemCols);
+    __syncwarp();
+    tc::tc_fence_before();
+    tc::cluster_sync();
+    tc::tc_fence_after();
+    const uint32_t tbase = bar->tmem_base;
+
+    if (warp == kProdWarp) {
+        if (lane == 0) {
+            int slot = 0;
+            uint32_t use = 0;
+            for (int s = 0; s < n_stages; ++s) {
+                if (!tc::mbar_wait(&bar->empty[slot], (use & 1u) ^ 1u, kTimeoutNs)) {
+                    atomicExch(err, 21);
+                    break;
+                }
+                uint8_t* st = base + (size_t)slot * kPairStageBytes;
+                const int x = (int)r0 + s * kTK;
+                tc::mbar_arrive_expect_tx(&bar->tma[slot], kPairStageBytes + NG * kTK * 4);
+                tc::tma_load_2d(st, &tmF, x, (int)a0, &bar->tma[slot]);
+                tc::tma_load_2d(st + kOffB, &tmB, x, (int)b0 + kPairB * (int)rank, &bar->tma[slot]);
+                tc::bulk_load(bar->w2[slot][0], w2 + (size_t)x * NG, NG * kTK * 4, &bar->tma[slot]);
+                if (++slot == kPairStages) {
+                    slot = 0;
+                    ++use;
+                }
+            }
+        }
+        __syncwarp();
+    } else if ((warp >= kCvtWarp0 && warp < kCvtWarp0 + 4) || (warp >= kPairCvtA1 && warp < kPairCvtA1 + 4)) {
+        // a converters of the even or the odd stages
+        const int m = 32 * (warp & 3) + lane;
+        const uint32_t ta_ = tbase + ((uint32_t)(32 * (warp & 3)) << 16) + kTmemA;
+        const int64_t cm = a0 + m;
+        const float as0 = (cm < k) ? ldexpf(1.f, ex.ea0[cm]) : 1.f;
+        const float as1 = (cm < k && NG == 2) ? ldexpf(1.f, ex.ea1[cm]) : 1.f;
+        const int g1 = warp >= kPairCvtA1 ? 1 : 0;
+        int slot = g1, ts = g1;
+        uint32_t use = 0, tuse = 0;
+        for (int s = g1; s < n_stages; s += 2) {
+            if (!tc::mbar_wait(&bar->tma[slot], use & 1u, kTimeoutNs)) {
+                atomicExch(err, 25);
+                break;
+            }
+            float x[32];
+            load_row(base + (size_t)slot * kPairStageBytes, m, x);
+            if (!tc::mbar_wait(&bar->tfree[ts], (tuse & 1u) ^ 1u, kTimeoutNs)) {
+                atomicExch(err, 26);
+                break;
+            }
+            tc::tc_fence_after();
+#pragma unroll
+            for (int gsel = 0; gsel < NG; ++gsel) {
+                const float as = gsel ? as1 : as0;
+                const uint32_t tg = ta_ + (uint32_t)ts * SL::cols + SL::gram_cols * gsel;
+#pragma unroll
+                for (int hf = 0; hf < 2; ++hf) {   // 16 rows: 8 words of hi pairs, 8 of lo
+                    uint32_t h[8], l[8];
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        const float* xc = x + 16 * hf + 4 * c;
+                        const float4 wv = reinterpret_cast<const float4*>(bar->w2[slot][gsel])[4 * hf + c];
+                        tc::split_f16x2((xc[0] * wv.x) * as, (xc[1] * wv.y) * as, h[2 * c], l[2 * c]);
+                        tc::split_f16x2((xc[2] * wv.z) * as, (xc[3] * wv.w) * as, h[2 * c + 1], l[2 * c + 1]);
+                    }
+                    tc::tmem_st8u(tg + 8u * hf, h);
+                    tc::tmem_st8u(tg + SL::lo_off + 8u * hf, l);
+                }
+            }
+            tc::tmem_wait_st();
+            tc::tc_fence_before();
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive_leader(&bar->full[slot]);
+            if ((slot += 2) >= kPairStages) {
+                slot -= kPairStages;
+                ++use;
+            }
+            if ((ts += 2) >= SL::n) {
+                ts -= SL::n;
+                ++tuse;
+            }
+        }
+    } else if (warp >= kCvtBWarp0 && warp < kCvtBWarp0 + 4) {
+        // b converters: row m of this CTA's half, its values 16 hf .. 16 hf + 15
+        const int e = threadIdx.x - 32 * kCvtBWarp0, m = e >> 1, hf = e & 1;
+        const int64_t cm = b0 + kPairB * rank + m;
+        const float bscale = (cm < k) ? ldexpf(1.f, ex.eb[cm]) : 1.f;
+        const uint32_t atom = (uint32_t)(m >> 3) * 1024u;
+        int slot = 0;
+        uint32_t use = 0;
+        for (int s = 0; s < n_stages; ++s) {
+            if (!tc::mbar_wait(&bar->tma[slot], use & 1u, kTimeoutNs)) {
+                atomicExch(err, 25);
+                break;
+            }
+            uint8_t* breg = base + (size_t)slot * kPairStageBytes + kOffB;
+            float4 v[4];
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+                v[c] = *reinterpret_cast<const float4*>(breg + tc::sw128_off((uint32_t)m, (uint32_t)(16 * hf + 4 * c)));
+            __syncwarp();   // the warp's raw rows are read before its atoms are rewritten
+            uint32_t h[8], l[8];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                tc::split_f16x2(v[c].x * bscale, v[c].y * bscale, h[2 * c], l[2 * c]);
+                tc::split_f16x2(v[c].z * bscale, v[c].w * bscale, h[2 * c + 1], l[2 * c + 1]);
+            }
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                const uint32_t off = atom + tc::sw64_off16((uint32_t)(m & 7), (uint32_t)(16 * hf + 8 * c));
+                *reinterpret_cast<uint4*>(breg + off) = make_uint4(h[4 * c], h[4 * c + 1], h[4 * c + 2], h[4 * c + 3]);
+                *reinterpret_cast<uint4*>(breg + off + 512) =
+                    make_uint4(l[4 * c], l[4 * c + 1], l[4 * c + 2], l[4 * c + 3]);
+            }
+            tc::fence_async_smem();
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive_leader(&bar->full[slot]);
+            if (++slot == kPairStages) {
+                slot = 0;
+                ++use;
+            }
+        }
+    } else if (warp == kMmaWarp || (NG == 2 && warp == kPairMma1)) {
+        // MMA issuers, one per Gram: the tensor core holds few MMAs queued, so the
+        // wait between two stages (some 300 clocks of a stage's 768) would leave it
+        // idle; with two issuers the other Gram's MMAs fill it
+        if (lane == 0 && rank == 0) {
+            constexpr uint32_t idesc = tc::idesc_f16(2 * kTT, kTT);
+            constexpr int kSteps = kTK / 16;
+            const uint32_t gsel = warp == kMmaWarp ? 0u : 1u;
+            uint64_t* accf = gsel ? &bar->accf2 : &bar->accf;
+            const uint32_t d = tbase + gsel * kTT;
+            const uint32_t a_g = tbase + kTmemA + SL::gram_cols * gsel;
+            // b-hi tile of stage 0; stage sl is kPairStageBytes / 16 further, b-lo 512
+            // bytes, a K step 32 bytes
+            const uint64_t db0 = tc::desc_sw64_sbo1024(tc::smem_u32(base + kOffB));
+            bool ok = true;
+            uint32_t use = 0, ts = 0;
+            for (int c = 0; c < n_chunks && ok; ++c) {
+                const int s0 = c * kFlushStages;
+                const int s1 = min(n_stages, s0 + kFlushStages);
+                if (c > 0) {   // both epilogues have read the previous chunk
+                    ok = tc::mbar_wait(&bar->acce[gsel], (uint32_t)((c - 1) & 1), kTimeoutNs);
+                    tc::tc_fence_after();
+                }
+                for (int sb = s0; sb < s1 && ok; sb += kPairStages, ++use) {
+#pragma unroll
+                    for (int sl = 0; sl < kPairStages; ++sl) {
+                        if (sb + sl >= s1) break;
+                        if (!tc::mbar_wait(&bar->full[sl], use & 1u, kTimeoutNs)) {
+                            ok = false;
+                            break;
+                        }
+                        tc::tc_fence_after();
+                        const uint32_t ahi = a_g + ts * SL::cols, alo = ahi + SL::lo_off;
+                        const uint64_t dbh = db0 + (uint64_t)(sl * (kPairStageBytes / 16));
+                        const uint64_t dbl = dbh + 512 / 16;
+                        const uint32_t acc0 = (sb + sl == s0) ? 0u : 1u;
+#pragma unroll
+                        for (int j = 0; j < kSteps; ++j) {
+                            tc::mma_f16_tmem_a_pair(d, ahi + 8u * j, dbl + 2 * j, idesc, j > 0 ? 1u : acc0);
+                            tc::mma_f16_tmem_a_pair(d, alo + 8u * j, dbh + 2 * j, idesc, 1u);
+                        }
+#pragma unroll
+                        for (int j = 0; j < kSteps; ++j)
+                            tc::mma_f16_tmem_a_pair(d, ahi + 8u * j, dbh + 2 * j, idesc, 1u);
+                        tc::mma_commit_pair(&bar->empty[sl]);
+                        tc::mma_commit_pair(&bar->tfree[ts]);
+                        ts = (ts + 1u) & (uint32_t)(SL::n - 1);
+                    }
+                }
+                if (ok) tc::mma_commit_pair(accf);
+            }
+            if (!ok) atomicExch(err, 22);
+            // retire every issued MMA before the TMEM is released
+            tc::mma_commit_pair(&bar->done);
+            if (!tc::mbar_wait(&bar->done, 0u, kTimeoutNs)) atomicExch(err, 23);
+        }
+        __syncwarp();
+    } else if (warp < kEpiWarps) {
+        // epilogue: as in the single-CTA kernel; a tile that is not wanted only
+        // hands its accumulators back
+        const int m = warp * 32 + lane;
+        if (valid)
+            for (int n = 0; n < NG * kTT; ++n) out[n * kTT + m] = 0.0;
+        bool ok = true;
+        for (int c = 0; c < n_chunks && ok; ++c) {
+#pragma unroll 1
+            for (int gsel = 0; gsel < NG; ++gsel) {
+                if (!tc::mbar_wait(gsel ? &bar->accf2 : &bar->accf, (uint32_t)(c & 1), kTimeoutNs)) {
+                    atomicExch(err, 24);
+                    ok = false;
+                    break;
+                }
+                tc::tc_fence_after();
+                const uint32_t tacc = tbase + ((uint32_t)(warp * 32) << 16) + (uint32_t)(gsel * kTT);
+                float* srow = scr + (size_t)gsel * kTT * kTT + m;
+#pragma unroll 1
+                for (int cb = 0; cb < (valid ? kTT / 32 : 0); ++cb) {
+                    float v[32];
+                    tc::tmem_ld32(tacc + 32u * cb, v);
+                    tc::tmem_wait_ld();
+#pragma unroll
+                    for (int n = 0; n < 32; ++n) srow[(32 * cb + n) * kTT] = v[n];
+                }
+                tc::tc_fence_before();
+                __syncwarp();
+                if (lane == 0) tc::mbar_arrive_leader(&bar->acce[gsel]);
+            }
+            if (!valid || !ok) continue;
+#pragma unroll 1
+            for (int e0 = 0; e0 < NG * kTT; e0 += 16) {
+                double o[16];
+                float v[16];
+#pragma unroll
+                for (int u = 0; u < 16; ++u) {
+                    o[u] = out[(size_t)(e0 + u) * kTT + m];
+                    v[u] = scr[(size_t)(e0 + u) * kTT + m];
+                }
+#pragma unroll
+                for (int u = 0; u < 16; ++u) out[(size_t)(e0 + u) * kTT + m] = o[u] + (double)v[u];
+            }
+        }
+    }
+    __syncwarp();
+    tc::tc_fence_before();
+    tc::cluster_sync();
+    tc::tc_fence_after();
+    if (warp == kMmaWarp) tc::tmem_dealloc_pair(tbase, kTmemCols);
+}
+
 // max and min of s_i^2 over i < N of each weight vector: mx[g] (atomicMax,
 // starts at 0) and mx[2 + g] (atomicMin, starts at all ones), float bits of
 // non-negative values, so unsigned order is float order.
@@ -539,13 +856,15 @@ __device__ __forceinline__ int f16_range_exp(double v) {
     return 14 - e;
 }
 
-// w2[i] = s_i^2 rounded to FP32 for i < N, zero up to len (the last stage of
-// the last row split may run past N).
+// s_i^2 rounded to FP32 for i < N, zero up to len (the last stage of the last row
+// split may run past N), the weights of a stage's kTK rows together: [stage][Gram][row].
 __global__ void gram_w2_kernel(const double* __restrict__ s, const double* __restrict__ s2, int64_t N, int64_t len,
-                               float* __restrict__ w2, float* __restrict__ w22) {
+                               float* __restrict__ w2) {
+    const int nG = s2 ? 2 : 1;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < len; i += (int64_t)gridDim.x * blockDim.x) {
-        w2[i] = (i < N) ? (float)(s[i] * s[i]) : 0.f;
-        if (s2) w22[i] = (i < N) ? (float)(s2[i] * s2[i]) : 0.f;
+        float* w = w2 + (i / kTK) * kTK * nG + i % kTK;
+        w[0] = (i < N) ? (float)(s[i] * s[i]) : 0.f;
+        if (s2) w[kTK] = (i < N) ? (float)(s2[i] * s2[i]) : 0.f;
     }
 }
 
@@ -684,6 +1003,14 @@ int run_transpose_f32(kevd_ctx* ctx, const float* F, int64_t ldF, int64_t N, int
     return KEVD_OK;
 }
 
+// Cost of a CTA of the pair kernel against one of gram_tc_kernel on the same rows:
+// the pairs also form the tiles (2 I, 2 I + 1) and, with an odd number of tile rows,
+// a row past the last, so they are taken where 2 n_pairs kPairCost <= n_tiles.
+// Times pair / single, two Grams: k = 2,000 (N = 500,000) 11.1 / 12.8 ms, 1,000
+// (200,000) 1.55 / 1.81, 768 1.02 / 1.09, 1,920 (100,000) 2.36 / 2.39 (142 for 120
+// tiles); the other way 500 0.65 / 0.65 and 640 1.15 / 0.96 (22 for 15 tiles).
+constexpr double kPairCost = 0.84;
+
 // Shared host path of the one- and two-Gram kernels (s2 == nullptr: one).
 static int gram_tc_impl(kevd_ctx* ctx, const float* FT, int64_t ldT, int64_t N, int64_t k, const unsigned* colmax,
                         const double* s, const double* s2, double* G, double* G2, cudaStream_t st) {
@@ -692,13 +1019,13 @@ static int gram_tc_impl(kevd_ctx* ctx, const float* FT, int64_t ldT, int64_t N, 
     if (!enc) return set_error(ctx, KEVD_ERR_CUDA, "gram_tc: cuTensorMapEncodeTiled unavailable");
     if ((ldT % 4) != 0 || ((uintptr_t)FT % 16) != 0)
         return set_error(ctx, KEVD_ERR_ARG, "gram_tc: FT must be 16-byte aligned with ldT %% 4 == 0");
-    CUtensorMap tmF;
-    {
+    CUtensorMap tmF, tmB;   // boxes of kTT columns (an a or b tile) and of kPairB (a CTA's half of b)
+    for (const int box_cols : {kTT, kPairB}) {
         const cuuint64_t gdim[2] = {(cuuint64_t)N, (cuuint64_t)k};
         const cuuint64_t gstride[1] = {(cuuint64_t)ldT * 4};
-        const cuuint32_t box[2] = {(cuuint32_t)kTK, (cuuint32_t)kTT};
+        const cuuint32_t box[2] = {(cuuint32_t)kTK, (cuuint32_t)box_cols};
         const cuuint32_t estr[2] = {1, 1};
-        CUresult cr = enc(&tmF, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, (void*)FT, gdim, gstride, box, estr,
+        CUresult cr = enc(box_cols == kTT ? &tmF : &tmB, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, (void*)FT, gdim, gstride, box, estr,
                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                           CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         if (cr != CUDA_SUCCESS) return set_error(ctx, KEVD_ERR_CUDA, "gram_tc: tensor map (F) failed (%d)", (int)cr);
@@ -719,11 +1046,9 @@ static int gram_tc_impl(kevd_ctx* ctx, const float* FT, int64_t ldT, int64_t N, 
     int* err = arena_get<int>(ctx, "tc.err", 1, &rc);
     unsigned* wmax = arena_get<unsigned>(ctx, "tc.wmax", 4, &rc);   // max, max, min, min
     int* exps = arena_get<int>(ctx, "tc.exps", (size_t)3 * k, &rc);   // eb, ea0, ea1
-    // squared weights, one 128-byte bulk copy per stage (row offsets are
-    // multiples of 32, so every copy is 128-byte aligned)
+    // squared weights, one bulk copy of 128 bytes a Gram per stage
     const int64_t w2_len = (N + kTK - 1) / kTK * kTK + kTK;
-    float* w2 = arena_get<float>(ctx, "tc.w2", (size_t)w2_len, &rc);
-    float* w22 = s2 ? arena_get<float>(ctx, "tc.w2b", (size_t)w2_len, &rc) : nullptr;
+    float* w2 = arena_get<float>(ctx, "tc.w2", (size_t)w2_len * nG, &rc);
     // FP32 flush staging indexed by SM id (ids below %nsmid; the kernel checks
     // the bound and reports code 7 if it is exceeded)
     const int n_scratch = std::max(256, 2 * ctx->num_sms);
@@ -735,7 +1060,7 @@ static int gram_tc_impl(kevd_ctx* ctx, const float* FT, int64_t ldT, int64_t N, 
     const int wgrid = (int)std::min<int64_t>((w2_len + 255) / 256, (int64_t)ctx->num_sms * 8);
     gram_wmax_kernel<<<wgrid, 256, 0, st>>>(s, s2, N, wmax);
     KEVD_LAUNCH(ctx);
-    gram_w2_kernel<<<wgrid, 256, 0, st>>>(s, s2, N, w2_len, w2, w22);
+    gram_w2_kernel<<<wgrid, 256, 0, st>>>(s, s2, N, w2_len, w2);
     KEVD_LAUNCH(ctx);
     // the split: f16 when every Gram's weights span at most kF16WeightRange
     // (the host reads the four extremes), else tf32
@@ -762,12 +1087,22 @@ static int gram_tc_impl(kevd_ctx* ctx, const float* FT, int64_t ldT, int64_t N, 
         auto launch = [&](auto kern) -> int {
             const size_t smem = f16 ? smem_bytes<true>() : smem_bytes<false>();
             KEVD_CUDA(ctx, raise_smem_limit(reinterpret_cast<const void*>(kern), (int)smem));
-            kern<<<grid, kThreads, smem, st>>>(tmF, w2, nG == 2 ? w22 : w2, ex, N, k, n_tiles, rows_per,
-                                                      partial, scratch, n_scratch, err);
+            kern<<<grid, kThreads, smem, st>>>(tmF, w2, ex, N, k, n_tiles, rows_per, partial, scratch, n_scratch, err);
             KEVD_LAUNCH(ctx);
             return KEVD_OK;
         };
-        if (nG == 1) {
+        int n_pairs = 0;
+        for (int I = 0; 2 * I < nt; ++I) n_pairs += std::min(nt, 2 * I + 2);
+        if (f16 && (double)(2 * n_pairs) * kPairCost <= (double)n_tiles) {
+            auto pair = [&](auto kern) -> int {
+                KEVD_CUDA(ctx, raise_smem_limit(reinterpret_cast<const void*>(kern), kPairSmem));
+                kern<<<2 * n_pairs * n_split, nG == 1 ? kPairThreads<1> : kPairThreads<2>, kPairSmem, st>>>(tmF, tmB, w2, ex, N, k, n_tiles, n_pairs,
+                                                                        rows_per, partial, scratch, n_scratch, err);
+                KEVD_LAUNCH(ctx);
+                return KEVD_OK;
+            };
+            KEVD_TRY(nG == 1 ? pair(&gram_tc_pair_kernel<1>) : pair(&gram_tc_pair_kernel<2>));
+        } else if (nG == 1) {
             KEVD_TRY(f16 ? launch(&gram_tc_kernel<1, true>) : launch(&gram_tc_kernel<1, false>));
         } else {
             KEVD_TRY(f16 ? launch(&gram_tc_kernel<2, true>) : launch(&gram_tc_kernel<2, false>));
