@@ -59,6 +59,7 @@ constexpr int kAPlane = kM * kKs * 2, kBPlane = kN * kKs * 2;
 constexpr int kStageBytes = kSlices * (kAPlane + kBPlane);
 constexpr int kThreads = 512;
 constexpr int kWarps = kThreads / 32;
+constexpr int kAWarps = 8, kBWarps = 4;      // expand the digits of A and of B
 constexpr int kMmaWarp = kWarps - 1;         // its lane 0 issues the MMAs
 constexpr uint32_t kTmemCols = 512;
 constexpr uint64_t kTimeoutNs = 4000000000ull;
@@ -102,15 +103,14 @@ __device__ __forceinline__ int digits_exp(uint64_t abs_bits) {
     return ex - 1023 + ((abs_bits & 0xfffffffffffffull) ? 1 : 0);
 }
 
-// n = 4 or 8 packed entries along K -> the 8- or 16-byte piece of each plane.
-template <int n>
-__device__ __forceinline__ void store_planes(const uint64_t (&w)[n], uint8_t* planes, int plane_bytes, uint32_t off) {
-    uint32_t h[kSlices][n / 2];
+// Eight packed entries along K -> the 16-byte piece of each plane.
+__device__ __forceinline__ void store_planes(const uint64_t (&w)[8], uint8_t* planes, int plane_bytes, uint32_t off) {
     const __half2 bias = __half2half2(__ushort_as_half((unsigned short)0xE480));   // -1152
 #pragma unroll
-    for (int p = 0; p < n / 2; ++p) {
+    for (int word = 0; word < 2; ++word) {   // digits 0 .. 3 in the high word, 4 .. 7 in the low one
+        uint32_t h[4][4];
 #pragma unroll
-        for (int word = 0; word < 2; ++word) {   // digits 0 .. 3 in the high word, 4 .. 7 in the low one
+        for (int p = 0; p < 4; ++p) {
             const uint32_t x0 = (uint32_t)(w[2 * p] >> (word ? 0 : 32)), x1 = (uint32_t)(w[2 * p + 1] >> (word ? 0 : 32));
             // the same bytes of both entries side by side: two digits per register
             const uint32_t g[2] = {__byte_perm(x0, x1, 0x6273), __byte_perm(x0, x1, 0x4051)};
@@ -119,15 +119,13 @@ __device__ __forceinline__ void store_planes(const uint64_t (&w)[n], uint8_t* pl
                 // 0x64uu is the f16 1024 + u; minus 1152 leaves the digit u - 128
                 const uint32_t v = __byte_perm(g[s >> 1], 0x64646464u, (s & 1) ? 0x4342 : 0x4140);
                 const __half2 d = __hadd2(*reinterpret_cast<const __half2*>(&v), bias);
-                h[4 * word + s][p] = *reinterpret_cast<const uint32_t*>(&d);
+                h[s][p] = *reinterpret_cast<const uint32_t*>(&d);
             }
         }
-    }
 #pragma unroll
-    for (int s = 0; s < kSlices; ++s) {
-        uint8_t* o = planes + s * plane_bytes + off;
-        if constexpr (n == 8) *reinterpret_cast<uint4*>(o) = make_uint4(h[s][0], h[s][1], h[s][2], h[s][3]);
-        else *reinterpret_cast<uint2*>(o) = make_uint2(h[s][0], h[s][1]);
+        for (int s = 0; s < 4; ++s)
+            *reinterpret_cast<uint4*>(planes + (4 * word + s) * plane_bytes + off) =
+                make_uint4(h[s][0], h[s][1], h[s][2], h[s][3]);
     }
 }
 
@@ -152,9 +150,10 @@ __device__ __forceinline__ void ld_here2(const uint64_t* p, uint64_t& a, uint64_
     asm volatile("ld.global.nc.v2.u64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(p));
 }
 
-// n entries along K, from k0 on, of output row m of the tile (zeros from k1 on).
-template <bool kGram, int n>
-__device__ __forceinline__ void load_words(const Operand& o, int m, int64_t k0, int64_t k1, uint64_t (&w)[n]) {
+// Eight entries along K, from k0 on, of output row m of the tile (zeros from k1 on).
+template <bool kGram>
+__device__ __forceinline__ void load_words(const Operand& o, int m, int64_t k0, int64_t k1, uint64_t (&w)[8]) {
+    constexpr int n = 8;
     const int left = m < o.count ? (int)max((int64_t)0, min((int64_t)n, k1 - k0)) : 0;
     if constexpr (kGram) {
         const uint64_t* src = o.p + k0 * o.ld + o.first + m;
@@ -190,7 +189,7 @@ __device__ __forceinline__ void tile_sums(const Operand& A, const Operand& B, in
     const int64_t n_st = k1 > k0 ? (k1 - k0 + kKs - 1) / kKs : 0;
     if (tid == 0) {
         for (int s = 0; s < 2; ++s) {
-            tc::mbar_init(&bar->full[s], kWarps);
+            tc::mbar_init(&bar->full[s], kAWarps + kBWarps);
             tc::mbar_init(&bar->empty[s], 1);
         }
         for (int d = 0; d < kDiags; ++d) {
@@ -281,33 +280,43 @@ __device__ __forceinline__ void tile_sums(const Operand& A, const Operand& B, in
         tc::mma_commit(&bar->empty[slot]);
         return true;
     };
-    // this thread's share of a stage: eight terms of a row of A, four of a row of B
-    const int am = kGram ? tid & 127 : tid >> 2, ak = 8 * (kGram ? tid >> 7 : tid & 3);
-    const int bm = kGram ? tid & 63 : tid >> 3, bk = 4 * (kGram ? tid >> 6 : tid & 7);
-    const uint32_t aoff = tc::sw64_off16((uint32_t)am, (uint32_t)ak), boff = tc::sw64_off16((uint32_t)bm, (uint32_t)bk);
-    uint64_t wa[8], wb[4];
-    load_words<kGram>(A, am, k0 + ak, k1, wa);
-    load_words<kGram>(B, bm, k0 + bk, k1, wb);
-    for (int64_t s = 0; s < n_st && ok; ++s) {
-        const int slot = (int)(s & 1);
-        if (!tc::mbar_wait(&bar->empty[slot], ((uint32_t)(s >> 1) & 1u) ^ 1u, kTimeoutNs)) {
-            atomicExch(err, 24);
-            ok = false;
-            break;
+    if (warp < kAWarps + kBWarps) {
+        // this thread's share of a stage: two pieces of eight terms of a row of A or of B
+        const bool is_a = warp < kAWarps;
+        const Operand& O = is_a ? A : B;
+        const int t = is_a ? tid : tid - 32 * kAWarps, rows = is_a ? kM : kN;
+        const int m0 = kGram ? t & (rows - 1) : t >> 2, m1 = kGram ? m0 : m0 + rows / 2;
+        const int g0 = kGram ? 8 * (t / rows) : 8 * (t & 3), g1 = kGram ? g0 + 16 : g0;
+        const int plane = is_a ? kAPlane : kBPlane;
+        uint8_t* planes = base + (is_a ? 0 : kSlices * kAPlane);
+        const uint32_t off0 = tc::sw64_off16((uint32_t)m0, (uint32_t)g0), off1 = tc::sw64_off16((uint32_t)m1, (uint32_t)g1);
+        uint64_t w0[8], w1[8];
+        load_words<kGram>(O, m0, k0 + g0, k1, w0);
+        load_words<kGram>(O, m1, k0 + g1, k1, w1);
+        for (int64_t s = 0; s < n_st && ok; ++s) {
+            const int slot = (int)(s & 1);
+            if (!tc::mbar_wait(&bar->empty[slot], ((uint32_t)(s >> 1) & 1u) ^ 1u, kTimeoutNs)) {
+                atomicExch(err, 24);
+                ok = false;
+                break;
+            }
+            const int64_t kn = k0 + (s + 1) * kKs;   // past the end: zeros, never used
+            store_planes(w0, planes + (size_t)slot * kStageBytes, plane, off0);
+            load_words<kGram>(O, m0, kn + g0, k1, w0);
+            store_planes(w1, planes + (size_t)slot * kStageBytes, plane, off1);
+            tc::fence_async_smem();
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(&bar->full[slot]);
+            load_words<kGram>(O, m1, kn + g1, k1, w1);
+            if (s % kBlockStages == 0 && s > 0) drain(s / kBlockStages - 1);
         }
-        uint8_t* st = base + (size_t)slot * kStageBytes;
-        store_planes(wa, st, kAPlane, aoff);
-        store_planes(wb, st + kSlices * kAPlane, kBPlane, boff);
-        tc::fence_async_smem();
-        __syncwarp();
-        if (lane == 0) tc::mbar_arrive(&bar->full[slot]);
-        const int64_t kn = k0 + (s + 1) * kKs;   // past the end: zeros, never used
-        load_words<kGram>(A, am, kn + ak, k1, wa);
-        load_words<kGram>(B, bm, kn + bk, k1, wb);
-        if (s % kBlockStages == 0 && s > 0) drain(s / kBlockStages - 1);
-        if (warp == kMmaWarp) {
-            if (lane == 0 && ok) ok = issue(s);
-            ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
+    } else {
+        for (int64_t s = 0; s < n_st && ok; ++s) {
+            if (s % kBlockStages == 0 && s > 0) drain(s / kBlockStages - 1);
+            if (warp == kMmaWarp) {
+                if (lane == 0 && ok) ok = issue(s);
+                ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
+            }
         }
     }
     if (ok && n_st > 0) drain((n_st - 1) / kBlockStages);
