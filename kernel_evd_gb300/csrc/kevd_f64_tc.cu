@@ -5,14 +5,16 @@
 // entry of its row (of its column for a Gram), q = rn(x 2^(62 - e)) with
 // |x| <= 2^e, and q into eight signed base-256 digits, q = sum_i a_i 256^(7-i)
 // with |a_0| <= 64 and a_i in [-128, 127].  Digits are exact in f16, products of
-// digits and their sums over a block of 128 terms are integers below 2^24, exact
-// in the FP32 accumulators.  The product of two entries is then
+// digits and their sums over a block of 192 terms are integers, exact in the FP32
+// accumulators up to 2^24 (only S_6 and S_7 below can pass that, by a third at most,
+// if the digits of all terms line up at +-128; they then lose units of 2^-60.  Squared
+// distances, whose exact zeros matter, keep blocks of 128 terms: always exact).  The product of two entries is then
 //
 //   x y = 2^(ex + ey) sum_{i,j} a_i b_j 2^(-8 (i + j) - 12)
 //
 // of which the 36 digit pairs with i + j <= 7 are computed, one accumulator per
 // i + j (what is left out is of the size of the last digit's rounding).  Every
-// 128 terms the eight integer sums S_d leave Tensor Memory and are added, still
+// 192 terms the eight integer sums S_d leave Tensor Memory and are added, still
 // exactly, to two 64-bit integers per output,
 //
 //   hi += S_0 2^24 + S_1 2^16 + S_2 2^8 + S_3,   lo likewise from S_4 .. S_7,
@@ -26,17 +28,19 @@
 // CTA (512 threads): output tile 128 x 64, 32 terms per stage, two stages of
 // shared memory (8 digit planes of A, 128 x 32 f16, and of B, 64 x 32 f16,
 // SWIZZLE_64B, 96 KB), eight 64-column accumulators in Tensor Memory (all 512
-// columns).  Every warp loads packed digits (8 bytes per entry; the next stage's
-// while this one is worked on), writes the f16 planes, and every fourth stage
-// drains its part of the accumulators (warp w: lanes 32 (w % 4), columns
-// 16 (w / 4)); one thread also issues the MMAs of a stage, plane i of A against
-// the 8 - i planes of B that it meets, side by side (24 MMAs of up to 256
+// columns).  Warps 0-7 (A) and 8-11 (B) load packed digits (8 bytes per entry; the
+// next stage's while this one is worked on) and write the f16 planes; every sixth
+// stage all warps drain their part of the accumulators (warp w: lanes 32 (w % 4),
+// columns 16 (w / 4)); a thread of warp 15 issues the MMAs of a stage, plane i of A
+// against the 8 - i planes of B that it meets, side by side (24 MMAs of up to 256
 // columns, 2,300 clocks, against 72 of 64 columns that each read A again).
 // Accumulator i is complete after plane i, so the first ones of a block are
 // drained while its last MMAs run.  Every wait is bounded and reports to an error
-// flag.  Gram of 200,000 x 1,000: 11.7 ms with its digits (FP64 pipe 204 ms); a
-// stage takes about 7,000 clocks: the digit expansion of a stage and the MMAs of
-// the one before overlap, and the expansion is the longer.
+// flag.  Gram of 200,000 x 1,000 with its digits: 7.7 ms (FP64 pipe 204 ms); 11.7 with
+// planes written by the issuing warp too, which then took planes and MMAs in turn,
+// 8.6 with blocks of 128 terms.  A stage takes about 4,900 clocks: 2,800 for the MMAs,
+// which read 240 KB of shared memory against 96 KB of stores, the rest mostly the
+// drains, during which the tensor core has at most two stages to work on.
 #include "kevd_internal.cuh"
 #include "kevd_f64_tc.cuh"
 #include "kevd_tc.cuh"
@@ -54,7 +58,7 @@ namespace {
 constexpr int kM = 128, kN = 64, kKs = 32;   // output tile, terms per stage
 constexpr int kSlices = 8;
 constexpr int kDiags = kSlices;              // digit pairs i + j = d, d < 8
-constexpr int kBlockStages = 4;              // 128 terms per integer block
+constexpr int kBlockStages = 6;              // 192 terms per integer block (kernel blocks: 128)
 constexpr int kAPlane = kM * kKs * 2, kBPlane = kN * kKs * 2;
 constexpr int kStageBytes = kSlices * (kAPlane + kBPlane);
 constexpr int kThreads = 512;
@@ -182,7 +186,7 @@ __device__ __forceinline__ void load_words(const Operand& o, int m, int64_t k0, 
 // One 128 x 64 tile: sums over k in [k0, k1) into (hi, lo) of the thread's 16
 // outputs, row 32 (warp % 4) + lane, columns 16 (warp / 4) ...  Called by the
 // whole CTA.
-template <bool kGram>
+template <bool kGram, int kBlockStages = ::kevd::kBlockStages>
 __device__ __forceinline__ void tile_sums(const Operand& A, const Operand& B, int64_t k0, int64_t k1, uint8_t* base,
                                           Bars* bar, int* err, int64_t (&hi)[16], int64_t (&lo)[16]) {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -253,15 +257,6 @@ __device__ __forceinline__ void tile_sums(const Operand& A, const Operand& B, in
         tc::tc_fence_after();
         const uint32_t a0 = tc::smem_u32(base + (size_t)slot * kStageBytes);
         const uint64_t da = tc::desc_sw64(a0), db = tc::desc_sw64(a0 + kSlices * kAPlane);
-        if (first && blk > 0) {   // the block before has left the accumulators
-#pragma unroll 1
-            for (int d = 0; d < kDiags; ++d)
-                if (!tc::mbar_wait(&bar->acce[d], (uint32_t)(blk - 1) & 1u, kTimeoutNs)) {
-                    atomicExch(err, 22);
-                    return false;
-                }
-            tc::tc_fence_after();
-        }
         // plane i of A against planes 0 .. 7 - i of B, which lie one behind the other
         // like the accumulators i .. 7 they go to: MMAs of up to 256 columns
 #pragma unroll
@@ -269,6 +264,15 @@ __device__ __forceinline__ void tile_sums(const Operand& A, const Operand& B, in
 #pragma unroll
             for (int j = 0; j < kSlices - i; j += 4) {
                 const int n = kN * min(4, kSlices - i - j);
+                if (i == 0 && first && blk > 0) {   // the block before has left these accumulators
+#pragma unroll 1
+                    for (int d = j; d < j + 4; ++d)
+                        if (!tc::mbar_wait(&bar->acce[d], (uint32_t)(blk - 1) & 1u, kTimeoutNs)) {
+                            atomicExch(err, 22);
+                            return false;
+                        }
+                    tc::tc_fence_after();
+                }
 #pragma unroll
                 for (int ks = 0; ks < kKs / 16; ++ks)   // +32 bytes of K per MMA
                     mma_f16_ss(tbase + (uint32_t)((i + j) * kN), da + (uint64_t)((i * kAPlane + 32 * ks) >> 4),
@@ -609,7 +613,7 @@ kernel_f64_tc_kernel(const uint64_t* __restrict__ xq, const int64_t* __restrict_
     const Operand A{xq, ldq, i0, min((int64_t)kM, n - i0)};
     const Operand B{sq, ldq, n0, min((int64_t)kN, r - n0)};
     int64_t hi[16], lo[16];
-    tile_sums<false>(A, B, 0, d, base, bar, err, hi, lo);
+    tile_sums<false, 4>(A, B, 0, d, base, bar, err, hi, lo);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t i = i0 + 32 * (warp & 3) + lane;
     if (i >= n) return;
