@@ -20,6 +20,7 @@
 // wherever it sits there.
 #include "kevd_internal.cuh"
 #include "kevd_nystrom.cuh"
+#include "kevd_pairtile.cuh"
 #include "kevd_tc.cuh"
 
 #include <cooperative_groups.h>
@@ -38,6 +39,12 @@ constexpr int kLanesR = 8;      // thread rows of the K tile and of the sums
 constexpr int kFeat = 128;      // features staged at a time
 constexpr int kMinThreads = kLanesR * kLm;
 
+// K tile: Q = 1 [state][landmark]; Q = 4 [landmark][thread row][q], so that the four
+// states of a sum thread are one 16-byte read
+constexpr int kKvPitch = kLanesR * 4 + 4;
+template <int Q>
+__host__ __device__ constexpr int kv_floats() { return Q == 4 ? kLm * kKvPitch : kLanesR * Q * (kLm + 1); }
+
 __host__ __device__ inline int feat_pitch(int d) { return ((d < kFeat ? d : kFeat) + 3) / 4 * 4 + 4; }
 
 // Shared memory of one CTA with Q states per thread row: two landmark tiles,
@@ -47,7 +54,7 @@ size_t smem_bytes(int d, int kc) {
     const size_t p = feat_pitch(d);
     const size_t tiles = (2 * kLm + kLanesR * Q) * p * sizeof(float);
     const size_t w = 2 * (size_t)kLm * kc * sizeof(float2);
-    const size_t kv = (size_t)kLanesR * Q * (kLm + 1) * sizeof(float);
+    const size_t kv = (size_t)kv_floats<Q>() * sizeof(float);
     return std::max(tiles + w + kv, (size_t)kLanesR * Q * kc * sizeof(double));
 }
 
@@ -61,6 +68,20 @@ __device__ __forceinline__ void pair_fma(float& s, float& c, float x, float2 w) 
     const float e = __fadd_rn(__fsub_rn(s, __fsub_rn(t, z)), __fsub_rn(p, z));
     s = t;
     c = __fadd_rn(c, __fmaf_rn(x, w.y, __fadd_rn(pe, e)));
+}
+
+// The same for two states at once (packed pairs: half of the issue slots).  np = -x w.x,
+// so that every difference is an FMA by -1, which rounds as the subtraction does.
+__device__ __forceinline__ void pair_fma2(f32x2& s, f32x2& c, f32x2 x, f32x2 wx, f32x2 nwx, f32x2 wy) {
+    const f32x2 m1 = pack2(-1.f, -1.f);
+    const f32x2 np = mul2(x, nwx);
+    const f32x2 pe = fma2(x, wx, np);
+    const f32x2 t = fma2(np, m1, s);
+    const f32x2 z = fma2(s, m1, t);
+    const f32x2 e1 = fma2(fma2(z, m1, t), m1, s);
+    const f32x2 e = fma2(add2(np, z), m1, e1);
+    s = t;
+    c = add2(c, fma2(x, wy, add2(pe, e)));
 }
 
 // 8-byte global -> shared copy; src_bytes 0 fills zeros.
@@ -92,9 +113,12 @@ __device__ __forceinline__ void stage_rows(const float* __restrict__ src, int64_
 // lane), then thread (rg, c) of 8 x kc adds the step's landmarks, in order, to
 // the sums of states rg + 8 q and column c.  The next step's tiles are in
 // flight meanwhile (cp.async).
-// Q = 4 halves the W loads per product against Q = 1; Q = 1 is for batches
+// Q = 4 halves the W loads per product against Q = 1 and sums pairs of states in
+// packed FP32 (16,384 states against 2,000 landmarks, 33 columns: 1,018 -> 903 us,
+// two thirds of the FP32 pipe; fewer CTAs per 32 states with more landmark groups
+// each is no faster: 923 to 956 us); Q = 1 is for batches
 // that would leave SMs without a CTA otherwise.
-template <int Q>
+template <int Q>   // 1 or 4
 __global__ void __launch_bounds__(544)
 nystrom_eval_kernel(const float* __restrict__ Y, int64_t n, const float* __restrict__ xs,
                     const float2* __restrict__ w, const int* __restrict__ ex, int64_t r, int d, int k_out,
@@ -106,7 +130,7 @@ nystrom_eval_kernel(const float* __restrict__ Y, int64_t n, const float* __restr
     float* xt = reinterpret_cast<float*>(ny_smem);            // 2 x kLm x p
     float* ys = xt + 2 * kLm * p;                             // kRows x p
     float2* wt = reinterpret_cast<float2*>(ys + kRows * p);   // 2 x kLm x kc
-    float* kv = reinterpret_cast<float*>(wt + 2 * kLm * kc);  // kRows x (kLm + 1)
+    float* kv = reinterpret_cast<float*>(wt + 2 * kLm * kc);  // kv_floats
     cg::cluster_group cluster = cg::this_cluster();
     const int group = (int)cluster.block_rank();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -132,6 +156,7 @@ nystrom_eval_kernel(const float* __restrict__ Y, int64_t n, const float* __restr
     };
     const int c = tid % kc, rg = tid / kc;
     float sum[Q], err[Q];
+    f32x2 sum2[2] = {0, 0}, err2[2] = {0, 0};   // Q = 4: pairs of states
 #pragma unroll
     for (int q = 0; q < Q; ++q) sum[q] = err[q] = 0.f;
 
@@ -181,22 +206,36 @@ nystrom_eval_kernel(const float* __restrict__ Y, int64_t n, const float* __restr
             }
         }
         if (warp < kLanesR) {
+            float v[Q];
 #pragma unroll
-            for (int q = 0; q < Q; ++q)
-                kv[(warp + kLanesR * q) * (kLm + 1) + lane] =
-                    (s * kLm + lane < r) ? kexp_scaled(dist[q], scale) : 0.f;
+            for (int q = 0; q < Q; ++q) v[q] = (s * kLm + lane < r) ? kexp_scaled(dist[q], scale) : 0.f;
+            if constexpr (Q == 4)
+                *reinterpret_cast<float4*>(kv + lane * kKvPitch + 4 * warp) = make_float4(v[0], v[1], v[2], v[3]);
+            else
+                kv[warp * (kLm + 1) + lane] = v[0];
         }
         __syncthreads();
         if (rg < kLanesR) {
             const float2* wc = wt + (s & 1) * kLm * kc + c;
-            const float* kr = kv + rg * (kLm + 1);
 #pragma unroll 4
             for (int j = 0; j < kLm; ++j) {
                 const float2 wv = wc[j * kc];
-#pragma unroll
-                for (int q = 0; q < Q; ++q) pair_fma(sum[q], err[q], kr[kLanesR * q * (kLm + 1) + j], wv);
+                if constexpr (Q == 4) {
+                    const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(kv + j * kKvPitch + 4 * rg);
+                    const f32x2 wx = pack2(wv.x, wv.x), nwx = pack2(-wv.x, -wv.x), wy = pack2(wv.y, wv.y);
+                    pair_fma2(sum2[0], err2[0], x.x, wx, nwx, wy);
+                    pair_fma2(sum2[1], err2[1], x.y, wx, nwx, wy);
+                } else {
+                    pair_fma(sum[0], err[0], kv[rg * (kLm + 1) + j], wv);
+                }
             }
         }
+    }
+    if constexpr (Q == 4) {
+        unpack2(sum2[0], sum[0], sum[1]);
+        unpack2(sum2[1], sum[2], sum[3]);
+        unpack2(err2[0], err[0], err[1]);
+        unpack2(err2[1], err[2], err[3]);
     }
     tc::cp_async_wait<0>();
     __syncthreads();
