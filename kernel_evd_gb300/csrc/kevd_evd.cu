@@ -327,7 +327,11 @@ __device__ __forceinline__ void df_fma(float& s, float& c, float x, float wh, fl
 // Partial column sums c[j] = sum_i w_i FT[j][i] (w == nullptr: ones) over this
 // CTA's row range.  CTA = 16 warps = 16 columns; the (hi, lo) weights of each
 // 2048-row chunk are staged once in shared memory for all 16 columns; each lane
-// sums 64 products as a double-FP32 pair, chunks are added in FP64.
+// sums 64 products as a double-FP32 pair, eight loads in flight, chunks are added
+// in FP64.  HBM: N = 2M, k = 2,000: two passes of this and two of evt_rowdot_kernel
+// 10.8 ms (9.4 at the copy rate); 11.9 with one load at a time here and eight there.
+// (The next chunk's weights read ahead and double-buffered: 13.2 ms, three CTAs per
+// SM instead of four.)
 __global__ void __launch_bounds__(512)
 evt_colsum_kernel(const float* __restrict__ FT, int64_t ldT, int64_t N, int64_t k, const double* __restrict__ w,
                   int64_t rows_per, double* __restrict__ partial) {
@@ -350,7 +354,15 @@ evt_colsum_kernel(const float* __restrict__ FT, int64_t ldT, int64_t N, int64_t 
         if (j < k) {
             const float* col = FT + j * ldT + i0;
             float ps = 0.f, pc = 0.f;
-            for (int t = lane; t < n; t += 32) df_fma(ps, pc, col[t], wsh[t], wsl[t]);
+            int t = lane;
+            for (; t + 7 * 32 < n; t += 8 * 32) {
+                float f[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u) f[u] = col[t + 32 * u];
+#pragma unroll
+                for (int u = 0; u < 8; ++u) df_fma(ps, pc, f[u], wsh[t + 32 * u], wsl[t + 32 * u]);
+            }
+            for (; t < n; t += 32) df_fma(ps, pc, col[t], wsh[t], wsl[t]);
             acc += (double)ps + (double)pc;
         }
     }
@@ -360,7 +372,9 @@ evt_colsum_kernel(const float* __restrict__ FT, int64_t ldT, int64_t N, int64_t 
 }
 
 // y_i = sum_j FT[j][i] v_j with v as an FP32 (hi, lo) pair; double-FP32 sums
-// of 32 terms, FP64 across them; yinv = 1/y; bad |= (y <= 0).
+// of 32 terms, FP64 across them; yinv = 1/y; bad |= (y <= 0).  Sixteen loads in
+// flight per thread; loading the next ones before the sums costs 64 registers and half
+// of the threads per SM (13.2 ms for the four passes).
 __global__ void __launch_bounds__(256)
 evt_rowdot_kernel(const float* __restrict__ FT, int64_t ldT, int64_t N, int64_t k, const double* __restrict__ v,
                   double* __restrict__ y, double* __restrict__ yinv, int* __restrict__ bad) {
@@ -378,7 +392,14 @@ evt_rowdot_kernel(const float* __restrict__ FT, int64_t ldT, int64_t N, int64_t 
         float ps = 0.f, pc = 0.f;
         const int64_t j1 = min(k, j0 + 32);
         int64_t j = j0;
-        for (; j + 8 <= j1; j += 8) {   // eight loads in flight, then the compensated sums in order
+        for (; j + 16 <= j1; j += 16) {   // sixteen loads in flight, then the compensated sums in order
+            float f[16];
+#pragma unroll
+            for (int u = 0; u < 16; ++u) f[u] = FT[(j + u) * ldT + i];
+#pragma unroll
+            for (int u = 0; u < 16; ++u) df_fma(ps, pc, f[u], vhl[2 * (j + u)], vhl[2 * (j + u) + 1]);
+        }
+        for (; j + 8 <= j1; j += 8) {
             float f[8];
 #pragma unroll
             for (int u = 0; u < 8; ++u) f[u] = FT[(j + u) * ldT + i];
