@@ -625,17 +625,12 @@ __device__ __forceinline__ bool group_view(int64_t r_old, int nacc_all, int grou
     nacc = min(kGroup, nacc_all - kGroup * group);
     return nacc > 0;
 }
-template <typename T>
-struct UpdSmem {
-    static constexpr int KC = 32;
-};
+constexpr int kUpdCols = 32;   // factor columns staged at a time
 
-template <typename T>
 __global__ void __launch_bounds__(256)
-rp_update_kernel(T* __restrict__ F, int64_t ldF, const float* __restrict__ X, int64_t N, int d,
-                 double scale, const int64_t* __restrict__ sacc, const double* __restrict__ minv,
-                 const float* __restrict__ minv_f, int b, const RoundState* st,
-                 double* __restrict__ dvec, double* __restrict__ dblk, int group) {
+rp_update_kernel(double* __restrict__ F, int64_t ldF, const float* __restrict__ X, int64_t N, int d,
+                 double scale, const int64_t* __restrict__ sacc, const double* __restrict__ minv, int b,
+                 const RoundState* st, double* __restrict__ dvec, double* __restrict__ dblk, int group) {
     if (st->done) return;
     int64_t r;
     int nacc;
@@ -644,22 +639,21 @@ rp_update_kernel(T* __restrict__ F, int64_t ldF, const float* __restrict__ X, in
         const int64_t o = (int64_t)kGroup * group;
         sacc += o;
         minv += o * b + o;
-        minv_f += o * b + o;
     }
-    constexpr int KC = UpdSmem<T>::KC;
+    constexpr int KC = kUpdCols;
     extern __shared__ __align__(16) unsigned char smraw[];
     // region 1 (phase A: X rows, kFeat features at a time; phase B: F tiles),
     // then Tm, then Minv
     constexpr int dp = kFeat + 1;
     const size_t reg1_a = (size_t)(kRowBlock + kGroup) * dp * sizeof(float);
-    const size_t reg1_b = (size_t)(kRowBlock + kGroup) * (KC + 1) * sizeof(T);
-    const size_t reg1 = (reg1_a > reg1_b ? reg1_a : reg1_b + 0);
+    const size_t reg1_b = (size_t)(kRowBlock + kGroup) * (KC + 1) * sizeof(double);
+    const size_t reg1 = reg1_a > reg1_b ? reg1_a : reg1_b;
     float* xr = reinterpret_cast<float*>(smraw);
     float* xs = xr + kRowBlock * dp;
-    T* At = reinterpret_cast<T*>(smraw);
-    T* Bt = At + kRowBlock * (KC + 1);
-    T* Tm = reinterpret_cast<T*>(smraw + ((reg1 + 15) / 16) * 16);   // 128 x (64+1)
-    T* Mv = Tm + kRowBlock * (kGroup + 1);                         // 64 x (64+1)
+    double* At = reinterpret_cast<double*>(smraw);
+    double* Bt = At + kRowBlock * (KC + 1);
+    double* Tm = reinterpret_cast<double*>(smraw + ((reg1 + 15) / 16) * 16);   // 128 x (64+1)
+    double* Mv = Tm + kRowBlock * (kGroup + 1);                         // 64 x (64+1)
     __shared__ double rowsq_s[kRowBlock];
 
     const int tid = threadIdx.x;
@@ -670,10 +664,10 @@ rp_update_kernel(T* __restrict__ F, int64_t ldF, const float* __restrict__ X, in
     // phase A: K(R, S_i) into Tm
     for (int e = tid; e < nacc * nacc; e += 256) {
         const int a = e / nacc, q = e - a * nacc;
-        Mv[a * (kGroup + 1) + q] = sizeof(T) == 8 ? (T)minv[a * b + q] : (T)minv_f[a * b + q];
+        Mv[a * (kGroup + 1) + q] = minv[a * b + q];
     }
     {
-        T acc[8][4];
+        double acc[8][4];
 #pragma unroll
         for (int i = 0; i < 8; ++i)
 #pragma unroll
@@ -691,16 +685,16 @@ rp_update_kernel(T* __restrict__ F, int64_t ldF, const float* __restrict__ X, in
             }
             __syncthreads();
             for (int k = 0; k < w; ++k) {
-                T vr[8], vs[4];
+                double vr[8], vs[4];
 #pragma unroll
-                for (int i = 0; i < 8; ++i) vr[i] = (T)xr[(ty + 16 * i) * dp + k];
+                for (int i = 0; i < 8; ++i) vr[i] = (double)xr[(ty + 16 * i) * dp + k];
 #pragma unroll
-                for (int j = 0; j < 4; ++j) vs[j] = (T)xs[min(tx + 16 * j, kGroup - 1) * dp + k];
+                for (int j = 0; j < 4; ++j) vs[j] = (double)xs[min(tx + 16 * j, kGroup - 1) * dp + k];
 #pragma unroll
                 for (int i = 0; i < 8; ++i)
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
-                        const T t = vr[i] - vs[j];
+                        const double t = vr[i] - vs[j];
                         acc[i][j] += t * t;
                     }
             }
@@ -710,18 +704,13 @@ rp_update_kernel(T* __restrict__ F, int64_t ldF, const float* __restrict__ X, in
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 const int c = tx + 16 * j;
-                T kv = 0;
-                if (c < nacc) {
-                    if (sizeof(T) == 8) kv = (T)exp(-scale * (double)acc[i][j]);
-                    else kv = (T)kexp_scaled((float)acc[i][j], split_scale(scale));
-                }
-                Tm[(ty + 16 * i) * (kGroup + 1) + c] = kv;
+                Tm[(ty + 16 * i) * (kGroup + 1) + c] = c < nacc ? exp(-scale * acc[i][j]) : 0.0;
             }
     }
     __syncthreads();
 
     // phase B: acc = F(R, 0:r) F(S_i, 0:r)^T
-    T acc[8][4];
+    double acc[8][4];
 #pragma unroll
     for (int i = 0; i < 8; ++i)
 #pragma unroll
@@ -730,16 +719,16 @@ rp_update_kernel(T* __restrict__ F, int64_t ldF, const float* __restrict__ X, in
         const int nc = (int)min((int64_t)KC, r - c0);
         for (int e = tid; e < kRowBlock * KC; e += 256) {
             const int rr = e / KC, c = e - rr * KC;
-            At[rr * (KC + 1) + c] = (rr < nrows && c < nc) ? F[(row0 + rr) * ldF + c0 + c] : (T)0;
+            At[rr * (KC + 1) + c] = (rr < nrows && c < nc) ? F[(row0 + rr) * ldF + c0 + c] : 0.0;
         }
         for (int e = tid; e < kGroup * KC; e += 256) {
             const int q = e / KC, c = e - q * KC;
-            Bt[q * (KC + 1) + c] = (q < nacc && c < nc) ? F[sacc[q] * ldF + c0 + c] : (T)0;
+            Bt[q * (KC + 1) + c] = (q < nacc && c < nc) ? F[sacc[q] * ldF + c0 + c] : 0.0;
         }
         __syncthreads();
 #pragma unroll 4
         for (int c = 0; c < KC; ++c) {
-            T va[8], vb[4];
+            double va[8], vb[4];
 #pragma unroll
             for (int i = 0; i < 8; ++i) va[i] = At[(ty + 16 * i) * (KC + 1) + c];
 #pragma unroll
@@ -758,19 +747,19 @@ rp_update_kernel(T* __restrict__ F, int64_t ldF, const float* __restrict__ X, in
         for (int j = 0; j < 4; ++j) Tm[(ty + 16 * i) * (kGroup + 1) + tx + 16 * j] -= acc[i][j];
     __syncthreads();
     // phase D: G = Tm Minv^T
-    T g[8][4];
+    double g[8][4];
 #pragma unroll
     for (int i = 0; i < 8; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j) g[i][j] = 0;
     for (int e = 0; e < nacc; ++e) {
-        T vt[8], vm[4];
+        double vt[8], vm[4];
 #pragma unroll
         for (int i = 0; i < 8; ++i) vt[i] = Tm[(ty + 16 * i) * (kGroup + 1) + e];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const int a = tx + 16 * j;
-            vm[j] = (a < nacc) ? Mv[a * (kGroup + 1) + e] : (T)0;
+            vm[j] = (a < nacc) ? Mv[a * (kGroup + 1) + e] : 0.0;
         }
 #pragma unroll
         for (int i = 0; i < 8; ++i)
@@ -787,7 +776,7 @@ rp_update_kernel(T* __restrict__ F, int64_t ldF, const float* __restrict__ X, in
             const int a = tx + 16 * j;
             if (a < nacc && rr < nrows) {
                 F[(row0 + rr) * ldF + r + a] = g[i][j];
-                sq += (double)g[i][j] * (double)g[i][j];
+                sq += g[i][j] * g[i][j];
             }
         }
 #pragma unroll
@@ -810,15 +799,13 @@ rp_update_kernel(T* __restrict__ F, int64_t ldF, const float* __restrict__ X, in
     if (tid == 0) dblk[blockIdx.x] = ((wsum[0] + wsum[1]) + (wsum[2] + wsum[3]));
 }
 
-template <typename T>
-static size_t update_smem(int d) {
-    (void)d;
+static size_t update_smem() {
     const int dp = kFeat + 1;
     const size_t reg1_a = (size_t)(kRowBlock + kGroup) * dp * sizeof(float);
-    const size_t reg1_b = (size_t)(kRowBlock + kGroup) * (UpdSmem<T>::KC + 1) * sizeof(T);
+    const size_t reg1_b = (size_t)(kRowBlock + kGroup) * (kUpdCols + 1) * sizeof(double);
     const size_t reg1 = ((std::max(reg1_a, reg1_b) + 15) / 16) * 16;
-    return reg1 + (size_t)kRowBlock * (kGroup + 1) * sizeof(T) +
-           (size_t)kGroup * (kGroup + 1) * sizeof(T);
+    return reg1 + (size_t)kRowBlock * (kGroup + 1) * sizeof(double) +
+           (size_t)kGroup * (kGroup + 1) * sizeof(double);
 }
 
 // One factorisation's buffers and launches.  setup() allocates (the sizes do not
@@ -882,9 +869,9 @@ struct RpRun {
             KEVD_CUDA(ctx, raise_smem_limit(reinterpret_cast<const void*>(factor()), std::max(fsm, (size_t)1024)));
         hsm = hgram_smem<T>(b);
         KEVD_CUDA(ctx, raise_smem_limit(reinterpret_cast<const void*>(&rp_hgram_kernel<T>), (int)hsm));
-        usm = update_smem<T>(d);
+        usm = update_smem();
         if constexpr (sizeof(T) == 8)
-            KEVD_CUDA(ctx, raise_smem_limit(reinterpret_cast<const void*>(&rp_update_kernel<T>), (int)usm));
+            KEVD_CUDA(ctx, raise_smem_limit(reinterpret_cast<const void*>(&rp_update_kernel), (int)usm));
         // FP32 factors take the tensor-core residual update when the layout allows
         // TMA and the kernel is not nearly diagonal (kernel_density_kernel)
         use_tc = sizeof(T) == 4 && tc_allowed && update_tc_supported(reinterpret_cast<const float*>(F), ldF, d);
@@ -942,8 +929,7 @@ struct RpRun {
             KEVD_TRY(launch_update_f32(ctx, (float*)F, ldF, X, N, d, scale, sacc, minv_f, b, rs, dvec, dblk, s));
         } else {
             for (int g = 0; g < (b + kGroup - 1) / kGroup; ++g) {
-                rp_update_kernel<T><<<(int)nblk, 256, usm, s>>>(F, ldF, X, N, d, scale, sacc, minv, minv_f, b, rs, dvec,
-                                                               dblk, g);
+                rp_update_kernel<<<(int)nblk, 256, usm, s>>>(F, ldF, X, N, d, scale, sacc, minv, b, rs, dvec, dblk, g);
                 KEVD_LAUNCH(ctx);
             }
         }
