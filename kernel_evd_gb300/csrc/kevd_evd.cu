@@ -430,11 +430,12 @@ __global__ void evt_zf_kernel(const double* __restrict__ Z, int64_t k, int m, in
 // per entry of U in increasing j.
 // CTA = 128 threads on 256 rows; thread t forms columns 16 h .. 16 h + 15 (h = t & 1)
 // of the four rows 4 (t >> 1) .. +3 as packed pairs of columns: a 16-byte read of F
-// (the next four columns' are in flight) and four of Z for 32 packed FMA.
-// N = 2M, k = 2,000: 6.0 ms (8.9 with scalar FMAs, 32 columns by 256 threads; FP32
-// pipe 3.5).
+// (the next eight columns' are in flight) and four of Z for 32 packed FMA.
+// N = 2M, k = 2,000: 5.7 ms (8.9 with scalar FMAs, 32 columns by 256 threads; FP32
+// pipe 3.5); four columns ahead and four CTAs per SM 6.0.
 constexpr int kUChunk = 64;
-__global__ void __launch_bounds__(128, 4)
+constexpr int kUAhead = 8;
+__global__ void __launch_bounds__(128, 3)
 evt_u_kernel(const float* __restrict__ FT, int64_t ldT, int64_t N, int64_t k, const float* __restrict__ Zf, int m,
              const double* __restrict__ dinv, float* __restrict__ U, float* __restrict__ Y) {
     __shared__ __align__(16) float Zs[2][kUChunk][32];
@@ -454,31 +455,26 @@ evt_u_kernel(const float* __restrict__ FT, int64_t ldT, int64_t N, int64_t k, co
     for (int r = 0; r < 4; ++r)
 #pragma unroll
         for (int q = 0; q < 8; ++q) acc[r][q] = 0;
-    float4 g[4];
+    float4 g[kUAhead];
     auto fetch = [&](int u, int64_t j) {
         g[u] = (valid && j < k) ? *reinterpret_cast<const float4*>(col + j * ldT) : make_float4(0.f, 0.f, 0.f, 0.f);
     };
     stage(0);
 #pragma unroll
-    for (int u = 0; u < 4; ++u) fetch(u, u);
+    for (int u = 0; u < kUAhead; ++u) fetch(u, u);
     for (int64_t c = 0; c < n_ch; ++c) {
         tc::cp_async_wait<0>();
         __syncthreads();   // chunk c is staged, and chunk c - 1 no longer read
         if (c + 1 < n_ch) stage(c + 1);
         const float (*Zc)[32] = Zs[c & 1];
 #pragma unroll 1
-        for (int jj = 0; jj < kUChunk; jj += 4) {
-            float4 f[4];
+        for (int jj = 0; jj < kUChunk; jj += kUAhead) {
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                f[u] = g[u];
-                fetch(u, c * kUChunk + jj + 4 + u);
-            }
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
+            for (int u = 0; u < kUAhead; ++u) {
                 const ulonglong2* zr = reinterpret_cast<const ulonglong2*>(Zc[jj + u] + 16 * h);
-                const f32x2 fr[4] = {pack2(f[u].x, f[u].x), pack2(f[u].y, f[u].y), pack2(f[u].z, f[u].z),
-                                     pack2(f[u].w, f[u].w)};
+                const float4 f = g[u];
+                const f32x2 fr[4] = {pack2(f.x, f.x), pack2(f.y, f.y), pack2(f.z, f.z), pack2(f.w, f.w)};
+                fetch(u, c * kUChunk + jj + kUAhead + u);
 #pragma unroll
                 for (int q4 = 0; q4 < 4; ++q4) {
                     const ulonglong2 z = zr[q4];
