@@ -578,7 +578,7 @@ evt_t1_kernel(const float* __restrict__ FT, int64_t ldT, int64_t N, int64_t k, c
         __syncthreads();
         const float* Fs = t1sm + (t & 1) * kT1Buf + 4 * jg * kT1Rows;
         const float* Ws = t1sm + (t & 1) * kT1Buf + kT1Cols * kT1Rows + 8 * qg;
-#pragma unroll 1
+#pragma unroll 4
         for (int i8 = 0; i8 < kT1Rows; i8 += 8) {
             f32x2 p[4][4];
 #pragma unroll
@@ -640,7 +640,8 @@ evt_t1_kernel(const float* __restrict__ FT, int64_t ldT, int64_t N, int64_t k, c
 // entries (8 (t >> 5) + r, t & 31), r < 8, of the 32 x 32 matrices, summed over 64
 // rows with compensation and beyond in FP64.
 // FP32 pipe: 32 (2 + 4 / 8) operations per element of F.  N = 2M, k = 2,000: with
-// T1 and the rotation 21.6 ms (26.6 with scalar FMAs and 4 x 4 tiles; FP32 pipe 14.4).
+// T1 and the rotation 20.4 ms (26.6 with scalar FMAs and 4 x 4 tiles; 21.6 with the
+// eight-term steps of both kernels not unrolled; FP32 pipe 14.4).
 constexpr int kHmRows = 128;
 constexpr int kHmFChunk = 32 * kHmRows;                 // floats of an F chunk, [column j][row i]
 constexpr int kHmBuf = kHmFChunk + 2 * 32 * 32;         // and the T1 hi and lo chunks
@@ -732,7 +733,7 @@ evt_hm_kernel(const float* __restrict__ FT, int64_t ldT, int64_t N, int64_t k, c
             __syncthreads();
             const float* Fs = hmsm + b * kHmBuf + 4 * ig;
             const float* Ts = hmsm + b * kHmBuf + kHmFChunk + 8 * qg;
-#pragma unroll 1
+#pragma unroll 4
             for (int j8 = 0; j8 < 32; j8 += 8) {
                 f32x2 p[4][4];
 #pragma unroll
