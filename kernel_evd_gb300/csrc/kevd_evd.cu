@@ -431,8 +431,8 @@ __global__ void evt_zf_kernel(const double* __restrict__ Z, int64_t k, int m, in
 // CTA = 128 threads on 256 rows; thread t forms columns 16 h .. 16 h + 15 (h = t & 1)
 // of the four rows 4 (t >> 1) .. +3 as packed pairs of columns: a 16-byte read of F
 // (the next eight columns' are in flight) and four of Z for 32 packed FMA.
-// N = 2M, k = 2,000: 5.7 ms (8.9 with scalar FMAs, 32 columns by 256 threads; FP32
-// pipe 3.5); four columns ahead and four CTAs per SM 6.0.
+// N = 2M, k = 2,000: 5.3 ms (8.9 with scalar FMAs, 32 columns by 256 threads; FP32
+// pipe 3.5); four columns ahead and four CTAs per SM 6.0, steps not unrolled 5.7.
 constexpr int kUChunk = 64;
 constexpr int kUAhead = 8;
 __global__ void __launch_bounds__(128, 3)
@@ -467,7 +467,7 @@ evt_u_kernel(const float* __restrict__ FT, int64_t ldT, int64_t N, int64_t k, co
         __syncthreads();   // chunk c is staged, and chunk c - 1 no longer read
         if (c + 1 < n_ch) stage(c + 1);
         const float (*Zc)[32] = Zs[c & 1];
-#pragma unroll 1
+#pragma unroll 2
         for (int jj = 0; jj < kUChunk; jj += kUAhead) {
 #pragma unroll
             for (int u = 0; u < kUAhead; ++u) {
