@@ -13,7 +13,8 @@
 // pipe and as much for the ex2 unit.  The exponentials run at the ex2 unit's
 // rate and the distances at 0.7 of the FMA pipe's; what is left is that they
 // overlap little (3.0 clocks per pair).  Independent groups that share barriers
-// with nobody overlap best: N = 200,000, d = 64, 64 scales takes 189 ms; as four
+// with nobody overlap best: N = 200,000, d = 64, 64 scales takes 187 ms (190
+// with two features of the distance loop unrolled, four are built); as four
 // CTAs per SM 212 ms, with groups made to alternate between distances and
 // exponentials 200 ms, with the next tile's distances woven into the exponentials
 // (two tiles of registers, three groups) 214 to 231 ms, and as two CTAs of 256
@@ -165,7 +166,7 @@ __device__ __forceinline__ void pt_dist(const float* __restrict__ X, int64_t N, 
         const int w4 = (min(kPtChunk, d - c0) + 3) & ~3;
         const float* xi = sm + 8 * (pt_tid() >> 4);
         const float* xj = sm + kPtChunk * kPtHalf + 8 * (pt_tid() & 15);
-#pragma unroll 2
+#pragma unroll 4
         for (int k = 0; k < w4; ++k) {
             const float4 i0 = *reinterpret_cast<const float4*>(xi + k * kPtHalf);
             const float4 i1 = *reinterpret_cast<const float4*>(xi + k * kPtHalf + 4);
