@@ -380,7 +380,9 @@ int run_calibrate_noalloc(const float* X, int64_t N, int d, const double* scales
 // a radix selection: three passes histogram bits [31:20], [19:8], [7:0] of the
 // distances whose higher bits match the prefix found so far, and the host walks
 // each histogram to the bin holding the wanted rank.  Every pass recomputes the
-// distances.
+// distances.  Counts are 64-bit: from N = 92,683 on there are more than 2^32 pairs,
+// and one bin may hold most of them.  A CTA counts in 32 bits and adds its counts to
+// the 64-bit ones at its end, so a launch gives it at most kHistUnits half tiles.
 //
 // Over all pairs the distances are nearly the whole cost, so one pass has to do
 // (run_bracketed_median): the distances of random pairs give a bracket that holds
@@ -390,6 +392,8 @@ int run_calibrate_noalloc(const float* X, int64_t N, int d, const double* scales
 // N = 20,000, d = 64: 1.25 ms, in three passes 3.08 ms.
 
 constexpr int kHistBins = 4096;
+using HistCount = unsigned long long;
+constexpr int64_t kHistUnits = 1 << 18;   // half tiles of 8,192 pairs per CTA and launch: 2^31 counts
 
 __device__ __forceinline__ void hist_add(unsigned* h, float D, int shift, unsigned mask,
                                          unsigned prefix, int hi_shift) {
@@ -399,15 +403,15 @@ __device__ __forceinline__ void hist_add(unsigned* h, float D, int shift, unsign
 }
 
 __global__ void __launch_bounds__(kPtThreads, 1)
-median_tiles_kernel(const float* __restrict__ X, int64_t N, int d, int64_t n_tiles, int shift,
-                    unsigned mask, unsigned prefix, int hi_shift, unsigned* __restrict__ hist) {
+median_tiles_kernel(const float* __restrict__ X, int64_t N, int d, int64_t unit0, int64_t n_units, int shift,
+                    unsigned mask, unsigned prefix, int hi_shift, HistCount* __restrict__ hist) {
     extern __shared__ __align__(16) float smem[];
     float* sm = smem + pt_group() * kPtSmemFloats;
     unsigned* h = reinterpret_cast<unsigned*>(smem + kPtGroups * kPtSmemFloats);
     for (int e = threadIdx.x; e < kHistBins; e += blockDim.x) h[e] = 0u;
     __syncthreads();
     const int64_t part = (int64_t)blockIdx.x * kPtGroups + pt_group(), parts = (int64_t)gridDim.x * kPtGroups;
-    const int64_t u0 = 2 * n_tiles * part / parts, u1 = 2 * n_tiles * (part + 1) / parts;
+    const int64_t u0 = unit0 + n_units * part / parts, u1 = unit0 + n_units * (part + 1) / parts;
     PtUnit unit = pt_unit(u0);
     int64_t staged = -1;
     for (int64_t u = u0; u < u1; ++u, pt_next(unit)) {
@@ -428,13 +432,13 @@ median_tiles_kernel(const float* __restrict__ X, int64_t N, int d, int64_t n_til
     }
     __syncthreads();
     for (int e = threadIdx.x; e < kHistBins; e += blockDim.x)
-        if (h[e]) atomicAdd(&hist[e], h[e]);
+        if (h[e]) atomicAdd(&hist[e], (HistCount)h[e]);
 }
 
 __global__ void median_pairs_kernel(const float* __restrict__ X, int d,
                                     const int64_t* __restrict__ pi, const int64_t* __restrict__ pl,
                                     int64_t n_pairs, int shift, unsigned mask, unsigned prefix,
-                                    int hi_shift, unsigned* __restrict__ hist) {
+                                    int hi_shift, HistCount* __restrict__ hist) {
     __shared__ unsigned h[kHistBins];
     for (int e = threadIdx.x; e < kHistBins; e += blockDim.x) h[e] = 0u;
     __syncthreads();
@@ -451,7 +455,7 @@ __global__ void median_pairs_kernel(const float* __restrict__ X, int d,
     }
     __syncthreads();
     for (int e = threadIdx.x; e < kHistBins; e += blockDim.x)
-        if (h[e]) atomicAdd(&hist[e], h[e]);
+        if (h[e]) atomicAdd(&hist[e], (HistCount)h[e]);
 }
 
 // Distances of n pseudo-random pairs (i, j), i != j.
@@ -572,7 +576,7 @@ median_collect_kernel(const float* __restrict__ X, int64_t N, int d, int64_t n_t
 // Histogram of (bits - lo) >> shift over the n collected distances with bits in
 // [lo, lo + 2^(shift + 12)).
 __global__ void __launch_bounds__(256) median_buffer_kernel(const float* __restrict__ buf, unsigned long long n,
-                                                            unsigned lo, int shift, unsigned* __restrict__ hist) {
+                                                            unsigned lo, int shift, HistCount* __restrict__ hist) {
     __shared__ unsigned h[kHistBins];
     for (int e = threadIdx.x; e < kHistBins; e += 256) h[e] = 0u;
     __syncthreads();
@@ -583,12 +587,12 @@ __global__ void __launch_bounds__(256) median_buffer_kernel(const float* __restr
     }
     __syncthreads();
     for (int e = threadIdx.x; e < kHistBins; e += 256)
-        if (h[e]) atomicAdd(&hist[e], h[e]);
+        if (h[e]) atomicAdd(&hist[e], (HistCount)h[e]);
 }
 
 // The median over all pairs in one pass; *found = false (the caller goes on with
 // the radix selection) when there is no room for the bracket or it misses.
-static int run_bracketed_median(kevd_ctx* ctx, const float* X, int64_t N, int d, uint64_t rank, unsigned* hist,
+static int run_bracketed_median(kevd_ctx* ctx, const float* X, int64_t N, int d, uint64_t rank, HistCount* hist,
                                 unsigned* bits, bool* found, cudaStream_t s) {
     *found = false;
     const int64_t nt = (N + kCalTile - 1) / kCalTile;
@@ -623,15 +627,15 @@ static int run_bracketed_median(kevd_ctx* ctx, const float* X, int64_t N, int d,
     if (rank < hc[0] || rank - hc[0] >= hc[1] || hc[1] > cap) return KEVD_OK;
     uint64_t left = rank - hc[0];
     unsigned lo = hbr[0];
-    std::vector<unsigned> hh(kHistBins);
+    std::vector<HistCount> hh(kHistBins);
     int shift = 0;
     while (((uint64_t)(hbr[1] - hbr[0]) + 1) >> shift > (uint64_t)kHistBins) ++shift;
     for (;;) {
-        KEVD_CUDA(ctx, cudaMemsetAsync(hist, 0, kHistBins * sizeof(unsigned), s));
+        KEVD_CUDA(ctx, cudaMemsetAsync(hist, 0, kHistBins * sizeof(HistCount), s));
         median_buffer_kernel<<<(unsigned)std::min<unsigned long long>((hc[1] + 1023) / 1024, 2ull * ctx->num_sms), 256, 0,
                                s>>>(buf, hc[1], lo, shift, hist);
         KEVD_LAUNCH(ctx);
-        KEVD_CUDA(ctx, cudaMemcpyAsync(hh.data(), hist, kHistBins * sizeof(unsigned), cudaMemcpyDeviceToHost, s));
+        KEVD_CUDA(ctx, cudaMemcpyAsync(hh.data(), hist, kHistBins * sizeof(HistCount), cudaMemcpyDeviceToHost, s));
         KEVD_CUDA(ctx, cudaStreamSynchronize(s));
         unsigned bin = 0;
         while (bin < (unsigned)kHistBins && left >= hh[bin]) left -= hh[bin++];
@@ -661,7 +665,7 @@ int run_pair_median(kevd_ctx* ctx, const float* X, int64_t N, int d, const int64
     const uint64_t total = exact ? (uint64_t)N * (uint64_t)(N - 1) / 2 : (uint64_t)n_pairs;
     uint64_t rank = (total - 1) / 2;  // lower median
     int st = KEVD_OK;
-    unsigned* hist = arena_get<unsigned>(ctx, "med.hist", kHistBins, &st);
+    HistCount* hist = arena_get<HistCount>(ctx, "med.hist", kHistBins, &st);
     if (st != KEVD_OK) return st;
     if (exact && (double)total * d >= kBracketWork && N <= 160000) {
         bool found = false;
@@ -680,20 +684,23 @@ int run_pair_median(kevd_ctx* ctx, const float* X, int64_t N, int d, const int64
     const unsigned masks[3] = {0xfffu, 0xfffu, 0xffu};
     unsigned prefix = 0;
     int hi_shift = 32;
-    std::vector<unsigned> hh(kHistBins);
+    std::vector<HistCount> hh(kHistBins);
     for (int pass = 0; pass < 3; ++pass) {
-        KEVD_CUDA(ctx, cudaMemsetAsync(hist, 0, kHistBins * sizeof(unsigned), s));
+        KEVD_CUDA(ctx, cudaMemsetAsync(hist, 0, kHistBins * sizeof(HistCount), s));
         if (exact) {
-            const int grid = (int)std::min<int64_t>(2 * n_tiles, ctx->num_sms);
-            median_tiles_kernel<<<grid, kPtThreads, smem, s>>>(X, N, d, n_tiles, shifts[pass],
-                                                        masks[pass], prefix, hi_shift, hist);
+            for (int64_t u = 0; u < 2 * n_tiles; u += ctx->num_sms * kHistUnits) {
+                const int64_t nu = std::min(2 * n_tiles - u, ctx->num_sms * kHistUnits);
+                median_tiles_kernel<<<(int)std::min<int64_t>(nu, ctx->num_sms), kPtThreads, smem, s>>>(
+                    X, N, d, u, nu, shifts[pass], masks[pass], prefix, hi_shift, hist);
+                KEVD_LAUNCH(ctx);
+            }
         } else {
             const int grid = (int)std::min<int64_t>((n_pairs + 255) / 256, (int64_t)ctx->num_sms * 4);
             median_pairs_kernel<<<grid, 256, 0, s>>>(X, d, pi, pl, n_pairs, shifts[pass],
                                                      masks[pass], prefix, hi_shift, hist);
+            KEVD_LAUNCH(ctx);
         }
-        KEVD_LAUNCH(ctx);
-        KEVD_CUDA(ctx, cudaMemcpyAsync(hh.data(), hist, kHistBins * sizeof(unsigned),
+        KEVD_CUDA(ctx, cudaMemcpyAsync(hh.data(), hist, kHistBins * sizeof(HistCount),
                                        cudaMemcpyDeviceToHost, s));
         KEVD_CUDA(ctx, cudaStreamSynchronize(s));
         uint64_t cum = 0;
