@@ -267,7 +267,12 @@ nystrom_eval_kernel(const float* __restrict__ Y, int64_t n, const float* __restr
     cluster.sync();   // no CTA leaves while its sums are read
 }
 
-// W column blockIdx.x: its binade and the FP32 pairs.
+// W column blockIdx.x: its binade and the FP32 pairs, scaled to 2^kWExp: K is as
+// small as 2^-126 for a state far from every landmark, and with |W| < 1 the low parts
+// of its products (2^-24 and 2^-48 of K W), then K W itself where the near landmarks
+// have small entries, left the FP32 range.  A sum over r < 2^20 landmarks stays below
+// 2^120, and the factor cancels in the quotient.
+constexpr int kWExp = 100;
 __global__ void __launch_bounds__(256) nystrom_pack_kernel(const double* __restrict__ zp, int64_t r, int kc,
                                                            float2* __restrict__ w, int* __restrict__ ex) {
     __shared__ double red[256];
@@ -281,8 +286,9 @@ __global__ void __launch_bounds__(256) nystrom_pack_kernel(const double* __restr
         if ((int)threadIdx.x < o) red[threadIdx.x] = fmax(red[threadIdx.x], red[threadIdx.x + o]);
         __syncthreads();
     }
-    int e = 0;
+    int e = kWExp;
     if (red[0] > 0.0 && isfinite(red[0])) frexp(red[0], &e);
+    e -= kWExp;
     for (int64_t j = threadIdx.x; j < r; j += 256) {
         const double v = ldexp(col[j], -e);
         const float h = (float)v;

@@ -11,7 +11,7 @@ namespace kevd {
 
 // Landmark rows, and W = [Z' | p1'] = L^{-T} [Z | c1] (r x (k_out + 1)) as the
 // query kernel reads it: row-major, each entry an FP32 pair hi + lo (48 bits)
-// of W 2^-ex[c], with 2^ex[c] the binade of the column's largest entry.
+// of W 2^-ex[c], with 2^(ex[c] + 100) the binade of the column's largest entry.
 struct Model {
     int64_t r = 0;
     int d = 0;
