@@ -388,8 +388,9 @@ int run_calibrate_noalloc(const float* X, int64_t N, int d, const double* scales
 // (run_bracketed_median): the distances of random pairs give a bracket that holds
 // the median and 1 to 2 % of all pairs; the pass counts the distances below it and
 // collects those inside, and the exact rank is selected among these.  A bracket
-// that misses (by the exact counts) leaves the call to the radix selection.
-// N = 20,000, d = 64: 1.25 ms, in three passes 3.08 ms.
+// that misses (by the exact counts) leaves the call to the radix selection, and so
+// does one that by the sample holds more pairs than fit the buffer (many ties),
+// before the pass.  N = 20,000, d = 64: 1.25 ms, in three passes 3.08 ms.
 
 constexpr int kHistBins = 4096;
 using HistCount = unsigned long long;
@@ -479,13 +480,16 @@ __global__ void __launch_bounds__(256) median_sample_kernel(const float* __restr
 }
 
 // br[0], br[1]: the bits of the sample's order statistics r0 and r1 rounded down
-// and up to multiples of 2^10 (two levels of 11 bits).  One CTA.
+// and up to multiples of 2^10 (two levels of 11 bits); br[2]: how many of the sample
+// lie in [br[0], br[1]).  One CTA.
 __global__ void __launch_bounds__(1024) median_bracket_kernel(const unsigned* __restrict__ bits, int n, int r0, int r1,
                                                               unsigned* __restrict__ br) {
     __shared__ unsigned h[2][2048];
     __shared__ unsigned pre[2];
     __shared__ int rank[2];
+    __shared__ unsigned b01[2], inside;
     if (threadIdx.x < 2) rank[threadIdx.x] = threadIdx.x ? r1 : r0;
+    if (threadIdx.x == 0) inside = 0u;
     for (int level = 0; level < 2; ++level) {
         for (int e = threadIdx.x; e < 2 * 2048; e += 1024) h[e >> 11][e & 2047] = 0u;
         __syncthreads();
@@ -507,17 +511,25 @@ __global__ void __launch_bounds__(1024) median_bracket_kernel(const unsigned* __
             while (bin < 2047 && r >= (int)hq[bin]) r -= (int)hq[bin++];
             rank[q] = r;
             if (level == 0) pre[q] = (unsigned)bin;
-            else br[q] = (((pre[q] << 11) | (unsigned)bin) + (unsigned)q) << 10;
+            else br[q] = b01[q] = (((pre[q] << 11) | (unsigned)bin) + (unsigned)q) << 10;
         }
         __syncthreads();
     }
+    unsigned in = 0u;
+    for (int t = threadIdx.x; t < n; t += 1024) in += bits[t] >= b01[0] && bits[t] < b01[1];
+    atomicAdd(&inside, in);
+    __syncthreads();
+    if (threadIdx.x == 0) br[2] = inside;
 }
 
 // One pass over all pairs: cnt[0] += distances below br[0], and those in
 // [br[0], br[1]) appended to buf (in any order; cnt[1] counts them, also past cap).
+// Nothing at all where more than max_inside of the sample lie in the bracket.
 __global__ void __launch_bounds__(kPtThreads, 1)
 median_collect_kernel(const float* __restrict__ X, int64_t N, int d, int64_t n_tiles, const unsigned* __restrict__ br,
-                      float* __restrict__ buf, unsigned long long cap, unsigned long long* __restrict__ cnt) {
+                      unsigned max_inside, float* __restrict__ buf, unsigned long long cap,
+                      unsigned long long* __restrict__ cnt) {
+    if (br[2] > max_inside) return;
     extern __shared__ __align__(16) float smem[];
     float* sm = smem + pt_group() * kPtSmemFloats;
     const int lane = threadIdx.x & 31;
@@ -605,7 +617,7 @@ static int run_bracketed_median(kevd_ctx* ctx, const float* X, int64_t N, int d,
     const unsigned long long cap = (unsigned long long)std::min<uint64_t>((uint64_t)(0.06 * (double)total), 1ull << 26);
     int st = KEVD_OK;
     float* buf = arena_get<float>(ctx, "med.buf", cap, &st);
-    unsigned* smp = arena_get<unsigned>(ctx, "med.smp", (size_t)n + 2, &st);
+    unsigned* smp = arena_get<unsigned>(ctx, "med.smp", (size_t)n + 3, &st);
     unsigned long long* cnt = arena_get<unsigned long long>(ctx, "med.cnt", 2, &st);
     if (st != KEVD_OK) return KEVD_OK;
     unsigned* br = smp + n;
@@ -617,7 +629,8 @@ static int run_bracketed_median(kevd_ctx* ctx, const float* X, int64_t N, int d,
     const size_t smem = (size_t)kPtGroups * kPtSmemFloats * sizeof(float);
     KEVD_CUDA(ctx, raise_smem_limit(reinterpret_cast<const void*>(&median_collect_kernel), (int)smem));
     const int grid = (int)std::min<int64_t>(2 * n_tiles, ctx->num_sms);
-    median_collect_kernel<<<grid, kPtThreads, smem, s>>>(X, N, d, n_tiles, br, buf, cap, cnt);
+    median_collect_kernel<<<grid, kPtThreads, smem, s>>>(X, N, d, n_tiles, br,
+                                                         (unsigned)((double)n * (double)cap / (double)total), buf, cap, cnt);
     KEVD_LAUNCH(ctx);
     unsigned hbr[2];
     unsigned long long hc[2];
@@ -649,10 +662,14 @@ static int run_bracketed_median(kevd_ctx* ctx, const float* X, int64_t N, int d,
     return KEVD_OK;
 }
 
-// Work (pairs x features) from which one pass with a bracket beats three; the
-// sample and its selection take about 90 us.  d = 64, three passes / bracket:
-// N = 2,900 178 / 231 us, 4,000 246 / 250, 6,000 453 / 310.
-constexpr double kBracketWork = 5e8;
+// Whether one pass with a bracket beats three.  A pass takes about 16 features' time a
+// pair beside its d; the sample and its selection 100 us and 0.1 us a feature.  Times,
+// three passes / bracket: N = 8,000, d = 3 176 / 201 us; 6,000, 16 189 / 199 and 8,000, 16
+// 267 / 227; 5,000, 64 324 / 272; 3,000, 128 264 / 282 and 4,000, 128 396 / 317; 2,000,
+// 1,024 832 / 850 and 3,000, 1,024 1,457 / 1,076.
+static bool bracket_pays(int64_t N, int d) {
+    return 0.5 * (double)N * (double)(N - 1) * (d + 16) >= 8e8 + 1.4e6 * d;
+}
 
 int run_pair_median(kevd_ctx* ctx, const float* X, int64_t N, int d, const int64_t* pi,
                     const int64_t* pl, int64_t n_pairs, double* median, cudaStream_t s) {
@@ -667,7 +684,7 @@ int run_pair_median(kevd_ctx* ctx, const float* X, int64_t N, int d, const int64
     int st = KEVD_OK;
     HistCount* hist = arena_get<HistCount>(ctx, "med.hist", kHistBins, &st);
     if (st != KEVD_OK) return st;
-    if (exact && (double)total * d >= kBracketWork && N <= 160000) {
+    if (exact && bracket_pays(N, d) && N <= 160000) {
         bool found = false;
         unsigned bits = 0;
         KEVD_TRY(run_bracketed_median(ctx, X, N, d, rank, hist, &bits, &found, s));
