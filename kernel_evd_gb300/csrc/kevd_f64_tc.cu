@@ -13,7 +13,8 @@
 //   x y = 2^(ex + ey) sum_{i,j} a_i b_j 2^(-8 (i + j) - 12)
 //
 // of which the 36 digit pairs with i + j <= 7 are computed, one accumulator per
-// i + j (what is left out is of the size of the last digit's rounding).  Every
+// i + j (what is left out is of the size of the last digit's rounding where the
+// entries are of one size; see tail pairs below).  Every
 // 192 terms the eight integer sums S_d leave Tensor Memory and are added, still
 // exactly, to two 64-bit integers per output,
 //
@@ -21,9 +22,19 @@
 //
 // so the long sum has no rounding at all; the result is rounded once to FP64.
 // The error of an output is thus the fixed-point rounding of its inputs,
-// 2^-63 of the row's (column's) largest entry each, against one FP64 rounding
-// per product and per sum: an entry keeps its 53 bits down to 2^-10 of the
-// largest.
+// 2^-63 of the row's (column's) largest entry each, and the pairs left out, against
+// one FP64 rounding per product and per sum: an entry keeps its 53 bits down to 2^-10
+// of the largest.
+//
+// Tail pairs (F from /linv).  There the entries of a row differ by orders of magnitude,
+// an output's products may all be small against the rows' largest entries, and the 7
+// pairs with i + j = 8 are 20 times the inputs' rounding.  They are added to the
+// accumulator of i + j = 7.  For that the digits carry their weight, a_i 2^(-8 i), which
+// f16 cannot hold and bf16 can (8 significant bits hold a digit): 14 more MMAs of 64
+// columns a stage, and two more operations per pair of digits.  N = 20,000, r = 1,000,
+// d = 64, errors of the entries of F relative to sum |K| |Linv|: rms 4.2e-16 without
+// the pairs, 6.2e-17 with them (2.4e-16 on the FP64 pipe); N = 100,000, r = 1,024, the
+// call 12.5 and 13.5 ms.
 //
 // CTA (512 threads): output tile 128 x 64, 32 terms per stage, two stages of
 // shared memory (8 digit planes of A, 128 x 32 f16, and of B, 64 x 32 f16,
@@ -45,6 +56,7 @@
 #include "kevd_f64_tc.cuh"
 #include "kevd_tc.cuh"
 
+#include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
 #include <algorithm>
@@ -107,7 +119,19 @@ __device__ __forceinline__ int digits_exp(uint64_t abs_bits) {
     return ex - 1023 + ((abs_bits & 0xfffffffffffffull) ? 1 : 0);
 }
 
-// Eight packed entries along K -> the 16-byte piece of each plane.
+// Two digits + 128, in bytes 0 and 2 of x, as two bf16 digits times 2^(-8 plane): u is
+// 128 + (u & 127) minus 256 or, with bit 7, 128, which bf16 holds.
+__device__ __forceinline__ uint32_t digits_bf16x2(uint32_t x, int plane) {
+    const uint32_t w = (uint32_t)plane << 10;   // 8 plane in the exponent field
+    const uint32_t hi = (x & 0x007f007fu) | ((0x4300u - w) * 0x10001u);
+    const uint32_t lo = (x & 0x00800080u) ^ ((0x4380u - w) * 0x10001u);
+    const __nv_bfloat162 d = __hsub2(*reinterpret_cast<const __nv_bfloat162*>(&hi), *reinterpret_cast<const __nv_bfloat162*>(&lo));
+    return *reinterpret_cast<const uint32_t*>(&d);
+}
+
+// Eight packed entries along K -> the 16-byte piece of each plane: f16 digits, or
+// (kTail) bf16 digits times 2^(-8 plane).
+template <bool kTail>
 __device__ __forceinline__ void store_planes(const uint64_t (&w)[8], uint8_t* planes, int plane_bytes, uint32_t off) {
     const __half2 bias = __half2half2(__ushort_as_half((unsigned short)0xE480));   // -1152
 #pragma unroll
@@ -120,6 +144,10 @@ __device__ __forceinline__ void store_planes(const uint64_t (&w)[8], uint8_t* pl
             const uint32_t g[2] = {__byte_perm(x0, x1, 0x6273), __byte_perm(x0, x1, 0x4051)};
 #pragma unroll
             for (int s = 0; s < 4; ++s) {
+                if constexpr (kTail) {
+                    h[s][p] = digits_bf16x2(__byte_perm(g[s >> 1], 0u, (s & 1) ? 0x4342 : 0x4140), 4 * word + s);
+                    continue;
+                }
                 // 0x64uu is the f16 1024 + u; minus 1152 leaves the digit u - 128
                 const uint32_t v = __byte_perm(g[s >> 1], 0x64646464u, (s & 1) ? 0x4342 : 0x4140);
                 const __half2 d = __hadd2(*reinterpret_cast<const __half2*>(&v), bias);
@@ -185,8 +213,8 @@ __device__ __forceinline__ void load_words(const Operand& o, int m, int64_t k0, 
 
 // One 128 x 64 tile: sums over k in [k0, k1) into (hi, lo) of the thread's 16
 // outputs, row 32 (warp % 4) + lane, columns 16 (warp / 4) ...  Called by the
-// whole CTA.
-template <bool kGram, int kBlockStages = ::kevd::kBlockStages>
+// whole CTA.  kTail: with the digit pairs i + j = 8.
+template <bool kGram, int kBlockStages = ::kevd::kBlockStages, bool kTail = false>
 __device__ __forceinline__ void tile_sums(const Operand& A, const Operand& B, int64_t k0, int64_t k1, uint8_t* base,
                                           Bars* bar, int* err, int64_t (&hi)[16], int64_t (&lo)[16]) {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -235,6 +263,11 @@ __device__ __forceinline__ void tile_sums(const Operand& A, const Operand& B, in
                 __syncwarp();
                 if (lane == 0) tc::mbar_arrive(&bar->acce[d]);
                 const int w = 1 << (8 * (3 - (d & 3)));
+                if constexpr (kTail) {   // the digits' weights: back to integers (i + j = 8 to the nearest)
+                    const float up = __int_as_float((127 + 8 * d) << 23);
+#pragma unroll
+                    for (int c = 0; c < 16; ++c) v[c] *= up;
+                }
                 if (half == 0) {
 #pragma unroll
                     for (int c = 0; c < 16; ++c) hi[c] += (int64_t)__float2int_rn(v[c]) * w;
@@ -276,8 +309,15 @@ __device__ __forceinline__ void tile_sums(const Operand& A, const Operand& B, in
 #pragma unroll
                 for (int ks = 0; ks < kKs / 16; ++ks)   // +32 bytes of K per MMA
                     mma_f16_ss(tbase + (uint32_t)((i + j) * kN), da + (uint64_t)((i * kAPlane + 32 * ks) >> 4),
-                               db + (uint64_t)((j * kBPlane + 32 * ks) >> 4), tc::idesc_f16(kM, n),
+                               db + (uint64_t)((j * kBPlane + 32 * ks) >> 4),
+                               kTail ? tc::idesc_bf16(kM, n) : tc::idesc_f16(kM, n),
                                first && i == 0 && ks == 0 ? 0u : 1u);
+            }
+            if (kTail && i > 0) {   // plane 8 - i of B
+#pragma unroll
+                for (int ks = 0; ks < kKs / 16; ++ks)
+                    mma_f16_ss(tbase + (uint32_t)((kDiags - 1) * kN), da + (uint64_t)((i * kAPlane + 32 * ks) >> 4),
+                               db + (uint64_t)(((kSlices - i) * kBPlane + 32 * ks) >> 4), tc::idesc_bf16(kM, kN), 1u);
             }
             if (last) tc::mma_commit(&bar->accf[i]);   // accumulator i is complete
         }
@@ -305,9 +345,9 @@ __device__ __forceinline__ void tile_sums(const Operand& A, const Operand& B, in
                 break;
             }
             const int64_t kn = k0 + (s + 1) * kKs;   // past the end: zeros, never used
-            store_planes(w0, planes + (size_t)slot * kStageBytes, plane, off0);
+            store_planes<kTail>(w0, planes + (size_t)slot * kStageBytes, plane, off0);
             load_words<kGram>(O, m0, kn + g0, k1, w0);
-            store_planes(w1, planes + (size_t)slot * kStageBytes, plane, off1);
+            store_planes<kTail>(w1, planes + (size_t)slot * kStageBytes, plane, off1);
             tc::fence_async_smem();
             __syncwarp();
             if (lane == 0) tc::mbar_arrive(&bar->full[slot]);
@@ -529,7 +569,7 @@ tri_f64_tc_kernel(const double* __restrict__ K, const double* __restrict__ Linv,
     if (blockIdx.x > 0) {
         const Operand A{Kq, ld, i0, min((int64_t)kM, M - i0)};
         const Operand B{Lq, ld, n0, min((int64_t)kN, r - n0)};
-        tile_sums<false>(A, B, 0, min(r, n0 + kN), base, bar, err, hi, lo);
+        tile_sums<false, kBlockStages, true>(A, B, 0, min(r, n0 + kN), base, bar, err, hi, lo);
     }
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t i = i0 + 32 * (warp & 3) + lane;

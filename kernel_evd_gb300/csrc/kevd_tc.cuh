@@ -251,6 +251,9 @@ __host__ __device__ constexpr uint32_t idesc_f16(int M, int N) {
     return (1u << 4) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
+// The same, A and B bf16.
+__host__ __device__ constexpr uint32_t idesc_bf16(int M, int N) { return idesc_f16(M, N) | (1u << 7) | (1u << 10); }
+
 // D[tmem] (+)= A * B^T, kind::f16, A read from Tensor Memory (row m in lane m,
 // 16 elements of K in 8 consecutive 32-bit columns, two per column with the
 // lower K index in the low half) and B from shared memory.
