@@ -347,7 +347,19 @@ int kevd_factor_from_linv(kevd_ctx* ctx, const float* X, int64_t N, int32_t d, d
     // 13.9 ms the call, 8.2 of them this product and 5.0 the kernel panels; relative
     // error against extended precision 1.2e-15); on the FP64 pipe (a triangular
     // multiply, half the work of a GEMM; 146 ms, 8.3e-15) where the product is
-    // smaller than the slices' launches, has no room, or Linv is not finite.
+    // smaller than the slices' launches, has no room, Linv is not finite, or the
+    // panel's outputs are too uneven for fixed point.
+    // Fixed point holds an output to its row's size.  Where the kernel spans many orders
+    // of magnitude, an output's own products may all be far below that: a sample of each
+    // panel's rows says how far (launch_tri_range).  The limits keep the product's error
+    // below half of an FP64 rounding, for an FP32 factor below 2^-34.  States of
+    // Kuramoto-Sivashinsky flows at the calibrated bandwidth measure 2^12 .. 2^13.7, at
+    // 1.25 times its scale 2^15 .. 2^17.7, at twice 2^24 .. 2^30.  A first panel that does
+    // not suit sends the whole call to the FP64 pipe; later ones are looked at in the end.
+    const double range_limit = precision == KEVD_FP64 ? 0x1p15 : 0x1p33;
+    const int64_t n_panels = (N + rows - 1) / rows;
+    double* part = nullptr;
+    int* skip = nullptr;
     uint64_t *Kq = nullptr, *Lq = nullptr;
     int *ek = nullptr, *el = nullptr, *pre = nullptr, *flags = nullptr;
     bool tc = (double)N * (double)r * (double)r >= 1e8;
@@ -358,6 +370,8 @@ int kevd_factor_from_linv(kevd_ctx* ctx, const float* X, int64_t N, int32_t d, d
         ek = arena_get<int>(ctx, "fl.ek", (size_t)rows, &st2);
         el = arena_get<int>(ctx, "fl.el", (size_t)r + 1, &st2);
         pre = arena_get<int>(ctx, "fl.pre", (size_t)rows * ((r + 63) / 64), &st2);
+        part = arena_get<double>(ctx, "fl.part", tri_range_size(r), &st2);
+        skip = arena_get<int>(ctx, "fl.skip", (size_t)n_panels, &st2);
         tc = st2 == KEVD_OK && (rows + 127) / 128 <= 65535;
     }
     if (tc) {
@@ -384,30 +398,19 @@ int kevd_factor_from_linv(kevd_ctx* ctx, const float* X, int64_t N, int32_t d, d
         if (ktc) KEVD_TRY(launch_digits_states(ctx, X, 0, idx, r, d, xe, sd, s));
     }
     double* Fp = nullptr;
-    if (!tc && precision == KEVD_MIXED) {
-        Fp = arena_get<double>(ctx, "fl.F", (size_t)rows * r, &st);
-        if (st != KEVD_OK) return set_error(ctx, st, "factor_from_linv: out of device memory");
-    }
     KEVD_BLAS(ctx, cublasSetStream(ctx->blas, s));
     const double one = 1.0;
-    for (int64_t r0 = 0; r0 < N; r0 += rows) {
-        const int64_t nr = std::min(rows, N - r0);
-        {
-            ProfScope ps(ctx, "linv_kernel_block", s);
-            if (ktc) {
-                KEVD_TRY(launch_digits_states(ctx, X, r0, nullptr, nr, d, xe, xd, s));
-                KEVD_TRY(launch_kernel_f64_tc(ctx, xd, nr, sd, r, d, xe, scale, Kp, r, flags, s));
-            } else {
-                KEVD_TRY(launch_kernel_block(ctx, X, N, d, scale, nullptr, r0, nr, idx, r, KEVD_FP64, Kp, r, s));
-            }
-        }
+    auto kernel_panel = [&](int64_t r0, int64_t nr) -> int {
+        ProfScope ps(ctx, "linv_kernel_block", s);
+        if (!ktc) return launch_kernel_block(ctx, X, N, d, scale, nullptr, r0, nr, idx, r, KEVD_FP64, Kp, r, s);
+        KEVD_TRY(launch_digits_states(ctx, X, r0, nullptr, nr, d, xe, xd, s));
+        return launch_kernel_f64_tc(ctx, xd, nr, sd, r, d, xe, scale, Kp, r, flags, s);
+    };
+    auto pipe_product = [&](int64_t r0, int64_t nr) -> int {
         ProfScope ps(ctx, "linv_multiply", s);
-        if (tc) {
-            KEVD_TRY(launch_digits_rows(ctx, Kp, nr, r, r, false, false, Kq, ek, pre, s));
-            KEVD_TRY(launch_tri_f64_tc(ctx, TriOperands{Kp, Li, Kq, Lq, ek, el, pre}, nr, r,
-                                       precision == KEVD_FP64 ? (double*)F + r0 * ldF : nullptr,
-                                       precision == KEVD_FP64 ? nullptr : (float*)F + r0 * ldF, ldF, flags, s));
-            continue;
+        if (precision == KEVD_MIXED && !Fp) {
+            Fp = arena_get<double>(ctx, "fl.F", (size_t)rows * r, &st);
+            if (st != KEVD_OK) return set_error(ctx, st, "factor_from_linv: out of device memory");
         }
         // (F panel)^T = Linv * (K panel)^T  in column-major terms
         double* dst = precision == KEVD_FP64 ? (double*)F + r0 * ldF : Fp;
@@ -420,11 +423,43 @@ int kevd_factor_from_linv(kevd_ctx* ctx, const float* X, int64_t N, int32_t d, d
             cast_d2f_kernel<<<grid, 256, 0, s>>>(Fp, nr, r, r, (float*)F + r0 * ldF, ldF);
             KEVD_LAUNCH(ctx);
         }
+        return KEVD_OK;
+    };
+    std::vector<int> unsuited((size_t)n_panels, 0);
+    for (int64_t q = 0; q < n_panels; ++q) {
+        const int64_t r0 = q * rows, nr = std::min(rows, N - r0);
+        KEVD_TRY(kernel_panel(r0, nr));
+        if (tc) {
+            ProfScope ps(ctx, "linv_multiply", s);
+            const TriOperands o{Kp, Li, Kq, Lq, ek, el, pre};
+            KEVD_TRY(launch_digits_rows(ctx, Kp, nr, r, r, false, false, Kq, ek, pre, s));
+            KEVD_TRY(launch_tri_range(ctx, o, nr, r, range_limit, part, skip + q, s));
+            if (q == 0) {
+                KEVD_CUDA(ctx, cudaMemcpyAsync(unsuited.data(), skip, sizeof(int), cudaMemcpyDeviceToHost, s));
+                KEVD_CUDA(ctx, cudaStreamSynchronize(s));
+                tc = unsuited[0] == 0;
+            }
+            if (tc)
+                KEVD_TRY(launch_tri_f64_tc(ctx, o, nr, r, precision == KEVD_FP64 ? (double*)F + r0 * ldF : nullptr,
+                                           precision == KEVD_FP64 ? nullptr : (float*)F + r0 * ldF, ldF, skip + q, flags,
+                                           s));
+        }
+        if (!tc) KEVD_TRY(pipe_product(r0, nr));
     }
     int herr = 0;
-    if (tc) KEVD_CUDA(ctx, cudaMemcpyAsync(&herr, flags, sizeof(int), cudaMemcpyDeviceToHost, s));
+    if (flags) KEVD_CUDA(ctx, cudaMemcpyAsync(&herr, flags, sizeof(int), cudaMemcpyDeviceToHost, s));
+    if (tc) KEVD_CUDA(ctx, cudaMemcpyAsync(unsuited.data(), skip, n_panels * sizeof(int), cudaMemcpyDeviceToHost, s));
     KEVD_CUDA(ctx, cudaStreamSynchronize(s));
     if (herr != 0) return set_error(ctx, KEVD_ERR_TIMEOUT, "factor_from_linv: pipeline wait timed out (code %d)", herr);
+    bool again = false;
+    for (int64_t q = 0; tc && q < n_panels; ++q) {
+        if (!unsuited[q]) continue;
+        const int64_t r0 = q * rows, nr = std::min(rows, N - r0);
+        KEVD_TRY(kernel_panel(r0, nr));
+        KEVD_TRY(pipe_product(r0, nr));
+        again = true;
+    }
+    if (again) KEVD_CUDA(ctx, cudaStreamSynchronize(s));
     return KEVD_OK;
 }
 

@@ -522,6 +522,12 @@ __global__ void __launch_bounds__(256) digits_rows_kernel(const double* __restri
         out[i * ld + c] = c < kc ? pack_digits(A[i * sr + c * sc], e) : kZeroDigits;
 }
 
+__device__ __forceinline__ double warp_sum(double v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
 // One output of a row product (NaN where an operand row is not finite).
 __device__ __forceinline__ double row_value(int64_t hi, int64_t lo, int e, int en) {
     return e == kDigitsNotFinite || en == kDigitsNotFinite ? (double)NAN : ldexp(tile_value(hi, lo), e + en);
@@ -556,11 +562,14 @@ rows_f64_tc_kernel(const uint64_t* __restrict__ Aq, const int* __restrict__ ea, 
 // a later tile when the entries of the tiles before lie more than 2^-kPrefixBits
 // below that largest entry.
 constexpr int kPrefixBits = 4;
+__device__ __forceinline__ bool tri_direct(int ek, int prefix) { return ek - prefix > kPrefixBits; }
+
 __global__ void __launch_bounds__(kThreads, 1)
 tri_f64_tc_kernel(const double* __restrict__ K, const double* __restrict__ Linv, const uint64_t* __restrict__ Kq,
                   const uint64_t* __restrict__ Lq, const int* __restrict__ ek, const int* __restrict__ el,
                   const int* __restrict__ prefix, int64_t M, int64_t r, int64_t ld, double* __restrict__ Fd,
-                  float* __restrict__ Ff, int64_t ldF, int* __restrict__ err) {
+                  float* __restrict__ Ff, int64_t ldF, const int* __restrict__ skip, int* __restrict__ err) {
+    if (*skip) return;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* base = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     Bars* bar = reinterpret_cast<Bars*>(base + 2 * (size_t)kStageBytes);
@@ -575,7 +584,7 @@ tri_f64_tc_kernel(const double* __restrict__ K, const double* __restrict__ Linv,
     const int64_t i = i0 + 32 * (warp & 3) + lane;
     if (i >= M) return;
     const int e = ek[i];
-    const bool direct = blockIdx.x == 0 || e - prefix[i * nb + blockIdx.x - 1] > kPrefixBits;
+    const bool direct = blockIdx.x == 0 || tri_direct(e, prefix[i * nb + blockIdx.x - 1]);
 #pragma unroll
     for (int c = 0; c < 16; ++c) {
         const int64_t n = n0 + 16 * (warp >> 2) + c;
@@ -590,6 +599,90 @@ tri_f64_tc_kernel(const double* __restrict__ K, const double* __restrict__ Linv,
         if (Fd) Fd[i * ldF + n] = v;
         else Ff[i * ldF + n] = (float)v;
     }
+}
+
+// |x| 2^-e in FP32, rounded towards 0, for |x| <= 2^e (0 below 2^-126).
+__device__ __forceinline__ float scaled_abs(double x, int e) {
+    const uint32_t hi = (uint32_t)__double2hiint(x) & 0x7fffffffu;
+    const int ex = (int)(hi >> 20) - e - (1023 - 127);
+    return ex <= 0 ? 0.f : __uint_as_float(((uint32_t)ex << 23) | ((hi & 0xfffffu) << 3) | ((uint32_t)__double2loint(x) >> 29));
+}
+
+// Sum and count over 32 columns of four sample rows of (n + 1) / S^2, S = sum_{k <= n}
+// |K(i, k) Linv(n, k)| / 2^(ek + el), for the outputs that the digits form.  Thread (j, c)
+// of 8 x 32 takes every eighth k of column c.
+__global__ void __launch_bounds__(256)
+tri_range_kernel(const double* __restrict__ K, const double* __restrict__ Linv, const int* __restrict__ ek,
+                 const int* __restrict__ el, const int* __restrict__ prefix, int64_t M, int64_t r,
+                 double* __restrict__ part) {
+    __shared__ float ks[128][4];
+    __shared__ float sums[8][32][4];
+    __shared__ int64_t row[4];
+    const int tid = threadIdx.x, c = tid & 31, j = tid >> 5;
+    const int64_t nb = (r + kN - 1) / kN, n0 = (int64_t)blockIdx.x * 32, n = n0 + c;
+    if (tid < 4) {
+        uint64_t z = ((uint64_t)blockIdx.y * 4 + tid + 1) * 0x9E3779B97F4A7C15ull;   // splitmix64
+        z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
+        z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
+        z ^= z >> 31;
+        row[tid] = (int64_t)((z >> 32) * (uint64_t)M >> 32);
+    }
+    __syncthreads();
+    const int en = n < r ? el[n] : 0;
+    const double* L = Linv + (n < r ? n : 0);
+    float s[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int64_t k0 = 0; k0 < min(r, n0 + 32); k0 += 128) {
+        __syncthreads();
+        for (int e = tid; e < 512; e += 256) {
+            const int64_t k = k0 + (e >> 2), i = row[e & 3];
+            ks[e >> 2][e & 3] = k < r ? scaled_abs(K[i * r + k], ek[i]) : 0.f;
+        }
+        __syncthreads();
+        const int kn = n < r ? (int)min((int64_t)128, n + 1 - k0) : 0;
+#pragma unroll 8
+        for (int k = j; k < kn; k += 8) {
+            const float l = scaled_abs(L[(k0 + k) * r], en);
+            const float4 x = *reinterpret_cast<const float4*>(ks[k]);
+            s[0] = fmaf(x.x, l, s[0]);
+            s[1] = fmaf(x.y, l, s[1]);
+            s[2] = fmaf(x.z, l, s[2]);
+            s[3] = fmaf(x.w, l, s[3]);
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) sums[j][c][q] = s[q];
+    __syncthreads();
+    if (j != 0) return;
+    double v = 0.0, cnt = 0.0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        float t = 0.f;
+        for (int u = 0; u < 8; ++u) t += sums[u][c][q];
+        const int64_t i = row[q];
+        if (n < r && n >= kN && !tri_direct(ek[i], prefix[i * nb + n / kN - 1])) {
+            v += (double)(n + 1) / ((double)t * (double)t);
+            cnt += 1.0;
+        }
+    }
+    v = warp_sum(v);
+    cnt = warp_sum(cnt);
+    if (c == 0) {
+        double* out = part + 2 * (blockIdx.y * gridDim.x + blockIdx.x);
+        out[0] = v;
+        out[1] = cnt;
+    }
+}
+
+// *skip from the parts, in a fixed order.  One warp.
+__global__ void tri_suited_kernel(const double* __restrict__ part, int n, double limit, int* __restrict__ skip) {
+    double v = 0.0, c = 0.0;
+    for (int q = threadIdx.x; q < n; q += 32) {
+        v += part[2 * q];
+        c += part[2 * q + 1];
+    }
+    v = warp_sum(v);
+    c = warp_sum(c);
+    if (threadIdx.x == 0) *skip = c == 0.0 || v <= limit * limit * c ? 0 : 1;   // NaN: skip
 }
 
 // ---- kernel blocks -------------------------------------------------------------------
@@ -738,12 +831,22 @@ int launch_rows_f64_tc(kevd_ctx* ctx, const uint64_t* A, const int* ea, int64_t 
 }
 
 int launch_tri_f64_tc(kevd_ctx* ctx, const TriOperands& o, int64_t M, int64_t r, double* Fd, float* Ff, int64_t ldF,
-                      int* err, cudaStream_t st) {
+                      const int* skip, int* err, cudaStream_t st) {
     KEVD_CUDA(ctx, raise_smem_limit(reinterpret_cast<const void*>(&tri_f64_tc_kernel), kSmem));
     const dim3 grid((unsigned)((r + kN - 1) / kN), (unsigned)((M + kM - 1) / kM));
     if (grid.y > kMaxRowTiles) return set_error(ctx, KEVD_ERR_ARG, "tri_f64_tc: too many rows");
     tri_f64_tc_kernel<<<grid, kThreads, kSmem, st>>>(o.K, o.Linv, o.Kq, o.Lq, o.ek, o.el, o.prefix, M, r, digits_ld(r),
-                                                     Fd, Ff, ldF, err);
+                                                     Fd, Ff, ldF, skip, err);
+    KEVD_LAUNCH(ctx);
+    return KEVD_OK;
+}
+
+int launch_tri_range(kevd_ctx* ctx, const TriOperands& o, int64_t M, int64_t r, double limit, double* part, int* skip,
+                     cudaStream_t st) {
+    const dim3 grid((unsigned)((r + 31) / 32), kRangeRows / 4);
+    tri_range_kernel<<<grid, 256, 0, st>>>(o.K, o.Linv, o.ek, o.el, o.prefix, M, r, part);
+    KEVD_LAUNCH(ctx);
+    tri_suited_kernel<<<1, 32, 0, st>>>(part, (int)(grid.x * grid.y), limit, skip);
     KEVD_LAUNCH(ctx);
     return KEVD_OK;
 }

@@ -42,8 +42,18 @@ struct TriOperands {
     const uint64_t *Kq, *Lq;
     const int *ek, *el, *prefix;
 };
+// *skip != 0: nothing is done.
 int launch_tri_f64_tc(kevd_ctx* ctx, const TriOperands& o, int64_t M, int64_t r, double* Fd, float* Ff, int64_t ldF,
-                      int* err, cudaStream_t st);
+                      const int* skip, int* err, cudaStream_t st);
+
+// Whether launch_tri_f64_tc keeps the outputs of this panel to FP64 accuracy, by a sample
+// of its rows: *skip = 0 where the root mean square over their outputs of
+// sqrt(n + 1) 2^(ek + el) / sum |K| |Linv| is at most limit, else 1; the product's error
+// is 2^-67.2 of the sum a unit.  part: device, tri_range_size(r) doubles.
+constexpr int kRangeRows = 32;
+inline size_t tri_range_size(int64_t r) { return (size_t)(2 * (kRangeRows / 4) * ((r + 31) / 32)); }
+int launch_tri_range(kevd_ctx* ctx, const TriOperands& o, int64_t M, int64_t r, double limit, double* part, int* skip,
+                     cudaStream_t st);
 
 // Kernel blocks K(i, c) = exp(-scale ||x_i - s_c||^2) in FP64 from exact squared
 // distances (integer digits of the FP32 states at one common exponent).
