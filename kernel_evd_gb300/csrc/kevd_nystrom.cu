@@ -118,7 +118,11 @@ __device__ __forceinline__ void stage_rows(const float* __restrict__ src, int64_
 // two thirds of the FP32 pipe; fewer CTAs per 32 states with more landmark groups
 // each is no faster: 923 to 956 us); Q = 1 is for batches
 // that would leave SMs without a CTA otherwise.
-template <int Q>   // 1 or 4
+//
+// kOne: one CTA, without a cluster, takes all groups of its states in turn: the same
+// sums in the same order, group by group.  Few landmarks leave a CTA of the cluster one
+// step or none, and its start, its staging of the states and the hand-over cost more.
+template <int Q, bool kOne>   // Q = 1 or 4
 __global__ void __launch_bounds__(544)
 nystrom_eval_kernel(const float* __restrict__ Y, int64_t n, const float* __restrict__ xs,
                     const float2* __restrict__ w, const int* __restrict__ ex, int64_t r, int d, int k_out,
@@ -131,13 +135,12 @@ nystrom_eval_kernel(const float* __restrict__ Y, int64_t n, const float* __restr
     float* ys = xt + 2 * kLm * p;                             // kRows x p
     float2* wt = reinterpret_cast<float2*>(ys + kRows * p);   // 2 x kLm x kc
     float* kv = reinterpret_cast<float*>(wt + 2 * kLm * kc);  // kv_floats
-    cg::cluster_group cluster = cg::this_cluster();
-    const int group = (int)cluster.block_rank();
+    const int group = kOne ? 0 : (int)cg::this_cluster().block_rank();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int64_t row0 = (int64_t)(blockIdx.x / kGroups) * kRows;
+    const int64_t row0 = (int64_t)(kOne ? blockIdx.x : blockIdx.x / kGroups) * kRows;
     const int64_t steps_all = (r + kLm - 1) / kLm;
     const int64_t per = (steps_all + kGroups - 1) / kGroups;
-    const int64_t s0 = min(steps_all, group * per), s1 = min(steps_all, s0 + per);
+    const int64_t s0 = min(steps_all, group * per), s1 = kOne ? steps_all : min(steps_all, s0 + per);
     const int n_f = (d + kFeat - 1) / kFeat;   // feature chunks per step
     const bool vec = (d & 3) == 0 && ((uintptr_t)Y & 15) == 0;
     const bool vecx = (d & 3) == 0;            // xs is an allocation of its own
@@ -159,6 +162,18 @@ nystrom_eval_kernel(const float* __restrict__ Y, int64_t n, const float* __restr
     f32x2 sum2[2] = {0, 0}, err2[2] = {0, 0};   // Q = 4: pairs of states
 #pragma unroll
     for (int q = 0; q < Q; ++q) sum[q] = err[q] = 0.f;
+    double total[Q];   // kOne: the groups so far
+#pragma unroll
+    for (int q = 0; q < Q; ++q) total[q] = 0.0;
+    auto unpack_sums = [&] {
+        if constexpr (Q == 4) {
+            unpack2(sum2[0], sum[0], sum[1]);
+            unpack2(sum2[1], sum[2], sum[3]);
+            unpack2(err2[0], err[0], err[1]);
+            unpack2(err2[1], err[2], err[3]);
+        }
+    };
+    int64_t left = per;   // kOne: steps of this group still to come
 
     if (s0 < s1) {
         stage_rows(Y, n, d, row0, kRows, 0, min(kFeat, d), vec, ys, p);
@@ -229,21 +244,38 @@ nystrom_eval_kernel(const float* __restrict__ Y, int64_t n, const float* __restr
                     pair_fma(sum[0], err[0], kv[rg * (kLm + 1) + j], wv);
                 }
             }
+            if (kOne && (--left == 0 || s + 1 == s1)) {
+                unpack_sums();
+#pragma unroll
+                for (int q = 0; q < Q; ++q) {
+                    total[q] += (double)sum[q] + (double)err[q];
+                    sum[q] = err[q] = 0.f;
+                }
+                sum2[0] = sum2[1] = err2[0] = err2[1] = 0;
+                left = per;
+            }
         }
     }
-    if constexpr (Q == 4) {
-        unpack2(sum2[0], sum[0], sum[1]);
-        unpack2(sum2[1], sum[2], sum[3]);
-        unpack2(err2[0], err[0], err[1]);
-        unpack2(err2[1], err[2], err[3]);
-    }
+    if (!kOne) unpack_sums();
     tc::cp_async_wait<0>();
     __syncthreads();
     double* part = reinterpret_cast<double*>(ny_smem);   // kRows x kc, over the tiles
     if (rg < kLanesR) {
 #pragma unroll
-        for (int q = 0; q < Q; ++q) part[(rg + kLanesR * q) * kc + c] = (double)sum[q] + (double)err[q];
+        for (int q = 0; q < Q; ++q)
+            part[(rg + kLanesR * q) * kc + c] = kOne ? total[q] : (double)sum[q] + (double)err[q];
     }
+    if constexpr (kOne) {
+        __syncthreads();
+        for (int e = tid; e < kRows * k_out; e += blockDim.x) {
+            const int rr = e / k_out, cc = e - rr * k_out;
+            if (row0 + rr < n)
+                Uy[(row0 + rr) * k_out + cc] =
+                    (float)ldexp(part[rr * kc + cc] / part[rr * kc + k_out], ex[cc] - ex[k_out]);
+        }
+        return;
+    }
+    cg::cluster_group cluster = cg::this_cluster();
     cluster.sync();
     // the cluster's CTAs share the outputs; every sum runs over the groups in order
     for (int e = group * blockDim.x + tid; e < kRows * k_out; e += kGroups * blockDim.x) {
@@ -297,17 +329,17 @@ __global__ void __launch_bounds__(256) nystrom_pack_kernel(const double* __restr
     if (threadIdx.x == 0) ex[c] = e;
 }
 
-template <int Q>
+template <int Q, bool kOne>
 int launch_eval(kevd_ctx* ctx, const Model& m, const float* Y, int64_t n, float* Uy, cudaStream_t s) {
     const int kc = m.k_out + 1;
     const int64_t blocks = (n + kLanesR * Q - 1) / (kLanesR * Q);
     const size_t smem = smem_bytes<Q>(m.d, kc);
-    const void* fn = reinterpret_cast<const void*>(&nystrom_eval_kernel<Q>);
+    const void* fn = reinterpret_cast<const void*>(&nystrom_eval_kernel<Q, kOne>);
     KEVD_CUDA(ctx, raise_smem_limit(fn, std::max(smem, (size_t)48 * 1024)));
     // 16 CTAs per cluster is above the portable 8
-    KEVD_CUDA(ctx, cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    if (!kOne) KEVD_CUDA(ctx, cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(blocks * kGroups));
+    cfg.gridDim = dim3((unsigned)(kOne ? blocks : blocks * kGroups));
     cfg.blockDim = dim3((unsigned)std::max(kMinThreads, (kLanesR * kc + 31) / 32 * 32));
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
@@ -316,8 +348,8 @@ int launch_eval(kevd_ctx* ctx, const Model& m, const float* Y, int64_t n, float*
     at[0].val.clusterDim.x = kGroups;
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
-    cfg.numAttrs = 1;
-    KEVD_CUDA(ctx, cudaLaunchKernelEx(&cfg, &nystrom_eval_kernel<Q>, Y, n, (const float*)m.xs, (const float2*)m.w,
+    cfg.numAttrs = kOne ? 0 : 1;
+    KEVD_CUDA(ctx, cudaLaunchKernelEx(&cfg, &nystrom_eval_kernel<Q, kOne>, Y, n, (const float*)m.xs, (const float2*)m.w,
                                       (const int*)m.ex, m.r, m.d, m.k_out, split_scale(m.scale), Uy));
     KEVD_LAUNCH(ctx);
     return KEVD_OK;
@@ -331,14 +363,25 @@ int launch_nystrom_pack(kevd_ctx* ctx, const double* zp, const Model& m, cudaStr
     return KEVD_OK;
 }
 
-// 32 states per cluster once those clusters give every SM a CTA (n > 300);
-// fewer states are served 8 per cluster.
+// Clusters split the landmarks 16 ways and start 16 CTAs for 32 states; one CTA walks
+// through all of them.  Times in us, clusters / one CTA (d = 64, 8 columns): 100
+// landmarks n = 1,000 27 / 23, 16,384 229 / 43; 300 1,000 27 / 48, 4,096 68 / 48, 65,536
+// 905 / 319; 1,000 4,096 97 / 132, 16,384 335 / 292; 2,000 16,384 581 / 563 (32 columns 898
+// / 992), 65,536 2,262 / 1,863.
+static bool one_cta(int64_t r, int64_t n) {
+    return 200 * ((r + kLm - 1) / kLm) <= std::min<int64_t>(n, 4096) + std::max<int64_t>(0, n - 4096) / 5;
+}
+
+// 32 states per cluster once those clusters give every SM a CTA (n > 300), or per CTA
+// (one_cta); fewer states are served 8 per cluster.
 int launch_nystrom_eval(kevd_ctx* ctx, const Model& m, const float* Y, int64_t n, float* Uy, cudaStream_t s) {
     constexpr int64_t kPiece = (int64_t)1 << 30;   // states per launch: the grid stays below 2^31 CTAs
     for (int64_t i = 0; i < n; i += kPiece) {
         const int64_t ni = std::min(kPiece, n - i);
-        if (ni > 2 * ctx->num_sms) KEVD_TRY(launch_eval<4>(ctx, m, Y + i * m.d, ni, Uy + i * m.k_out, s));
-        else KEVD_TRY(launch_eval<1>(ctx, m, Y + i * m.d, ni, Uy + i * m.k_out, s));
+        auto launch = ni <= 2 * ctx->num_sms ? &launch_eval<1, false>
+                      : one_cta(m.r, ni)     ? &launch_eval<4, true>
+                                             : &launch_eval<4, false>;
+        KEVD_TRY(launch(ctx, m, Y + i * m.d, ni, Uy + i * m.k_out, s));
     }
     return KEVD_OK;
 }
