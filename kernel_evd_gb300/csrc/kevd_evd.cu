@@ -184,7 +184,7 @@ __global__ void ev_gram_reduce_kernel(const double* __restrict__ partial, int n_
     for (int e = threadIdx.x; e < kGT * kGT; e += blockDim.x) {
         const int ia = e / kGT, ib = e - ia * kGT;
         const int64_t ga = ta * kGT + ia, gb = tb * kGT + ib;
-        if (ga >= k || gb >= k) continue;
+        if (ga >= k || gb > ga) continue;   // of a diagonal tile one triangle: the other rounds differently
         double s = 0.0;
         for (int p = 0; p < n_split; ++p) s += partial[((int64_t)p * n_tiles + t) * kGT * kGT + e];
         G[gb * k + ga] = s;   // (ga, gb)
