@@ -221,7 +221,8 @@ int kevd_rpchol(kevd_ctx* ctx, const float* X, int64_t N, int32_t d,
  * parallel branches of one CUDA graph, which is launched on stream until all
  * jobs have stopped (kernels of a stopped job return at once).  use_graph == 0:
  * the same rounds are issued on one stream per job.  The jobs' workspaces stay
- * with ctx when they hold at most 1 GiB. */
+ * with ctx when they hold at most 1 GiB; they and the buffers of other calls
+ * are given back when a call on ctx runs out of device memory. */
 typedef struct {
     const float* X;
     int64_t N;

@@ -619,7 +619,10 @@ static int run_bracketed_median(kevd_ctx* ctx, const float* X, int64_t N, int d,
     float* buf = arena_get<float>(ctx, "med.buf", cap, &st);
     unsigned* smp = arena_get<unsigned>(ctx, "med.smp", (size_t)n + 3, &st);
     unsigned long long* cnt = arena_get<unsigned long long>(ctx, "med.cnt", 2, &st);
-    if (st != KEVD_OK) return KEVD_OK;
+    if (st != KEVD_OK) {
+        for (const char* b : {"med.buf", "med.smp", "med.cnt"}) ctx->arena.idle(b);
+        return KEVD_OK;
+    }
     unsigned* br = smp + n;
     KEVD_CUDA(ctx, cudaMemsetAsync(cnt, 0, 2 * sizeof(*cnt), s));
     median_sample_kernel<<<n / 256, 256, 0, s>>>(X, N, d, n, smp);

@@ -32,6 +32,7 @@ void* Arena::get(const std::string& name, size_t bytes, int* status) {
     if (*status != KEVD_OK) return nullptr;
     Buf& b = bufs_[name];
     if (bytes == 0) bytes = 1;
+    if (b.call != kHeld) b.call = call_;
     if (b.n >= bytes) return b.p;
     if (b.p) cudaFree(b.p);
     b.p = nullptr;
@@ -68,6 +69,29 @@ void Arena::release() {
     bufs_.clear();
 }
 
+void Arena::idle(const std::string& name) {
+    auto it = bufs_.find(name);
+    if (it != bufs_.end() && it->second.call != kHeld) it->second.call = -1;
+}
+
+void Arena::hold(const std::string& name) {
+    auto it = bufs_.find(name);
+    if (it != bufs_.end()) it->second.call = kHeld;
+}
+
+bool Arena::reclaim() {
+    bool any = false;
+    for (auto& kv : bufs_) {
+        Buf& b = kv.second;
+        if (!b.p || b.call >= call_) continue;
+        cudaFree(b.p);
+        b.p = nullptr;
+        b.n = 0;
+        any = true;
+    }
+    return any;
+}
+
 }  // namespace kevd
 
 struct kevd_model {
@@ -76,8 +100,9 @@ struct kevd_model {
 
 using namespace kevd;
 
-#define KEVD_CHECK_CTX(ctx) \
-    if (!(ctx)) return KEVD_ERR_ARG
+#define KEVD_CHECK_CTX(ctx)            \
+    if (!(ctx)) return KEVD_ERR_ARG; \
+    (ctx)->arena.begin_call()
 
 static void resolve_profile(kevd_ctx* ctx) {
     for (auto& r : ctx->pending) {
@@ -397,6 +422,12 @@ int kevd_factor_from_linv(kevd_ctx* ctx, const float* X, int64_t N, int32_t d, d
         ktc = ktc && st2 == KEVD_OK && (rows + 127) / 128 <= 65535;
         if (ktc) KEVD_TRY(launch_digits_states(ctx, X, 0, idx, r, d, xe, sd, s));
     }
+    auto idle_digits = [&] {
+        for (const char* b : {"fl.Kq", "fl.Lq", "fl.ek", "fl.el", "fl.pre", "fl.part", "fl.skip"}) ctx->arena.idle(b);
+    };
+    if (!ktc)
+        for (const char* b : {"fl.xq", "fl.xn", "fl.sq", "fl.sn"}) ctx->arena.idle(b);
+    if (!tc && !flags) idle_digits();
     double* Fp = nullptr;
     KEVD_BLAS(ctx, cublasSetStream(ctx->blas, s));
     const double one = 1.0;
@@ -406,9 +437,11 @@ int kevd_factor_from_linv(kevd_ctx* ctx, const float* X, int64_t N, int32_t d, d
         KEVD_TRY(launch_digits_states(ctx, X, r0, nullptr, nr, d, xe, xd, s));
         return launch_kernel_f64_tc(ctx, xd, nr, sd, r, d, xe, scale, Kp, r, flags, s);
     };
+    bool again = false;   // panels once more
     auto pipe_product = [&](int64_t r0, int64_t nr) -> int {
         ProfScope ps(ctx, "linv_multiply", s);
         if (precision == KEVD_MIXED && !Fp) {
+            if (!tc || again) idle_digits();   // from here on every panel comes this way
             Fp = arena_get<double>(ctx, "fl.F", (size_t)rows * r, &st);
             if (st != KEVD_OK) return set_error(ctx, st, "factor_from_linv: out of device memory");
         }
@@ -451,13 +484,12 @@ int kevd_factor_from_linv(kevd_ctx* ctx, const float* X, int64_t N, int32_t d, d
     if (tc) KEVD_CUDA(ctx, cudaMemcpyAsync(unsuited.data(), skip, n_panels * sizeof(int), cudaMemcpyDeviceToHost, s));
     KEVD_CUDA(ctx, cudaStreamSynchronize(s));
     if (herr != 0) return set_error(ctx, KEVD_ERR_TIMEOUT, "factor_from_linv: pipeline wait timed out (code %d)", herr);
-    bool again = false;
     for (int64_t q = 0; tc && q < n_panels; ++q) {
         if (!unsuited[q]) continue;
+        again = true;
         const int64_t r0 = q * rows, nr = std::min(rows, N - r0);
         KEVD_TRY(kernel_panel(r0, nr));
         KEVD_TRY(pipe_product(r0, nr));
-        again = true;
     }
     if (again) KEVD_CUDA(ctx, cudaStreamSynchronize(s));
     return KEVD_OK;
@@ -547,9 +579,9 @@ int kevd_nystrom_prepare(kevd_ctx* ctx, const float* X, int64_t N, int32_t d, do
     m->m.d = d;
     m->m.k_out = k_out;
     m->m.scale = scale;
-    if (cudaMalloc(&m->m.xs, (size_t)r * d * sizeof(float)) != cudaSuccess ||
-        cudaMalloc(&m->m.w, (size_t)r * (k_out + 1) * sizeof(float2)) != cudaSuccess ||
-        cudaMalloc(&m->m.ex, (size_t)(k_out + 1) * sizeof(int)) != cudaSuccess) {
+    if (device_alloc(ctx, (void**)&m->m.xs, (size_t)r * d * sizeof(float)) != cudaSuccess ||
+        device_alloc(ctx, (void**)&m->m.w, (size_t)r * (k_out + 1) * sizeof(float2)) != cudaSuccess ||
+        device_alloc(ctx, (void**)&m->m.ex, (size_t)(k_out + 1) * sizeof(int)) != cudaSuccess) {
         cudaGetLastError();
         kevd_model_destroy(m);
         return set_error(ctx, KEVD_ERR_NOMEM, "nystrom_prepare: out of device memory");

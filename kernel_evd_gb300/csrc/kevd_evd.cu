@@ -1003,7 +1003,10 @@ static int u_f64_tc(kevd_ctx* ctx, const double* F, int64_t ldF, int64_t N, int6
     uint64_t* zq = arena_get<uint64_t>(ctx, "f64.zq", (size_t)k_out * ld, &rc);
     int* ea = arena_get<int>(ctx, "f64.ea", (size_t)panel, &rc);
     int* ez = arena_get<int>(ctx, "f64.ez", (size_t)k_out + 1, &rc);
-    if (rc != KEVD_OK) return KEVD_OK;
+    if (rc != KEVD_OK) {
+        for (const char* b : {"f64.q", "f64.zq", "f64.ea", "f64.ez"}) ctx->arena.idle(b);
+        return KEVD_OK;
+    }
     int* err = ez + k_out;
     KEVD_CUDA(ctx, cudaMemsetAsync(err, 0, sizeof(int), st));
     KEVD_TRY(launch_digits_rows(ctx, Z, k_out, k, k, false, false, zq, ez, nullptr, st));

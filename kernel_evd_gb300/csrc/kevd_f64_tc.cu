@@ -908,6 +908,14 @@ int run_gram_f64_tc(kevd_ctx* ctx, const double* F, int64_t N, int64_t k, int64_
     double* partial = arena_get<double>(ctx, "f64.part", (size_t)n_split * n_tiles * kM * kN, &rc);
     unsigned long long* colmax = arena_get<unsigned long long>(ctx, "f64.max", (size_t)2 * k, &rc);   // and diag8
     int* e = arena_get<int>(ctx, "f64.exp", (size_t)k + 2, &rc);
+    // the caller's later buffers come first: these are free for them once the call
+    // returns, and with no room for all of them none is kept
+    struct Idle {
+        kevd_ctx* ctx;
+        ~Idle() {
+            for (const char* b : {"f64.q", "f64.part", "f64.max", "f64.exp"}) ctx->arena.idle(b);
+        }
+    } idle{ctx};
     if (rc != KEVD_OK) return KEVD_OK;   // no room for the slices: not done
     int* flags = e + k;                  // error, unsuited column
     KEVD_CUDA(ctx, cudaMemsetAsync(colmax, 0, (size_t)2 * k * sizeof(*colmax), st));

@@ -29,12 +29,21 @@ struct Error {
 };
 
 // One named, growable device buffer per purpose.  Buffers are reused across
-// calls and only grow; they are released with the context.
+// calls and only grow; they are released with the context, and those that the
+// current call does not use when memory runs out (reclaim).
 class Arena {
   public:
     ~Arena() { release(); }
     void* get(const std::string& name, size_t bytes, int* status);
     void release();
+    // A call of the C interface begins: buffers got before are no longer in use.
+    void begin_call() { ++call_; }
+    // The current call is done with a buffer (or did without it).
+    void idle(const std::string& name);
+    // A buffer that stays in use across calls.
+    void hold(const std::string& name);
+    // Free the buffers that are not in use (waits for the device); whether there were any.
+    bool reclaim();
     size_t total() const {
         size_t t = 0;
         for (const auto& kv : bufs_) t += kv.second.n;
@@ -45,8 +54,11 @@ class Arena {
     struct Buf {
         void* p = nullptr;
         size_t n = 0;
+        int64_t call = -1;   // the last call that got it
     };
+    static constexpr int64_t kHeld = INT64_MAX;
     std::map<std::string, Buf> bufs_;
+    int64_t call_ = 0;
 };
 
 }  // namespace kevd
@@ -160,16 +172,33 @@ class ProfScope {
 
 void free_batch_pool(kevd_ctx* ctx);   // kevd_rpchol.cu
 
+// Out of device memory: give back what ctx keeps but does not use now, the batch's
+// workspaces and the buffers of earlier calls; whether there was anything.
+inline bool reclaim_memory(kevd_ctx* ctx) {
+    const bool pool = ctx->batch_pool != nullptr;
+    free_batch_pool(ctx);
+    return ctx->arena.reclaim() || pool;
+}
+
 template <typename T>
 T* arena_get(kevd_ctx* ctx, const char* name, size_t count, int* st) {
-    const int before = *st;
+    if (*st != KEVD_OK) return nullptr;
     T* p = static_cast<T*>(ctx->arena.get(name, count * sizeof(T), st));
-    if (!p && ctx->batch_pool) {   // out of memory: give the batch's workspaces back first
-        *st = before;
-        free_batch_pool(ctx);
+    if (!p && reclaim_memory(ctx)) {
+        *st = KEVD_OK;
         p = static_cast<T*>(ctx->arena.get(name, count * sizeof(T), st));
     }
     return p;
+}
+
+// cudaMalloc for what does not belong to the workspace, on the same terms.
+inline cudaError_t device_alloc(kevd_ctx* ctx, void** p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation && reclaim_memory(ctx)) {
+        cudaGetLastError();
+        e = cudaMalloc(p, bytes);
+    }
+    return e;
 }
 
 inline cudaStream_t as_stream(void* s) { return static_cast<cudaStream_t>(s); }

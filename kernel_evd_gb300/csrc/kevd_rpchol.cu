@@ -1249,21 +1249,27 @@ int run_rpchol_batched(kevd_ctx* ctx, kevd_rpchol_job* jobs, int n_jobs, int use
     // before the pool is taken: an allocation of ctx may give the pool back
     int* cnt = arena_get<int>(ctx, "rp.density", n_jobs, &rc);
     if (rc != KEVD_OK) return set_error(ctx, rc, "rpchol_batched: out of device memory");
-    rc = batch_pool(ctx, jobs, n_jobs, &pool);
-    if (rc == KEVD_OK) rc = rpchol_batched(ctx, jobs, n_jobs, use_graph != 0, *pool, cnt, &graph, &exec, s);
-    if (rc != KEVD_OK) {
-        // work may still be in flight on the caller's or the jobs' streams
-        cudaStreamSynchronize(s);
-        for (auto& x : pool->slots)
-            if (x.st) cudaStreamSynchronize(x.st);
-        cudaGetLastError();
+    // out of memory beside workspaces kept from earlier calls: once more without them
+    for (bool kept = ctx->batch_pool != nullptr;; kept = false) {
+        rc = batch_pool(ctx, jobs, n_jobs, &pool);
+        if (rc == KEVD_OK) rc = rpchol_batched(ctx, jobs, n_jobs, use_graph != 0, *pool, cnt, &graph, &exec, s);
+        if (rc != KEVD_OK) {
+            // work may still be in flight on the caller's or the jobs' streams
+            cudaStreamSynchronize(s);
+            for (auto& x : pool->slots)
+                if (x.st) cudaStreamSynchronize(x.st);
+            cudaGetLastError();
+        }
+        if (exec) cudaGraphExecDestroy(exec);
+        if (graph) cudaGraphDestroy(graph);
+        exec = nullptr;
+        graph = nullptr;
+        size_t held = 0;
+        for (auto& x : pool->slots) held += x.c ? x.c->arena.total() : 0;
+        if (held > kBatchKeepBytes || (int)pool->slots.size() > kBatchKeepJobs || rc != KEVD_OK) free_batch_pool(ctx);
+        const bool idle = rc == KEVD_ERR_NOMEM && ctx->arena.reclaim();
+        if (rc != KEVD_ERR_NOMEM || !(kept || idle)) return rc;
     }
-    if (exec) cudaGraphExecDestroy(exec);
-    if (graph) cudaGraphDestroy(graph);
-    size_t held = 0;
-    for (auto& x : pool->slots) held += x.c ? x.c->arena.total() : 0;
-    if (held > kBatchKeepBytes || (int)pool->slots.size() > kBatchKeepJobs || rc != KEVD_OK) free_batch_pool(ctx);
-    return rc;
 }
 
 // Gather rows idx of F (first ncols columns) into a column-major FP64 n x ncols

@@ -199,6 +199,8 @@ void factor_worker(kevd_server* s, int wi) {
         // keeps for the next request (no allocation or free per request)
         float* X = arena_get<float>(w.ctx, "srv.X", (size_t)r->N * r->d, &rc);
         void* F = arena_get<uint8_t>(w.ctx, "srv.F", fbytes, &rc);
+        w.ctx->arena.hold("srv.X");   // across the calls below
+        w.ctx->arena.hold("srv.F");
         std::vector<int64_t> piv((size_t)r->k);
         kevd_rpchol_result res = {0, 0, 0.0};
         if (rc == KEVD_OK && cudaMemcpyAsync(X, r->X.data(), (size_t)r->N * r->d * 4, cudaMemcpyHostToDevice,
