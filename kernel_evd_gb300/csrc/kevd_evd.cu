@@ -976,9 +976,6 @@ static int gram_f64(kevd_ctx* ctx, const double* F, int64_t ldF, int64_t N, int6
     return gram<double>(ctx, F, ldF, N, k, wbuf, G, st);
 }
 
-// U = Dtil^{-1} F Z (row-major float) of an FP64 factor, in exact slices on the
-// tensor cores, row panels of at most 2 GiB of digits at a time; *done = false
-// when there is no room for them.
 // U and Y of at most 32 columns of Z from the column-major FP32 factor.
 static int u_f32(kevd_ctx* ctx, const float* FT, int64_t ldT, int64_t N, int64_t k, const double* Z, int m,
                  const double* dinv, float* U, float* Y, cudaStream_t s) {
@@ -993,6 +990,10 @@ static int u_f32(kevd_ctx* ctx, const float* FT, int64_t ldT, int64_t N, int64_t
     return KEVD_OK;
 }
 
+// U = Dtil^{-1} F Z (row-major float) of an FP64 factor, in exact slices on the
+// tensor cores, row panels of at most 2 GiB of digits at a time; *done = false
+// when there is no room for them.  Fixed point holds U to 2^-62 of max |F_i| max |Z_c|;
+// Z, an FP64 eigenvector, is known to 2^-53 of its largest entry.
 static int u_f64_tc(kevd_ctx* ctx, const double* F, int64_t ldF, int64_t N, int64_t k, const double* Z, int k_out,
                     const double* dinv, float* U, bool* done, cudaStream_t st) {
     *done = false;

@@ -1,5 +1,9 @@
 // FP64 products on the tensor cores in exact slices.
 //
+// The method is the error-free slicing of K. Ozaki, T. Ogita, S. Oishi and S. M. Rump,
+// Error-free transformations of matrix multiplication by using fast routines of matrix
+// multiplication, Numer. Algorithms 59 (2012), with digits in fixed point.
+//
 // The FP64 pipe of this GPU does 2 FMAs per clock and SM; the f16 tensor pipe
 // does 4096.  A matrix entry is turned into fixed point relative to the largest
 // entry of its row (of its column for a Gram), q = rn(x 2^(62 - e)) with

@@ -9,10 +9,10 @@ struct kevd_ctx;
 
 namespace kevd {
 
-// G (k x k, column-major, full) = F^T diag(s)^2 F of a row-major FP64 factor.
-// *done = false (nothing written) when the call does not suit the slices: the
-// workspace does not fit, or a column's largest entry is so far above its
-// root mean square that fixed point would lose digits (the caller then takes
+// G (k x k, column-major, full) = F^T diag(s)^2 F of a row-major FP64 factor, an entry
+// to a few 2^-53 of sqrt(G_aa G_bb).  *done = false, and G undefined, when the call does
+// not suit the slices: the workspace does not fit, or a column's largest entry is so far
+// above its root mean square that fixed point would lose digits (the caller then takes
 // the FP64 SIMT Gram).  s: device, N doubles.  Synchronises the stream.
 int run_gram_f64_tc(kevd_ctx* ctx, const double* F, int64_t N, int64_t k, int64_t ldF, const double* s, double* G,
                     bool* done, cudaStream_t st);

@@ -1,15 +1,13 @@
 // Residual update of one block-RPCholesky pass for an FP32 factor on the FP32
 // pipe: layouts the tensor-core update cannot read by TMA (ldF not a multiple of
-// 4) and nearly diagonal kernels.  The same pass as rp_update_kernel<float> of
-// kevd_rpchol.cu did, operation by operation:
+// 4) and nearly diagonal kernels.  The operations and their order are part of the
+// result, because the pivots of a run follow every rounding of d:
 //
 //   P(i, q) = sum_c F(i, c) F(s_q, c)   one FMA chain in increasing c
 //   T = K(i, s_q) - P                   direct distances in increasing feature order
 //   G = T L_i^{-T}                      one FMA chain in increasing e
 //   d(i) <- max(d(i) - sum_a G(i, a)^2, 0) in FP64, the squares added over a = t,
 //           t + 16, .. first and then over t in a butterfly (8, 4, 2, 1)
-//
-// because the pivots of a run follow every rounding of d.
 //
 // CTA = 128 threads on 128 rows x NC columns (NC = 32 or 64 by the block size b:
 // with one width of 64 a block of 32 did twice the products it needs); thread

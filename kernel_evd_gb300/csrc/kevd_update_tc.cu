@@ -50,6 +50,7 @@
 // MMA's B reads.
 #include "kevd_internal.cuh"
 #include "kevd_pairtile.cuh"
+#include "kevd_round.cuh"
 #include "kevd_tc.cuh"
 
 #include <cuda.h>
@@ -119,21 +120,11 @@ struct Bars {
 __device__ __forceinline__ bool is_cvt_warp(int w) { return w == 2 || w == 3 || (w >= 8 && w <= 13); }
 __device__ __forceinline__ int cvt_group(int w) { return w >= 10 ? 1 : 0; }
 
-struct RoundView {   // must match the RoundState layout of kevd_rpchol.cu
-    int64_t rank;
-    int64_t r_old;
-    int32_t nacc;
-    int32_t done;
-    int32_t rounds;
-    int32_t cur;
-    double total;
-};
-
 // Update pass g of a round that accepted more than kCols columns: columns
 // r_old + kCols g .. against the factor's first r_old + kCols g columns (the
 // same split as the SIMT update in kevd_rpchol.cu).  False when the pass has
 // no column.
-__device__ __forceinline__ bool pass_view(const RoundView* st, int group, int64_t& r, int& nacc) {
+__device__ __forceinline__ bool pass_view(const RoundState* st, int group, int64_t& r, int& nacc) {
     if (st->done) return false;
     r = st->r_old + (int64_t)kCols * group;
     nacc = min(kCols, st->nacc - kCols * group);
@@ -150,7 +141,7 @@ __device__ __forceinline__ void load_ktile(const CUtensorMap* tmk, uint8_t* ktil
 __global__ void __launch_bounds__(kThreads, 1)
 update_tc_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ CUtensorMap tmk,
                  float* __restrict__ F, int64_t ldF, int64_t N, const float* __restrict__ minv_f, int b,
-                 const uint8_t* __restrict__ bprep, const RoundView* st, double* __restrict__ dvec,
+                 const uint8_t* __restrict__ bprep, const RoundState* st, double* __restrict__ dvec,
                  double* __restrict__ dblk, int* __restrict__ err, int group) {
     int64_t r;
     int nacc;
@@ -447,10 +438,9 @@ update_tc_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant
             // T[a0 .. a0 + 15], which no later block needs.  A lane forms four outputs
             // of four rows as packed pairs, each G[a] one FMA chain over e = 0 .. in
             // increasing order (the zero terms above the diagonal leave it unchanged):
-            // 32 bytes of shared memory a lane serve 16 FMAs.  The whole tail
-            // of a row block takes 17k clocks (25k with a row's outputs in one thread,
-            // bound by its reads of L_i^{-1}), so updates of r < 600 columns no longer wait
-            // for it: N = 2M, k = 2,000, all updates 58.5 -> 55.8 ms.
+            // 32 bytes of shared memory a lane serve 16 FMAs.  N = 2M, k = 2,000, all
+            // updates 55.8 ms; 58.5 with a row's outputs in one thread, bound by its reads
+            // of L_i^{-1}.
             __syncwarp();   // the warp's rows of T are staged
             {
                 const int h = 8 * q + (lane & 7), oq = lane >> 3;
@@ -563,7 +553,7 @@ constexpr size_t kKcSmem = (size_t)kPtChunk * (kRows + kCols) * sizeof(float);
 
 __global__ void __launch_bounds__(kKcThreads, kKcCtasPerSm)
 update_kcols_kernel(const float* __restrict__ X, int64_t N, int d, ScalePair scale, const int64_t* __restrict__ sacc,
-                    const RoundView* st, float* __restrict__ Kc, int group) {
+                    const RoundState* st, float* __restrict__ Kc, int group) {
     int64_t r_unused;
     int nacc;
     if (!pass_view(st, group, r_unused, nacc)) return;
@@ -632,7 +622,7 @@ update_kcols_kernel(const float* __restrict__ X, int64_t N, int d, ScalePair sca
 // stage s -> [hi: 64 rows x 32 cols][lo], K-major SW128 (rows >= nacc and
 // columns >= r are zero).
 __global__ void update_prep_kernel(const float* __restrict__ F, int64_t ldF, const int64_t* __restrict__ sacc,
-                                   const RoundView* st, int n_stages_max, uint8_t* __restrict__ bprep, int group) {
+                                   const RoundState* st, int n_stages_max, uint8_t* __restrict__ bprep, int group) {
     int64_t r;
     int nacc;
     if (!pass_view(st, group, r, nacc)) return;
@@ -720,7 +710,7 @@ int launch_update_tc(kevd_ctx* ctx, float* F, int64_t ldF, int64_t N, int64_t k_
     int rc = KEVD_OK;
     uint8_t* bprep = arena_get<uint8_t>(ctx, "utc.bprep", (size_t)std::max(1, n_stages_max) * 2 * kBTile, &rc);
     if (rc != KEVD_OK) return set_error(ctx, rc, "update_tc: out of device memory");
-    const RoundView* rv = static_cast<const RoundView*>(round_state);
+    const RoundState* rv = static_cast<const RoundState*>(round_state);
     // K(R, S_i): update_kcols_kernel writes an N x 64 buffer that the update
     // kernel loads by TMA, one 128-row tile per row block
     float* Kc = nullptr;
