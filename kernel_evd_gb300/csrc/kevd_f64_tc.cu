@@ -642,12 +642,14 @@ __device__ __forceinline__ float scaled_abs(double x, int e) {
 
 // Sum and count over 32 columns of four sample rows of (n + 1) / S^2, S = sum_{k <= n}
 // |K(i, k) Linv(n, k)| / 2^(ek + el), for the outputs that the digits form.  Thread (j, c)
-// of 8 x 32 takes every eighth k of column c.
+// of 8 x 32 takes every eighth k of column c.  One wave of latency-bound CTAs; 1,024
+// terms staged at a time for few barriers.
+constexpr int kRangeChunk = 1024;
 __global__ void __launch_bounds__(256)
 tri_range_kernel(const double* __restrict__ K, const double* __restrict__ Linv, const int* __restrict__ ek,
                  const int* __restrict__ el, const int* __restrict__ prefix, int64_t M, int64_t r,
                  double* __restrict__ part) {
-    __shared__ float ks[128][4];
+    __shared__ __align__(16) float ks[kRangeChunk][4];
     __shared__ float sums[8][32][4];
     __shared__ int64_t row[4];
     const int tid = threadIdx.x, c = tid & 31, j = tid >> 5;
@@ -663,15 +665,19 @@ tri_range_kernel(const double* __restrict__ K, const double* __restrict__ Linv, 
     const int en = n < r ? el[n] : 0;
     const double* L = Linv + (n < r ? n : 0);
     float s[4] = {0.f, 0.f, 0.f, 0.f};
-    for (int64_t k0 = 0; k0 < min(r, n0 + 32); k0 += 128) {
+    const int64_t kend = min(r, n0 + 32);
+    for (int64_t k0 = 0; k0 < kend; k0 += kRangeChunk) {
+        const int kc = (int)min((int64_t)kRangeChunk, kend - k0);
         __syncthreads();
-        for (int e = tid; e < 512; e += 256) {
-            const int64_t k = k0 + (e >> 2), i = row[e & 3];
-            ks[e >> 2][e & 3] = k < r ? scaled_abs(K[i * r + k], ek[i]) : 0.f;
+        {   // a wave along the row: row tid / 64 of the four
+            const int64_t i = row[tid >> 6];
+            const int e = ek[i];
+#pragma unroll 4
+            for (int k = tid & 63; k < kc; k += 64) ks[k][tid >> 6] = scaled_abs(K[i * r + k0 + k], e);
         }
         __syncthreads();
-        const int kn = n < r ? (int)min((int64_t)128, n + 1 - k0) : 0;
-#pragma unroll 8
+        const int kn = n < r ? (int)min((int64_t)kc, n + 1 - k0) : 0;
+#pragma unroll 16
         for (int k = j; k < kn; k += 8) {
             const float l = scaled_abs(L[(k0 + k) * r], en);
             const float4 x = *reinterpret_cast<const float4*>(ks[k]);
