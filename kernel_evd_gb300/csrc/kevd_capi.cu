@@ -369,9 +369,8 @@ int kevd_factor_from_linv(kevd_ctx* ctx, const float* X, int64_t N, int32_t d, d
     KEVD_CUDA(ctx, cudaMemcpyAsync(Li, Linv, (size_t)r * r * sizeof(double), cudaMemcpyHostToDevice, s));
     // F panel = (K panel) Linv^T, Linv lower triangular (its upper part is never
     // read).  In exact slices on the tensor cores (N = 100,000, r = 1,024, d = 64:
-    // 13.9 ms the call, 8.2 of them this product and 5.0 the kernel panels; relative
-    // error against extended precision 1.2e-15); on the FP64 pipe (a triangular
-    // multiply, half the work of a GEMM; 146 ms, 8.3e-15) where the product is
+    // 13.7 ms the call, 8.5 of them this product and 5.0 the kernel panels); on the FP64
+    // pipe (a triangular multiply, half the work of a GEMM; 146 ms) where the product is
     // smaller than the slices' launches, has no room, Linv is not finite, or the
     // panel's outputs are too uneven for fixed point.
     // Fixed point holds an output to its row's size.  Where the kernel spans many orders

@@ -13,7 +13,8 @@
 //
 // The landmarks are cut into kGroups fixed groups (a function of r alone), one
 // CTA of a 16-CTA cluster each; the groups' sums meet in FP64 through
-// distributed shared memory, in group order.  A single state then occupies 16
+// distributed shared memory, in group order (or one CTA walks through the groups, where
+// landmarks are few for the batch).  A single state then occupies 16
 // SMs instead of one, no workspace is needed (calls on any streams are
 // independent, and the launch can be captured), and no thread ever combines
 // two states: a state's values are bit-identical whatever batch it is in and
