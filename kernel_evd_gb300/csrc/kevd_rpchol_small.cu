@@ -174,16 +174,16 @@ rp_small_propose_kernel(const double* __restrict__ F, int64_t ldF, const float* 
         acc = warp_sum(acc);
         if (lane == 0) part[pr][g] = acc;
         if (g == 0) {
+            // p == q too: a state with an infinity or a NaN has no distance to itself, H is
+            // NaN and it is rejected
             double d2 = 0.0;
-            if (p != q) {
-                const float* xp = X + props[p] * d;
-                const float* xq = X + props[q] * d;
-                for (int k = lane; k < d; k += 32) {
-                    const double v = (double)xp[k] - (double)xq[k];
-                    d2 += v * v;
-                }
-                d2 = warp_sum(d2);
+            const float* xp = X + props[p] * d;
+            const float* xq = X + props[q] * d;
+            for (int k = lane; k < d; k += 32) {
+                const double v = (double)xp[k] - (double)xq[k];
+                d2 += v * v;
             }
+            d2 = warp_sum(d2);
             if (lane == 0) kss[pr] = exp(-scale * d2);
         }
     }
